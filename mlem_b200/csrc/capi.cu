@@ -82,14 +82,18 @@ namespace {
 
 namespace mlem {
 SparseView csr_view(const mlem_ctx* c) {
-    return SparseView{c->row_ptr, reinterpret_cast<const uint4*>(c->elems), c->R, c->Z,
-                      c->row_order, c->row_order ? c->row_ranges : nullptr};
+    SparseView v{c->row_ptr, reinterpret_cast<const uint4*>(c->elems), c->R, c->Z,
+                 c->row_order, c->row_order ? c->row_ranges : nullptr};
+    v.max_len = c->max_row_len;
+    return v;
 }
 }  // namespace mlem
 
 namespace {
 SparseView csc_view(const mlem_ctx* c) {
-    return SparseView{c->col_ptr, reinterpret_cast<const uint4*>(c->celems), c->C, c->Z};
+    SparseView v{c->col_ptr, reinterpret_cast<const uint4*>(c->celems), c->C, c->Z};
+    v.max_len = c->max_col_len;
+    return v;
 }
 
 int sm_count(int device) {
@@ -762,22 +766,22 @@ int enqueue_iteration(mlem_ctx* c, const mlem_tuning& t, bool stats,
                 const bool by_visit = csc_by_visit(c, t);
                 if (by_visit && !c->celems_vis)
                     return fail(c, MLEM_ERR_STATE, "the CSC in visiting order is not built");
-                SparseView fw = csr;
+                // the forward pass visits the rows in the sorted order where there
+                // is one, whatever the visit: a row's sum does not depend on it
+                SparseView fw = csr_view(c);
                 SparseView bk = csc_view(c);
                 if (by_visit) {
                     fw.out_by_visit = true;
                     bk.pairs = reinterpret_cast<const uint4*>(c->celems_vis);
-                    if (c->act_ready && c->row_pos) {
-                        // walk only the rows with counts; the others keep calcCorrel 0
+                    if (c->csc_act_ready) {
+                        // only the rows with counts: the cut copy has no entry of another
+                        // row, so the others' correlations are not read
                         fw.order = c->act_order;
                         fw.vrange = c->act_ranges;
                         fw.n_dev = c->act_n;
                         fw.out_pos = c->row_pos;
-                        CK(c, cudaMemsetAsync(c->correl, 0, (size_t)c->R * Bp * 4, st));
-                        if (c->csc_act_ready) {  // and only the entries of those rows
-                            bk.pairs = reinterpret_cast<const uint4*>(c->csc_act);
-                            bk.len = c->csc_act_len;
-                        }
+                        bk.pairs = reinterpret_cast<const uint4*>(c->csc_act);
+                        bk.len = c->csc_act_len;
                     }
                 }
                 for (uint32_t f0 = 0; f0 < Bp; f0 += T)
@@ -944,7 +948,8 @@ void phase_bytes_for(const mlem_ctx* c, int bk_mode, int frame_tile, double* byt
         if (!exact && c->n_long) launches[0] += 2;  // the long-row kernels
     } else {
         bytes[0] = tiles * csr_pass + B * (4.0 * C + 4.0 * R + 4.0 * R);  // x, sino, correl
-        if (act && csc_act) bytes[0] += B * 4.0 * (double)c->R;  // the correlations zeroed
+        if (act && csc_act && !c->csc_act_ready)  // the other rows: range, counts, a zero written
+            bytes[0] += ((double)c->R - R) * (8.0 + B * 8.0);
         launches[0] = exact ? 1 : nt;
     }
     if (mode == MLEM_BK_CSC) {

@@ -40,169 +40,6 @@ namespace {
     (void)VW;
 
 // ---------------------------------------------------------------------------
-// Forward projection (+ calcCorrel).
-// ---------------------------------------------------------------------------
-template <int G, int BT>
-__global__ void __launch_bounds__(256) k_fwproj(SparseView csr, const float* __restrict__ x,
-                                                uint32_t B, uint32_t f0,
-                                                const int32_t* __restrict__ sino,
-                                                float* __restrict__ c, float* __restrict__ y) {
-    MLEM_WARP_LOOP_SETUP
-    const uint2* el = reinterpret_cast<const uint2*>(csr.pairs);
-    // Only the correlation wanted: a row whose counts are zero in the tile's
-    // frames has calcCorrel 0 whatever its projection, so its elements are
-    // not read (the counts are loaded beside the row range).
-    const bool skip_empty = c != nullptr && y == nullptr;
-    // the visiting positions: a device-built list (the rows with counts) or all n
-    const uint64_t nv = visit_count(csr);
-    for (uint64_t base = warp * RPW; base < nv; base += nwarps * RPW) {
-        const uint64_t v = base + lw / G;
-        const bool active = v < nv;
-        uint64_t r = 0, b = 0, e = 0;
-        int32_t s[VW];
-#pragma unroll
-        for (int i = 0; i < VW; ++i) s[i] = 0;
-        if (active) {
-            if (csr.vrange) {  // a sorted visit: the row's range in one load
-                const ulonglong2 q = csr.vrange[v];
-                r = csr.order[v];
-                b = q.x;
-                e = q.y;
-            } else {
-                r = row_at(csr, v);
-                b = csr.ptr[r];
-                e = csr.ptr[r + 1];
-            }
-            if (c) ld_counts<VW>(sino + r * B + f0 + sub * VW, s);
-        }
-        if (skip_empty) {
-            bool any = false;
-#pragma unroll
-            for (int i = 0; i < VW; ++i) any |= s[i] != 0;
-            // the group's frames are split over its FL lanes: all of them decide
-#pragma unroll
-            for (int o = 1; o < FL; o <<= 1) any |= __shfl_xor_sync(MLEM_FULL_MASK, any, o) != 0;
-            if (!any) e = b;  // an empty walk: the sum is 0, calcCorrel 0
-        }
-        float acc[VW];
-        row_dot<G, BT, false>(el, b, e, lane, x, B, f0 + sub * VW, acc, ps, ph);
-        slot_allreduce<G, BT>(acc);
-        if (active && lane < FL) {
-            const uint64_t pos = csr.out_pos ? (uint64_t)csr.out_pos[r] : v;
-            const uint64_t oidx = (csr.out_by_visit ? pos : r) * B + f0 + sub * VW;
-            if (y) st_vec<VW>(y + oidx, acc);
-            if (c) {
-                float o[VW];
-#pragma unroll
-                for (int i = 0; i < VW; ++i) o[i] = correl_of(s[i], acc[i]);
-                st_vec<VW>(c + oidx, o);
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Back projection over the CSC copy (+ calcUpdate).
-// ---------------------------------------------------------------------------
-template <int G, int BT>
-__global__ void __launch_bounds__(256) k_bkproj_csc(SparseView csc, const float* __restrict__ c,
-                                                    uint32_t B, uint32_t f0,
-                                                    const float* __restrict__ norm,
-                                                    float* __restrict__ x, float* __restrict__ u) {
-    MLEM_WARP_LOOP_SETUP
-    const uint2* el = reinterpret_cast<const uint2*>(csc.pairs);
-    for (uint64_t base = warp * RPW; base < csc.n; base += nwarps * RPW) {
-        const uint64_t col = base + lw / G;
-        const bool active = col < csc.n;
-        uint64_t b = 0, e = 0;
-        if (active) span_of(csc, col, b, e);
-        float acc[VW];
-        row_dot<G, BT, false>(el, b, e, lane, c, B, f0 + sub * VW, acc, ps, ph);
-        slot_allreduce<G, BT>(acc);
-        if (active && lane < FL) {
-            const uint64_t idx = col * B + f0 + sub * VW;
-            if (norm) {
-                const float n = norm[col];
-                float xv[VW];
-                ld_plain<VW>(x + idx, xv);
-#pragma unroll
-                for (int i = 0; i < VW; ++i) xv[i] *= update_factor(acc[i], n);
-                st_vec<VW>(x + idx, xv);
-            } else {
-                st_vec<VW>(u + idx, acc);
-            }
-        }
-    }
-}
-
-// The same back projection at one frame per pass and 32 lanes per column,
-// with each warp's batches of 256 elements pipelined in registers across its
-// columns: the element loads of the next batch (of this column or of the
-// warp's next column) go out before the current batch's correlation gathers,
-// so a batch costs about one memory round trip instead of two.  The lanes add
-// their elements in the order of k_bkproj_csc<32, 1> and the same butterfly
-// combines them: the results are those of that kernel, bit for bit.
-__global__ void __launch_bounds__(256) k_bkproj_csc_pipe(SparseView csc, const float* __restrict__ c,
-                                                         uint32_t B, uint32_t f0,
-                                                         const float* __restrict__ norm,
-                                                         float* __restrict__ x) {
-    constexpr int kBatch = 8;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint64_t ps = l2_evict_first(), ph = l2_evict_last();
-    const uint2* el = reinterpret_cast<const uint2*>(csc.pairs);
-    const uint64_t n = csc.n;
-    uint64_t col = warp;
-    if (col >= n) return;
-    uint64_t k0 = 0, e = 0;
-    span_of(csc, col, k0, e);
-    uint2 q[kBatch];
-#pragma unroll
-    for (int t = 0; t < kBatch; ++t) {
-        const uint64_t k = k0 + lane + 32 * t;
-        q[t] = k < e ? ld_stream2(el + k, ps) : make_uint2(0u, 0u);
-    }
-    float acc = 0.0f;
-    for (;;) {
-        // the next batch: the rest of this column, else the warp's next column
-        uint64_t ncol = col, nk0 = k0 + 32 * kBatch, ne = e;
-        if (nk0 >= e) {
-            ncol = col + nwarps;
-            nk0 = ne = 0;
-            if (ncol < n) span_of(csc, ncol, nk0, ne);
-        }
-        uint2 qn[kBatch];
-#pragma unroll
-        for (int t = 0; t < kBatch; ++t) {
-            const uint64_t k = nk0 + lane + 32 * t;
-            qn[t] = k < ne ? ld_stream2(el + k, ps) : make_uint2(0u, 0u);
-        }
-        float xv[kBatch];
-#pragma unroll
-        for (int t = 0; t < kBatch; ++t)
-            xv[t] = k0 + lane + 32 * t < e ? ld_hot(c + (size_t)q[t].x * B + f0, ph) : 0.0f;
-#pragma unroll
-        for (int t = 0; t < kBatch; ++t) acc = fmaf(__uint_as_float(q[t].y), xv[t], acc);
-        if (ncol != col) {  // the column is complete: k_bkproj_csc's butterfly and epilogue
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) acc += __shfl_xor_sync(MLEM_FULL_MASK, acc, o);
-            if (lane == 0) {
-                const uint64_t idx = col * B + f0;
-                x[idx] *= update_factor(acc, norm[col]);
-            }
-            acc = 0.0f;
-            if (ncol >= n) break;
-        }
-        col = ncol;
-        k0 = nk0;
-        e = ne;
-#pragma unroll
-        for (int t = 0; t < kBatch; ++t) q[t] = qn[t];
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Back projection by atomic scatter over the CSR (the reference GPU drivers'
 // approach, mlem_cuda/helper_files/cudaKernels.cu:155-178, kept for
 // comparison and chosen by the autotuner where it wins).
@@ -430,8 +267,6 @@ cudaError_t dispatch(const LaunchCfg& cfg, cudaStream_t st, Args... args);
             KERNEL<G, BT><<<grid, 256, 0, st>>>(a...);                                 \
         }                                                                              \
     };
-MLEM_KERNEL_FUNCTOR(FwprojK, k_fwproj)
-MLEM_KERNEL_FUNCTOR(BkprojCscK, k_bkproj_csc)
 MLEM_KERNEL_FUNCTOR(ScatterK, k_bkproj_scatter)
 template <int G, int BT>
 struct FusedK {  // file order
@@ -482,29 +317,6 @@ bool cfg_valid(const LaunchCfg& c) {
                    c.frame_tile == 8 || c.frame_tile == 16;
     // lanes per element (frame_tile / min(frame_tile, 4)) never exceed the group
     return g && t && c.blocks_per_sm >= 1 && c.blocks_per_sm <= 8 && c.sm_count >= 1;
-}
-
-cudaError_t fwproj(const SparseView& csr, const float* x, uint32_t B, uint32_t f0,
-                   const int32_t* sino, float* c, float* y, const LaunchCfg& cfg,
-                   cudaStream_t st) {
-    if (!cfg_valid(cfg) || (B % cfg.frame_tile) || (f0 % cfg.frame_tile)) return cudaErrorInvalidValue;
-    if (csr.n == 0) return cudaSuccess;
-    return dispatch<FwprojK>(cfg, st, csr, x, B, f0, sino, c, y);
-}
-
-cudaError_t bkproj_csc(const SparseView& csc, const float* c, uint32_t B, uint32_t f0,
-                       const float* norm, float* x, float* u, const LaunchCfg& cfg,
-                       cudaStream_t st) {
-    if (!cfg_valid(cfg) || (B % cfg.frame_tile) || (f0 % cfg.frame_tile)) return cudaErrorInvalidValue;
-    if (csc.n == 0) return cudaSuccess;
-    if (cfg.group == 32 && cfg.frame_tile == 1 && norm) {
-        // the pipelined kernel (same results); 8 CTAs per SM measured best for
-        // it whatever the configuration's blocks per SM (plain-full: 1.40 ms
-        // against 1.66 for k_bkproj_csc<32, 1> at 4, the CSC method's choice)
-        k_bkproj_csc_pipe<<<8 * cfg.sm_count, 256, 0, st>>>(csc, c, B, f0, norm, x);
-        return cudaGetLastError();
-    }
-    return dispatch<BkprojCscK>(cfg, st, csc, c, B, f0, norm, x, u);
 }
 
 cudaError_t bkproj_scatter(const SparseView& csr, const float* c, uint32_t B, uint32_t f0,

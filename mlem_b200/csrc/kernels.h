@@ -43,10 +43,13 @@ struct SparseView {
     // k_fwproj only, with out_by_visit and a device-built list (n_dev): the
     // position of row r in the full visiting order is out_pos[r].
     const uint32_t* out_pos = nullptr;
-    // CSC kernels (k_bkproj_csc, k_bkproj_csc_pipe) only, when non-null:
-    // column col holds len[col] entries from ptr[col] (the rest of its span
-    // is unused), the layout csc_active_build writes.
+    // k_bkproj_csc only, when non-null: column col holds len[col] entries from
+    // ptr[col] (the rest of its span is unused), the layout csc_active_build
+    // writes.
     const uint32_t* len = nullptr;
+    // The longest row (column), for the gather passes' choice of lanes; ~0 when
+    // unknown.
+    uint32_t max_len = ~0u;
 };
 
 // Entry range of column (or row) i: [ptr[i], ptr[i + 1]), or len[i] entries from ptr[i].

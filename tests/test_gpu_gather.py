@@ -1,0 +1,71 @@
+"""The gather passes (forward projection over rows, back projection over
+columns) at the sizes where their batches, lane groups and lane rule turn
+over: rows and columns of 0, 1 and batch +- 1 elements, few long columns, many
+short rows, one row far longer than the rest, and caller vectors on 4-, 8- and
+16-byte boundaries, for every group and frame tile.  Every sum must lie within
+the rounding of a float sum of its products: n 2^-23 sum |v x|."""
+import numpy as np
+import pytest
+
+from mlem_b200 import api, formats
+
+pytestmark = pytest.mark.gpu
+
+
+def matrix(kind, rng):
+    if kind == "edges":  # around multiples of every batch (lanes x depth), 1 to 384 elements
+        lens = np.array([0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32, 33, 47, 48, 49, 63, 64,
+                         65, 95, 96, 97, 127, 128, 129, 191, 192, 193, 255, 256, 257, 383, 384, 385, 0, 0])
+        R, C = lens.size, 97
+    elif kind == "few-columns":  # long columns, fewer than the resident groups
+        lens, R, C = np.full(20000, 6), 20000, 11
+    elif kind == "many-rows":  # 8 lanes a row and a column
+        lens, R, C = rng.integers(0, 5, 60000), 60000, 30000
+    else:  # one row and one column far longer than a group's share
+        lens = rng.integers(0, 5, 60000)
+        lens[777] = 70000
+        R, C = 60000, 30000
+    end = np.cumsum(lens).astype(np.uint64)
+    el = np.zeros(int(end[-1]), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, C, el.size)
+    if kind == "one-long":
+        el["index"][rng.random(el.size) < 0.3] = 4
+    el["value"] = rng.uniform(-1.0, 1.7, el.size)
+    return formats.Csr4(R, C, end, el)
+
+
+def sums(m, x, transpose):
+    """float64 sums, their magnitudes and their lengths."""
+    rows = np.repeat(np.arange(m.n_rows), np.diff(np.concatenate([[0], m.row_end.astype(np.int64)])))
+    cols, v = m.elems["index"].astype(np.int64), m.elems["value"].astype(np.float64)
+    to, frm, n = (cols, rows, m.n_cols) if transpose else (rows, cols, m.n_rows)
+    p = v[:, None] * x.astype(np.float64)[frm]
+    out, mag = np.zeros((n, x.shape[1])), np.zeros((n, x.shape[1]))
+    np.add.at(out, to, p)
+    np.add.at(mag, to, np.abs(p))
+    return out, mag, np.bincount(to, minlength=n)[:, None]
+
+
+@pytest.mark.parametrize("kind", ["edges", "few-columns", "many-rows", "one-long"])
+def test_gather_passes_against_float64(kind):
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(11)
+    m = matrix(kind, rng)
+    st = torch.cuda.current_stream().cuda_stream
+    with api.Context.from_matrix(m) as ctx:
+        for B in (1, 2, 4, 8, 16, 3):
+            x, y = (rng.uniform(0.1, 1.0, (n, B)).astype(np.float32) for n in (m.n_cols, m.n_rows))
+            want = {"fw": sums(m, x, False), "bk": sums(m, y, True)}
+            for group in (4, 8, 16, 32):
+                ctx.set_tuning(bk_mode=api.BK_CSC, group=group, frame_tile=1, blocks_per_sm=8)
+                # the vectors `shift` floats past a 512-byte boundary: any float boundary at one
+                # frame, 8 bytes at two and 16 at more
+                for shift in (0, 1 if B in (1, 3) else 2 if B == 2 else 4):
+                    for way, src, n, call in (("fw", x, m.n_rows, ctx.fwproj_d), ("bk", y, m.n_cols, ctx.bkproj_d)):
+                        a = torch.zeros(src.size + shift, device="cuda")
+                        a[shift:] = torch.from_numpy(src.reshape(-1)).cuda()
+                        o = torch.full((n * B + shift,), np.nan, device="cuda")
+                        call(a[shift:].data_ptr(), o[shift:].data_ptr(), B, st)
+                        got = o[shift:].cpu().numpy().reshape(n, B)
+                        ref, mag, cnt = want[way]
+                        assert np.all(np.abs(got - ref) <= 2.0 ** -23 * (cnt + 1) * mag), (way, B, group, shift)
