@@ -435,6 +435,7 @@ int finish_create(mlem_ctx* c) {
     TRY(dev_alloc(c, &c->norm_nat, std::max<uint32_t>(c->C, 1)));
     TRY(norm_views(c));
     TRY(dev_alloc(c, &c->counter, 64));
+    CK(c, cudaMemsetAsync(c->counter, 0, 64 * sizeof(unsigned int), c->stream));
     // Row visiting order, from the device column indices (after the remap).
     if (!(c->flags & MLEM_FLAG_NO_ROW_ORDER) && c->R > 1) {
         uint32_t* order = nullptr;
@@ -450,6 +451,7 @@ int finish_create(mlem_ctx* c) {
         CK(c, row_ranges_build(csr_view(c), c->row_order, c->row_ranges, c->stream));
     }
     if (c->max_row_len > kLongRowElems) TRY(build_long_rows(c));
+    CK(c, cudaStreamSynchronize(c->stream));  // the next call may use another stream
     default_tuning(c);
     return MLEM_OK;
 }
@@ -543,6 +545,7 @@ int alloc_frames(mlem_ctx* c, uint32_t B) {
     TRY(dev_alloc(c, &c->correl, (size_t)c->R * Bp));
     TRY(dev_alloc(c, &c->update, (size_t)c->C * Bp));
     TRY(dev_alloc(c, &c->stats_scratch, stats_scratch_bytes(Bp)));
+    CK(c, cudaMemsetAsync(c->stats_scratch, 0, stats_scratch_bytes(Bp), c->stream));
     TRY(dev_alloc(c, &c->inits_dev, Bp));
     if (c->n_long) TRY(dev_alloc(c, &c->f_long, (size_t)c->n_long * Bp));
     CK(c, cudaMemsetAsync(c->sino, 0, (size_t)c->R * Bp * 4, c->stream));
@@ -736,6 +739,13 @@ int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, cudaStr
     return fused_pass(c, t, csr, c->x, c->sino, c->update, c->Bp, c->counter, st);
 }
 
+// The census is one launch in the two-pass methods without an update kernel of
+// their own (its launches are then a good part of a small iteration), two in
+// the others.
+bool stats_in_one(const mlem_ctx* c, int bk_mode) {
+    return (c->flags & MLEM_FLAG_EXACT) || bk_mode == MLEM_BK_CSC || bk_mode == MLEM_BK_REGION;
+}
+
 int enqueue_iteration(mlem_ctx* c, const mlem_tuning& t, bool stats,
                       const PhaseEvents* pe = nullptr) {
     const SparseView csr = csr_visit(c, t);
@@ -874,7 +884,7 @@ int enqueue_iteration(mlem_ctx* c, const mlem_tuning& t, bool stats,
     TRY(mark(c, pe, 3));
     if (stats)
         CK(c, image_stats(c->x, c->C, Bp, c->B, c->stats_scratch, c->stats_slot, c->hist_sums,
-                          c->hist_zeros, c->hist_subn, st));
+                          c->hist_zeros, c->hist_subn, stats_in_one(c, t.bk_mode), st));
     TRY(mark(c, pe, 4));
     return MLEM_OK;
 }
@@ -915,7 +925,7 @@ void phase_bytes_for(const mlem_ctx* c, int bk_mode, int frame_tile, double* byt
         launches[0] = nt + 1;
         launches[1] = nt;
         bytes[3] = 4.0 * C * B;
-        launches[3] = 2;
+        launches[3] = 1;
         return;
     }
     if (mode == MLEM_BK_MIRRORED) {
@@ -964,7 +974,7 @@ void phase_bytes_for(const mlem_ctx* c, int bk_mode, int frame_tile, double* byt
         launches[2] = 1;
     }
     bytes[3] = 4.0 * C * B;
-    launches[3] = 2;
+    launches[3] = mode == MLEM_BK_CSC ? 1 : 2;
 }
 
 void voxel_permutation(uint32_t nx, uint32_t ny, uint32_t nz, std::vector<uint32_t>& perm) {
@@ -1009,13 +1019,15 @@ void drop_graph(mlem_ctx* c) {
     c->graph_iters = 0;
 }
 
-// Capture `n` iterations (slot reset + n x (iteration + statistics)) into *out.
-int capture_into(mlem_ctx* c, int n, cudaGraphExec_t* out) {
+// Capture `n` iterations (slot reset + n x (iteration + statistics), or the
+// iterations alone) into *out.
+int capture_into(mlem_ctx* c, int n, bool stats, cudaGraphExec_t* out) {
     CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int s = MLEM_OK;
-    cudaError_t e = cudaMemsetAsync(c->stats_slot, 0, sizeof(unsigned int), c->stream);
+    cudaError_t e = stats ? cudaMemsetAsync(c->stats_slot, 0, sizeof(unsigned int), c->stream)
+                          : cudaSuccess;
     if (e != cudaSuccess) s = fail(c, MLEM_ERR_CUDA, "capture memset: %s", cudaGetErrorString(e));
-    for (int i = 0; i < n && s == MLEM_OK; ++i) s = enqueue_iteration(c, c->tuning, true);
+    for (int i = 0; i < n && s == MLEM_OK; ++i) s = enqueue_iteration(c, c->tuning, stats);
     cudaGraph_t g = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
     if (s != MLEM_OK) { if (g) cudaGraphDestroy(g); return s; }
@@ -1029,10 +1041,11 @@ int capture_into(mlem_ctx* c, int n, cudaGraphExec_t* out) {
     return MLEM_OK;
 }
 
-int capture(mlem_ctx* c, int n) {
+int capture(mlem_ctx* c, int n, bool stats) {
     drop_graph(c);
-    TRY(capture_into(c, n, &c->graph));
+    TRY(capture_into(c, n, stats, &c->graph));
     c->graph_iters = n;
+    c->graph_stats = stats;
     c->graph_dirty = false;
     return MLEM_OK;
 }
@@ -1521,7 +1534,7 @@ int mlem_kernels_per_iteration(const mlem_ctx* c, int* n) {
     if (!c || !n) return fail(nullptr, MLEM_ERR_INVALID, "null argument");
     if (!c->Bp) return fail(const_cast<mlem_ctx*>(c), MLEM_ERR_STATE, "no frames");
     const int tiles = (int)(c->Bp / (uint32_t)c->tuning.frame_tile);
-    int k = 2;  // image statistics
+    int k = stats_in_one(c, c->tuning.bk_mode) ? 1 : 2;  // image statistics
     if (c->flags & MLEM_FLAG_EXACT) k += 2;
     else if (c->tuning.bk_mode == MLEM_BK_CSC) k += 2 * tiles;
     else if (c->tuning.bk_mode == MLEM_BK_ATOMIC) k += 2 * tiles + 1;
@@ -1725,16 +1738,18 @@ int mlem_iterate(mlem_ctx* c, int n, double* sums, uint64_t* zeros, uint64_t* su
         TRY(ensure_region(c, c->tuning.frame_tile));
     // Chunks of up to 64 iterations, each one graph launch.
     const int chunk = std::min(n, 64);
+    const bool stats = sums || zeros || subn;  // the census only when the caller takes it
     TRY(ensure_history(c, chunk));
-    if (c->graph_dirty || !c->graph || c->graph_iters != chunk) TRY(capture(c, chunk));
+    if (c->graph_dirty || !c->graph || c->graph_iters != chunk || c->graph_stats != stats)
+        TRY(capture(c, chunk, stats));
     int done = 0;
     while (done < n) {
         const int k = std::min(chunk, n - done);
         if (k == chunk) {
             CK(c, cudaGraphLaunch(c->graph, c->stream));
         } else {
-            CK(c, cudaMemsetAsync(c->stats_slot, 0, 4, c->stream));
-            for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, c->tuning, true));
+            if (stats) CK(c, cudaMemsetAsync(c->stats_slot, 0, 4, c->stream));
+            for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, c->tuning, stats));
         }
         const size_t cnt = (size_t)k * c->B;
         if (sums) CK(c, cudaMemcpyAsync(sums + (size_t)done * c->B, c->hist_sums, cnt * 8,
@@ -1782,9 +1797,9 @@ int mlem_step_host(mlem_ctx* c, const int32_t* sino, float* images, uint32_t B) 
     c->images_ready = true;
     if (c->tuning.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
         TRY(ensure_region(c, c->tuning.frame_tile));
-    if (c->graph_dirty || !c->graph || c->graph_iters != 1) {
+    if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
         TRY(ensure_history(c, 1));
-        TRY(capture(c, 1));
+        TRY(capture(c, 1, false));
     }
     CK(c, cudaGraphLaunch(c->graph, c->stream));
     TRY(download_images(c, images));
@@ -1845,9 +1860,9 @@ static int stream_steps(mlem_ctx* c, const int32_t* const* sinos, float* const* 
         CK(c, cudaEventRecord(c->ev_sfree[cur], c->stream));
         TRY(build_active(c, false, false));
         ++c->sino_gen;
-        if (c->graph_dirty || !c->graph || c->graph_iters != 1) {
+        if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
             TRY(ensure_history(c, 1));
-            TRY(capture(c, 1));
+            TRY(capture(c, 1, false));
         }
         CK(c, cudaGraphLaunch(c->graph, c->stream));
         if (images && images[k]) {  // this iteration's images, once the buffer's last download is done
@@ -1921,13 +1936,13 @@ static int stream_steps_overlap(mlem_ctx* c, const int32_t* const* sinos, float*
         c->csc_act_ready = false;
         c->graph_dirty = true;
     }
-    if (c->graph_dirty || !c->graph || c->graph_iters != 1) {
+    if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
         TRY(ensure_history(c, 1));
-        TRY(capture(c, 1));
+        TRY(capture(c, 1, false));
     }
     if (!c->graph_alt) {
         swap_sets(c);
-        const int s = capture_into(c, 1, &c->graph_alt);
+        const int s = capture_into(c, 1, false, &c->graph_alt);
         swap_sets(c);
         TRY(s);
     }

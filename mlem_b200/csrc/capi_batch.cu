@@ -67,6 +67,7 @@ struct mlem_batch {
 
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
+    bool graph_stats = false;  // the graph holds the census
     bool graph_dirty = true;
     std::vector<const void*> graph_sig;  // context pointers the graph holds
 
@@ -390,7 +391,7 @@ int batch_enqueue(mlem_batch* b, bool stats, const PhaseEvents* pe = nullptr) {
     if (stats)
         for (mlem_ctx* c : b->ctx)
             BCK(b, image_stats(c->x, c->C, c->Bp, c->B, c->stats_scratch, c->stats_slot,
-                               c->hist_sums, c->hist_zeros, c->hist_subn, st));
+                               c->hist_sums, c->hist_zeros, c->hist_subn, false, st));
     TRY(bmark(b, pe, 4));
     return MLEM_OK;
 }
@@ -406,11 +407,11 @@ void batch_drop_graph(mlem_batch* b) {
     b->graph_iters = 0;
 }
 
-int batch_capture(mlem_batch* b, int n) {
+int batch_capture(mlem_batch* b, int n, bool stats) {
     batch_drop_graph(b);
     BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    int s = batch_reset_slots(b);
-    for (int i = 0; i < n && s == MLEM_OK; ++i) s = batch_enqueue(b, true);
+    int s = stats ? batch_reset_slots(b) : MLEM_OK;
+    for (int i = 0; i < n && s == MLEM_OK; ++i) s = batch_enqueue(b, stats);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (s != MLEM_OK) { if (g) cudaGraphDestroy(g); return s; }
@@ -419,6 +420,7 @@ int batch_capture(mlem_batch* b, int n) {
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return bfail(b, MLEM_ERR_CUDA, "instantiate: %s", cudaGetErrorString(e));
     b->graph_iters = n;
+    b->graph_stats = stats;
     b->graph_dirty = false;
     return MLEM_OK;
 }
@@ -529,6 +531,9 @@ int mlem_batch_create(mlem_batch** out, mlem_ctx* const* ctxs, uint32_t n_ctx) {
         cudaGetLastError();
         return bail(bfail(b, MLEM_ERR_NOMEM, "batch descriptors: cudaMalloc failed"));
     }
+    if (cudaMemsetAsync(b->counter, 0, kMaxGroups * kCounterStride * sizeof(unsigned int), b->stream) !=
+        cudaSuccess)
+        return bail(bfail(b, MLEM_ERR_CUDA, "batch counters: cudaMemsetAsync failed"));
     s = batch_refresh(b, 1);
     if (s != MLEM_OK) return bail(s);
     *out = b;
@@ -778,15 +783,18 @@ int mlem_batch_iterate(mlem_batch* b, int n, double* const* sums) {
     BCK(b, cudaSetDevice(b->device));
     const int chunk = std::min(n, 64);
     TRY(batch_refresh(b, chunk));
-    if (b->graph_dirty || !b->graph || b->graph_iters != chunk) TRY(batch_capture(b, chunk));
+    bool stats = false;  // the census only when the caller takes it
+    for (size_t i = 0; sums && i < b->ctx.size(); ++i) stats = stats || sums[i];
+    if (b->graph_dirty || !b->graph || b->graph_iters != chunk || b->graph_stats != stats)
+        TRY(batch_capture(b, chunk, stats));
     int done = 0;
     while (done < n) {
         const int k = std::min(chunk, n - done);
         if (k == chunk) {
             BCK(b, cudaGraphLaunch(b->graph, b->stream));
         } else {
-            TRY(batch_reset_slots(b));
-            for (int i = 0; i < k; ++i) TRY(batch_enqueue(b, true));
+            if (stats) TRY(batch_reset_slots(b));
+            for (int i = 0; i < k; ++i) TRY(batch_enqueue(b, stats));
         }
         bool any = false;
         for (size_t i = 0; sums && i < b->ctx.size(); ++i) {

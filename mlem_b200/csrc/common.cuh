@@ -65,15 +65,17 @@ __device__ __forceinline__ uint4 ld_keep(const uint4* ptr, uint64_t pol) {
     return r;
 }
 
+// The gathered vectors: not the .nc form, as the kernel before the reading one
+// writes them and the two may overlap (pdl_wait below).
 __device__ __forceinline__ float ld_hot(const float* ptr, uint64_t pol) {
     float r;
-    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r) : "l"(ptr), "l"(pol));
+    asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r) : "l"(ptr), "l"(pol));
     return r;
 }
 
 __device__ __forceinline__ float4 ld_hot4(const float4* ptr, uint64_t pol) {
     float4 r;
-    asm("ld.global.nc.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+    asm("ld.global.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
         : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
         : "l"(ptr), "l"(pol));
     return r;
@@ -121,6 +123,47 @@ __device__ __forceinline__ float correl_of(int32_t s, float f) {
 // calcUpdate factor (mlem_seq/seqcsr4mlem.cpp:128).
 __device__ __forceinline__ float update_factor(float u, float n) {
     return n != 0.0f ? u / n : u;
+}
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel started with launch_dependent may
+// begin while the kernel before it in the stream is still running its last
+// blocks, so its launch hides behind that tail.  pdl_wait() blocks until every earlier kernel has finished
+// and its writes are visible; it is each kernel's first statement, so nothing
+// is read or written before it and every thread passes it (a kernel that ended
+// without waiting would let its own successor run beside its predecessor).
+// pdl_release() directly after it lets the next kernel be launched.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                                    cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// A work counter's grab by one thread of a CTA, and the CTA's exit: the last
+// CTA to leave sets both words back to 0 for the next launch (they start as 0),
+// so no launch needs a memset before it.
+__device__ __forceinline__ uint32_t work_grab(unsigned int* counter) { return atomicAdd(counter, 1u); }
+__device__ __forceinline__ void work_leave(unsigned int* counter) {
+    if (atomicAdd(counter + 1, 1u) == gridDim.x - 1) {
+        counter[0] = 0u;
+        counter[1] = 0u;
+    }
 }
 
 }  // namespace mlem

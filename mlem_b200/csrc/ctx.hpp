@@ -172,6 +172,7 @@ struct mlem_ctx {
     mlem_tuning tuning{};
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
+    bool graph_stats = false;  // the graph holds the census
     bool graph_dirty = true;
 
     std::string err;

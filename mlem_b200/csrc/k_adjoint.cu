@@ -90,12 +90,17 @@ __global__ void __launch_bounds__(256) k_adjoint_chunked(SparseView csr, const f
     __shared__ uint32_t s_chunk;
     const uint64_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint64_t n = csr.n;
+    pdl_wait();
+    pdl_release();
     for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(counter, 1u);
+        if (threadIdx.x == 0) s_chunk = work_grab(counter);
         __syncthreads();
         const uint64_t ci = s_chunk;
         __syncthreads();  // s_chunk is rewritten by the next grab
-        if (ci >= (n + chunk - 1) / chunk) return;  // block-uniform
+        if (ci >= (n + chunk - 1) / chunk) {  // block-uniform
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
         const uint64_t r0 = ci * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
         adjoint_row_range<OP, SORTED>(csr, x, sino, rows, u, r0, r1, warp, nwarps);
     }
@@ -109,21 +114,15 @@ cudaError_t adjoint_pass(int op, const SparseView& csr, const float* x, const in
     if (csr.n == 0) return cudaSuccess;
     if (op != kOpRatio && op != kOpAdjoint) return cudaErrorInvalidValue;
     const bool sorted = csr.order && csr.vrange;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     // 4 CTAs of 256 threads per SM; about 16 chunks per CTA, at least 32 rows each
     const int grid = std::max(1, sm_count * 4);
     const uint64_t chunk64 = std::max<uint64_t>(32, ((uint64_t)csr.n + (uint64_t)grid * 16 - 1) /
                                                         ((uint64_t)grid * 16));
     const uint32_t chunk = (uint32_t)std::min<uint64_t>(chunk64, 0xffffffffull);
-    if (op == kOpRatio) {
-        if (sorted) k_adjoint_chunked<kOpRatio, true><<<grid, 256, 0, st>>>(csr, x, sino, rows, u, chunk, counter);
-        else k_adjoint_chunked<kOpRatio, false><<<grid, 256, 0, st>>>(csr, x, sino, rows, u, chunk, counter);
-    } else {
-        if (sorted) k_adjoint_chunked<kOpAdjoint, true><<<grid, 256, 0, st>>>(csr, x, sino, rows, u, chunk, counter);
-        else k_adjoint_chunked<kOpAdjoint, false><<<grid, 256, 0, st>>>(csr, x, sino, rows, u, chunk, counter);
-    }
-    return cudaGetLastError();
+    const auto kernel = op == kOpRatio
+                            ? (sorted ? k_adjoint_chunked<kOpRatio, true> : k_adjoint_chunked<kOpRatio, false>)
+                            : (sorted ? k_adjoint_chunked<kOpAdjoint, true> : k_adjoint_chunked<kOpAdjoint, false>);
+    return launch_dependent(kernel, grid, 256, 0, st, csr, x, sino, rows, u, chunk, counter);
 }
 
 }  // namespace mlem

@@ -34,16 +34,21 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch_fused(const BatchTab
                                                                    uint32_t n_items,
                                                                    unsigned int* __restrict__ counter) {
     __shared__ BatchItem s_item;
+    pdl_wait();
+    pdl_release();
     const uint64_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
-            const uint32_t it = atomicAdd(counter, 1u);
+            const uint32_t it = work_grab(counter);
             s_item = it < n_items ? items[it] : BatchItem{0u, 0u, 0u, 1u};
         }
         __syncthreads();
         const BatchItem item = s_item;
         __syncthreads();                 // s_item is rewritten by the next grab
-        if (item.pad) return;            // block-uniform: no items left
+        if (item.pad) {                  // block-uniform: no items left
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
         const BatchMat& m = t.mats[item.mat];
         const uint32_t Bp = m.Bp;
 #pragma unroll 1
@@ -63,18 +68,23 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch_staged(const BatchTa
                                                                     unsigned int* __restrict__ counter) {
     extern __shared__ uint4 s_stage[];
     __shared__ BatchItem s_item;
+    pdl_wait();
+    pdl_release();
     const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint2* stages = reinterpret_cast<const uint2*>(s_stage) + (size_t)warp * kStages * kStageCap;
     const uint32_t sa = (uint32_t)__cvta_generic_to_shared(stages);
     for (;;) {
         if (threadIdx.x == 0) {
-            const uint32_t it = atomicAdd(counter, 1u);
+            const uint32_t it = work_grab(counter);
             s_item = it < n_items ? items[it] : BatchItem{0u, 0u, 0u, 1u};
         }
         __syncthreads();
         const BatchItem item = s_item;
         __syncthreads();                 // s_item is rewritten by the next grab
-        if (item.pad) return;            // block-uniform: no items left
+        if (item.pad) {                  // block-uniform: no items left
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
         const BatchMat& m = t.mats[item.mat];
         const uint32_t Bp = m.Bp;
 #pragma unroll 1
@@ -91,8 +101,8 @@ cudaError_t launch_batch_staged(const BatchTable& t, const BatchItem* items, uin
     cudaError_t e = cudaFuncSetAttribute(k_batch_staged<BT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_batch_staged<BT><<<grid, kBatchThreads, smem, st>>>(t, items, n_items, counter);
-    return cudaGetLastError();
+    return launch_dependent(k_batch_staged<BT>, grid, kBatchThreads, smem, st, t, items, n_items,
+                            counter);
 }
 
 // Interleaved schedule: the rows of all matrices form one virtual row space
@@ -105,6 +115,8 @@ cudaError_t launch_batch_staged(const BatchTable& t, const BatchItem* items, uin
 // arguments instead of taking registers.
 template <int BT, bool SORTED>
 __global__ void __launch_bounds__(kBatchThreads, 4) k_batch_interleaved(const BatchTable t) {
+    pdl_wait();
+    pdl_release();
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t total = t.row_base[t.n];
@@ -132,14 +144,19 @@ __global__ void __launch_bounds__(1024, 1) k_fused_chunked(SparseView csr,
                                                                      unsigned int* __restrict__ counter) {
     __shared__ uint32_t s_chunk;
     const uint64_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    pdl_wait();
+    pdl_release();
     for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(counter, 1u);
+        if (threadIdx.x == 0) s_chunk = work_grab(counter);
         __syncthreads();
         const uint64_t ci = s_chunk;
         __syncthreads();  // s_chunk is rewritten by the next grab
         // re-read per chunk (a cached load) rather than held in a register
         const uint64_t n = visit_count(csr);
-        if (ci >= (n + chunk - 1) / chunk) return;  // block-uniform
+        if (ci >= (n + chunk - 1) / chunk) {  // block-uniform
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
         const uint64_t r0 = ci * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
 #pragma unroll 1
         for (uint32_t f0 = 0; f0 < B; f0 += BT)
@@ -157,37 +174,33 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
         return cudaErrorInvalidValue;
     if (ctas_per_sm != 1 && ctas_per_sm != 2 && ctas_per_sm != 4) return cudaErrorInvalidValue;
     if (!csr.order || !csr.vrange) return cudaErrorInvalidValue;  // a sorted visit
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     // the resident CTAs: 64 registers x 1024 threads per SM, in 1, 2 or 4 CTAs
     const int grid = std::max(1, sm_count * ctas_per_sm), threads = 1024 / ctas_per_sm;
     switch (frame_tile) {
-        case 1: k_fused_chunked<1><<<grid, threads, 0, st>>>(csr, x, B, sino, u, chunk_rows, counter); break;
-        case 2: k_fused_chunked<2><<<grid, threads, 0, st>>>(csr, x, B, sino, u, chunk_rows, counter); break;
-        case 4: k_fused_chunked<4><<<grid, threads, 0, st>>>(csr, x, B, sino, u, chunk_rows, counter); break;
-        case 8: k_fused_chunked<8><<<grid, threads, 0, st>>>(csr, x, B, sino, u, chunk_rows, counter); break;
-        case 16: k_fused_chunked<16><<<grid, threads, 0, st>>>(csr, x, B, sino, u, chunk_rows, counter); break;
+        case 1: return launch_dependent(k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 2: return launch_dependent(k_fused_chunked<2>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 4: return launch_dependent(k_fused_chunked<4>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 8: return launch_dependent(k_fused_chunked<8>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 16: return launch_dependent(k_fused_chunked<16>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
-#define MLEM_BATCH_TILES(KERNEL, ...)                                                \
-    switch (frame_tile) {                                                            \
-        case 1: (sorted ? KERNEL<1, true> : KERNEL<1, false>)<<<__VA_ARGS__; break;  \
-        case 2: (sorted ? KERNEL<2, true> : KERNEL<2, false>)<<<__VA_ARGS__; break;  \
-        case 4: (sorted ? KERNEL<4, true> : KERNEL<4, false>)<<<__VA_ARGS__; break;  \
-        case 8: (sorted ? KERNEL<8, true> : KERNEL<8, false>)<<<__VA_ARGS__; break;  \
-        case 16: (sorted ? KERNEL<16, true> : KERNEL<16, false>)<<<__VA_ARGS__; break; \
-        default: return cudaErrorInvalidValue;                                       \
+#define MLEM_BATCH_TILES(KERNEL, ...)                                                               \
+    switch (frame_tile) {                                                                           \
+        case 1: return launch_dependent(sorted ? KERNEL<1, true> : KERNEL<1, false>, __VA_ARGS__);  \
+        case 2: return launch_dependent(sorted ? KERNEL<2, true> : KERNEL<2, false>, __VA_ARGS__);  \
+        case 4: return launch_dependent(sorted ? KERNEL<4, true> : KERNEL<4, false>, __VA_ARGS__);  \
+        case 8: return launch_dependent(sorted ? KERNEL<8, true> : KERNEL<8, false>, __VA_ARGS__);  \
+        case 16: return launch_dependent(sorted ? KERNEL<16, true> : KERNEL<16, false>, __VA_ARGS__); \
+        default: return cudaErrorInvalidValue;                                                      \
     }
 
 cudaError_t batch_interleaved(const BatchTable& t, int frame_tile, bool sorted, int sm_count,
                               int blocks_per_sm, cudaStream_t st) {
     if (t.n == 0 || t.n > kBatchTableMax) return cudaErrorInvalidValue;
     const int grid = std::max(1, sm_count * blocks_per_sm);
-    MLEM_BATCH_TILES(k_batch_interleaved, grid, kBatchThreads, 0, st>>>(t))
-    return cudaGetLastError();
+    MLEM_BATCH_TILES(k_batch_interleaved, grid, kBatchThreads, 0, st, t)
 }
 
 cudaError_t batch_fused(const BatchTable& t, const BatchItem* items, uint32_t n_items,
@@ -195,12 +208,9 @@ cudaError_t batch_fused(const BatchTable& t, const BatchItem* items, uint32_t n_
                         int blocks_per_sm, cudaStream_t st) {
     if (n_items == 0) return cudaSuccess;
     if (t.n == 0 || t.n > kBatchTableMax) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     const int grid = std::max(1, std::min<int>((int)std::min<uint32_t>(n_items, 1u << 30),
                                                sm_count * blocks_per_sm));
-    MLEM_BATCH_TILES(k_batch_fused, grid, kBatchThreads, 0, st>>>(t, items, n_items, counter))
-    return cudaGetLastError();
+    MLEM_BATCH_TILES(k_batch_fused, grid, kBatchThreads, 0, st, t, items, n_items, counter)
 }
 
 cudaError_t batch_staged(const BatchTable& t, const BatchItem* items, uint32_t n_items,
@@ -210,8 +220,6 @@ cudaError_t batch_staged(const BatchTable& t, const BatchItem* items, uint32_t n
     if (t.n == 0 || t.n > kBatchTableMax) return cudaErrorInvalidValue;
     for (uint32_t i = 0; i < t.n; ++i)
         if (!t.mats[i].csr.order || !t.mats[i].csr.vrange) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     // at most 4 resident CTAs: each holds 32 KiB of stages
     const int grid = std::max(1, std::min<int>((int)std::min<uint32_t>(n_items, 1u << 30),
                                                sm_count * std::min(blocks_per_sm, 4)));

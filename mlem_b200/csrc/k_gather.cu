@@ -50,7 +50,8 @@ struct GLanes {
     static constexpr int FL = BT / VW;
 };
 
-// VW floats when `in`, else zeros.
+// VW floats when `in`, else zeros.  Not the .nc form: the kernel before this one
+// (which it may overlap up to pdl_wait) writes the vector.
 template <int VW>
 __device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW], uint64_t pol) {
     if constexpr (VW == 8) {
@@ -59,7 +60,7 @@ __device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW
             "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
             "mov.f32 %4, 0f00000000;\n\tmov.f32 %5, 0f00000000;\n\tmov.f32 %6, 0f00000000;\n\t"
             "mov.f32 %7, 0f00000000;\n\t"
-            "@p ld.global.nc.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;\n\t}"
+            "@p ld.global.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;\n\t}"
             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
               "=f"(v[7])
             : "l"(p), "l"(pol), "r"((uint32_t)in));
@@ -67,20 +68,20 @@ __device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
             "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-            "@p ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n\t}"
+            "@p ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n\t}"
             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
             : "l"(p), "l"(pol), "r"((uint32_t)in));
     } else if constexpr (VW == 2) {
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
             "mov.f32 %1, 0f00000000;\n\t"
-            "@p ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;\n\t}"
+            "@p ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;\n\t}"
             : "=f"(v[0]), "=f"(v[1])
             : "l"(p), "l"(pol), "r"((uint32_t)in));
     } else {
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "@p ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
+            "@p ld.global.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
             : "=f"(v[0])
             : "l"(p), "l"(pol), "r"((uint32_t)in));
     }
@@ -138,6 +139,9 @@ constexpr int kGatherCtas = 4;
 // calcCorrel.  SKIP: only the correlation is wanted and the visit is not a
 // list of rows with counts, so a row whose counts are zero in the tile's
 // frames (calcCorrel 0 whatever its projection) is walked as an empty one.
+// Tiles of up to four frames only: with eight or sixteen few rows are empty in
+// every frame, and the counts of two rows held per lane left the gathers no
+// registers (1.50 ms against 1.03 on 1,048,576 rows, 16 frames).
 // ---------------------------------------------------------------------------
 template <int G, int BT, bool SKIP>
 struct FwOp {
@@ -151,13 +155,14 @@ struct FwOp {
     bool writer;
     struct Row {
         const uint2* b;
-        uint64_t n;             // elements
+        uint64_t n;                // elements
         uint32_t r;
         int32_t s[SKIP ? VW : 1];  // SKIP: the counts, loaded with the range
     };
     struct Pre {
-        uint32_t o;     // output row
-        int32_t s[VW];
+        uint32_t o;                      // output row
+        uint32_t r;
+        int32_t s[VW < 8 ? VW : 1];      // the counts, a row ahead
     };
     __device__ __forceinline__ uint64_t count() const { return visit_count(csr); }
     // Row of visiting position v: loaded two rows ahead, so that its counts
@@ -185,9 +190,6 @@ struct FwOp {
             int any = 0;
 #pragma unroll
             for (int i = 0; i < VW; ++i) any |= q.s[i];
-            // the group's frames are split over its FL lanes: all of them decide
-#pragma unroll
-            for (int o = 1; o < GLanes<BT>::FL; o <<= 1) any |= __shfl_xor_sync(gmask, any, o);
             return any ? q.n : 0;
         } else {
             return q.n;
@@ -195,14 +197,16 @@ struct FwOp {
     }
     __device__ __forceinline__ Pre pre(const Row& q, uint32_t v) const {
         Pre p;
-        p.o = q.r;
+        p.o = p.r = q.r;
+        if constexpr (VW < 8) {
 #pragma unroll
-        for (int i = 0; i < VW; ++i) p.s[i] = 0;
-        if constexpr (SKIP) {
+            for (int i = 0; i < VW; ++i) p.s[i] = 0;
+            if constexpr (SKIP) {
 #pragma unroll
-            for (int i = 0; i < VW; ++i) p.s[i] = q.s[i];
-        } else if (c && writer) {
-            g_counts<VW>(sino + (size_t)q.r * B + off, p.s);
+                for (int i = 0; i < VW; ++i) p.s[i] = q.s[i];
+            } else if (c && writer) {
+                g_counts<VW>(sino + (size_t)q.r * B + off, p.s);
+            }
         }
         if (csr.out_by_visit && writer) p.o = csr.out_pos ? csr.out_pos[q.r] : v;
         return p;
@@ -212,9 +216,16 @@ struct FwOp {
         const size_t o = (size_t)p.o * B + off;
         if (y) g_store<VW>(y + o, acc);
         if (c) {
+            int32_t s[VW];
+            if constexpr (VW < 8) {
+#pragma unroll
+                for (int i = 0; i < VW; ++i) s[i] = p.s[i];
+            } else {  // eight counts held over the row cost more than this wait
+                g_counts<VW>(sino + (size_t)p.r * B + off, s);
+            }
             float t[VW];
 #pragma unroll
-            for (int i = 0; i < VW; ++i) t[i] = correl_of(p.s[i], acc[i]);
+            for (int i = 0; i < VW; ++i) t[i] = correl_of(s[i], acc[i]);
             g_store<VW>(c + o, t);
         }
     }
@@ -240,7 +251,7 @@ struct BkOp {
     };
     struct Pre {
         float n;
-        float x[VW];
+        float x[VW < 8 ? VW : 1];
     };
     __device__ __forceinline__ uint64_t count() const { return csc.n; }
     __device__ __forceinline__ uint32_t id(uint32_t v) const { return v; }
@@ -254,11 +265,9 @@ struct BkOp {
     __device__ __forceinline__ Pre pre(const Row&, uint32_t v) const {
         Pre p;
         p.n = 0.0f;
-#pragma unroll
-        for (int i = 0; i < VW; ++i) p.x[i] = 0.0f;
         if (norm && writer) {
             p.n = norm[v];
-            g_load<VW>(x + (size_t)v * B + off, p.x);
+            if constexpr (VW < 8) g_load<VW>(x + (size_t)v * B + off, p.x);
         }
         return p;
     }
@@ -267,8 +276,14 @@ struct BkOp {
         const size_t o = (size_t)v * B + off;
         if (norm) {
             float t[VW];
+            if constexpr (VW < 8) {
 #pragma unroll
-            for (int i = 0; i < VW; ++i) t[i] = p.x[i] * update_factor(acc[i], p.n);
+                for (int i = 0; i < VW; ++i) t[i] = p.x[i];
+            } else {
+                g_load<VW>(x + o, t);
+            }
+#pragma unroll
+            for (int i = 0; i < VW; ++i) t[i] *= update_factor(acc[i], p.n);
             g_store<VW>(x + o, t);
         } else {
             g_store<VW>(u + o, acc);
@@ -286,6 +301,8 @@ __device__ __forceinline__ void gather_walk(const Op& op, const float* __restric
     constexpr uint32_t kBatch = D * EPS;
     const int slot = (threadIdx.x & (G - 1)) / FL;
     const uint64_t ps = l2_evict_first(), ph = l2_evict_last();
+    pdl_wait();
+    pdl_release();
     const uint32_t n = (uint32_t)op.count();
     if (v >= n) return;
     uint32_t rows = (n - v - 1) / stride;  // rows after the current one
@@ -411,11 +428,12 @@ struct FwRun {
                            const float* x, uint32_t B, uint32_t f0, const int32_t* sino, float* c,
                            float* y) {
         const int grid = gather_grid<G, BT>(cfg, csr.n);
-        if (c && !y && !csr.n_dev)
-            k_fwproj<G, BT, true><<<grid, kGatherThreads, 0, st>>>(csr, x, B, f0, sino, c, y);
-        else
-            k_fwproj<G, BT, false><<<grid, kGatherThreads, 0, st>>>(csr, x, B, f0, sino, c, y);
-        return cudaGetLastError();
+        if constexpr (BT <= 4)
+            if (c && !y && !csr.n_dev)
+                return launch_dependent(k_fwproj<G, BT, true>, grid, kGatherThreads, 0, st, csr, x, B,
+                                        f0, sino, c, y);
+        return launch_dependent(k_fwproj<G, BT, false>, grid, kGatherThreads, 0, st, csr, x, B, f0,
+                                sino, c, y);
     }
 };
 
@@ -424,9 +442,8 @@ struct BkRun {
     static cudaError_t run(const LaunchCfg& cfg, cudaStream_t st, const SparseView& csc,
                            const float* c, uint32_t B, uint32_t f0, const float* norm, float* x,
                            float* u) {
-        k_bkproj_csc<G, BT><<<gather_grid<G, BT>(cfg, csc.n), kGatherThreads, 0, st>>>(
-            csc, c, B, f0, norm, x, u);
-        return cudaGetLastError();
+        return launch_dependent(k_bkproj_csc<G, BT>, gather_grid<G, BT>(cfg, csc.n), kGatherThreads, 0,
+                                st, csc, c, B, f0, norm, x, u);
     }
 };
 

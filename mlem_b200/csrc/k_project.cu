@@ -84,6 +84,8 @@ __global__ void __launch_bounds__(256) k_fused_row(SparseView csr, const float* 
                                                    float* __restrict__ u) {
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    pdl_wait();
+    pdl_release();
     fused_row_range<G, BT, SORTED>(csr, x, B, f0, sino, u, 0, visit_count(csr), warp, nwarps);
 }
 
@@ -94,6 +96,8 @@ template <bool ONE_FRAME>
 __global__ void k_apply_update(float* __restrict__ x, float* __restrict__ u,
                                const float* __restrict__ norm, uint64_t n, uint32_t B,
                                bool zero_u) {
+    pdl_wait();
+    pdl_release();
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t col = ONE_FRAME ? i : i / B;
@@ -234,6 +238,8 @@ template <bool ONE_FRAME>
 __global__ void k_apply_update_subset(float* __restrict__ x, float* __restrict__ u,
                                       const float* __restrict__ norm_s,
                                       const float* __restrict__ norm, uint64_t n, uint32_t B) {
+    pdl_wait();
+    pdl_release();
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t col = ONE_FRAME ? i : i / B;
@@ -272,14 +278,14 @@ template <int G, int BT>
 struct FusedK {  // file order
     template <typename... A>
     static void run(int grid, cudaStream_t st, A... a) {
-        k_fused_row<G, BT, false><<<grid, 256, 0, st>>>(a...);
+        launch_dependent(k_fused_row<G, BT, false>, grid, 256, 0, st, a...);
     }
 };
 template <int G, int BT>
 struct FusedSortedK {  // sorted visiting order (csr.order + csr.vrange)
     template <typename... A>
     static void run(int grid, cudaStream_t st, A... a) {
-        k_fused_row<G, BT, true><<<grid, 256, 0, st>>>(a...);
+        launch_dependent(k_fused_row<G, BT, true>, grid, 256, 0, st, a...);
     }
 };
 #undef MLEM_KERNEL_FUNCTOR
@@ -340,9 +346,8 @@ cudaError_t apply_update(float* x, float* u, const float* norm, uint32_t C, uint
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    if (B == 1) k_apply_update<true><<<grid, 256, 0, st>>>(x, u, norm, n, B, zero_u);
-    else k_apply_update<false><<<grid, 256, 0, st>>>(x, u, norm, n, B, zero_u);
-    return cudaGetLastError();
+    return launch_dependent(B == 1 ? k_apply_update<true> : k_apply_update<false>, grid, 256, 0, st, x,
+                            u, norm, n, B, zero_u);
 }
 
 cudaError_t apply_update_subset(float* x, float* u, const float* norm_s, const float* norm,
@@ -350,9 +355,8 @@ cudaError_t apply_update_subset(float* x, float* u, const float* norm_s, const f
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    if (B == 1) k_apply_update_subset<true><<<grid, 256, 0, st>>>(x, u, norm_s, norm, n, B);
-    else k_apply_update_subset<false><<<grid, 256, 0, st>>>(x, u, norm_s, norm, n, B);
-    return cudaGetLastError();
+    return launch_dependent(B == 1 ? k_apply_update_subset<true> : k_apply_update_subset<false>, grid,
+                            256, 0, st, x, u, norm_s, norm, n, B);
 }
 
 cudaError_t subset_column_sums_exact(const SparseView& csc, uint32_t S, uint32_t s, float* norm,

@@ -37,14 +37,19 @@ __global__ void __launch_bounds__(kStagedThreads, 4) k_fused_staged(SparseView c
     const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint2* stages = reinterpret_cast<const uint2*>(s_stage) + (size_t)warp * kStages * kStageCap;
     const uint32_t sa = (uint32_t)__cvta_generic_to_shared(stages);
+    pdl_wait();
+    pdl_release();
     for (;;) {
-        if (threadIdx.x == 0) s_chunk = atomicAdd(counter, 1u);
+        if (threadIdx.x == 0) s_chunk = work_grab(counter);
         __syncthreads();
         const uint64_t ci = s_chunk;
         __syncthreads();  // s_chunk is rewritten by the next grab
         // re-read per chunk (a cached load) rather than held in a register
         const uint64_t n = visit_count(csr);
-        if (ci >= (n + chunk - 1) / chunk) return;  // block-uniform
+        if (ci >= (n + chunk - 1) / chunk) {  // block-uniform
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
         const uint64_t r0 = ci * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
 #pragma unroll 1
         for (uint32_t f0 = 0; f0 < B; f0 += BT)
@@ -61,8 +66,8 @@ cudaError_t launch_staged(const SparseView& csr, const float* x, uint32_t B, con
     cudaError_t e = cudaFuncSetAttribute(k_fused_staged<BT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_fused_staged<BT><<<grid, kStagedThreads, smem, st>>>(csr, x, B, sino, u, chunk_rows, counter);
-    return cudaGetLastError();
+    return launch_dependent(k_fused_staged<BT>, grid, kStagedThreads, smem, st, csr, x, B, sino, u,
+                            chunk_rows, counter);
 }
 
 }  // namespace
@@ -75,8 +80,6 @@ cudaError_t fused_staged(const SparseView& csr, const float* x, uint32_t B, int 
         return cudaErrorInvalidValue;
     if (ctas_per_sm < 1 || ctas_per_sm > 4) return cudaErrorInvalidValue;
     if (!csr.order || !csr.vrange) return cudaErrorInvalidValue;  // a sorted visit
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     const int grid = std::max(1, sm_count * ctas_per_sm);
     switch (frame_tile) {
         case 1: return launch_staged<1>(csr, x, B, sino, u, chunk_rows, grid, counter, st);

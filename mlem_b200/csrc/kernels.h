@@ -192,15 +192,17 @@ cudaError_t column_sums_exact(const SparseView& csc, float* norm, cudaStream_t s
 cudaError_t column_sums_atomic(const SparseView& csr, uint32_t C, float* norm, cudaStream_t st);
 
 // ---- per-frame image statistics (sum in double, zeros, subnormals) -----
-// Deterministic: fixed-order block tree.  `partial` needs stats_scratch_bytes.
-// B is the interleave stride; the first n_out frames are written.  When
+// Deterministic: fixed-order block tree.  `partial` needs stats_scratch_bytes,
+// zeroed once.  B is the interleave stride (a padded frame count); the first
+// n_out frames are written.  one_launch: the last block adds the partials,
+// else a second kernel does.  When
 // `slot` is non-null, results go to row *slot of [n][n_out] outputs and the
 // kernel then increments *slot (so one captured graph serves every
 // iteration).
 size_t stats_scratch_bytes(uint32_t B);
 cudaError_t image_stats(const float* x, uint32_t C, uint32_t B, uint32_t n_out, void* partial,
                         unsigned int* slot, double* sums, unsigned long long* zeros,
-                        unsigned long long* subnormals, cudaStream_t st);
+                        unsigned long long* subnormals, bool one_launch, cudaStream_t st);
 
 // ---- layout helpers -------------------------------------------------------
 // out[p(i)*Bp + b] = in[b*n + i] for b < B (n items per frame; pad frames
@@ -399,7 +401,8 @@ static_assert(sizeof(BatchTable) <= 32764, "kernel parameter space (CUDA >= 12.1
 
 // Items schedule: every item does u[mat] += A^T correl(A x) over its rows,
 // all frames of its matrix in passes of frame_tile (1, 2, 4, 8 or 16;
-// divides every Bp).  `counter` (one uint) is reset on the stream first.
+// divides every Bp).  `counter` (two
+// words, 0 between launches: the last CTA to leave resets them) hands out items.
 // sorted: every matrix of the table is visited in its sorted order (their
 // views carry order and vrange); else every one in file order.
 cudaError_t batch_fused(const BatchTable& t, const BatchItem* items, uint32_t n_items,

@@ -23,7 +23,7 @@ struct Lanes {
 
 __device__ __forceinline__ float2 ld_hot2(const float2* ptr, uint64_t pol) {
     float2 r;
-    asm("ld.global.nc.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(r.x), "=f"(r.y)
+    asm("ld.global.L2::cache_hint.v2.f32 {%0,%1}, [%2], %3;" : "=f"(r.x), "=f"(r.y)
         : "l"(ptr), "l"(pol));
     return r;
 }
