@@ -137,6 +137,7 @@ void default_tuning(mlem_ctx* c) {
     c->tuning.blocks_per_sm = 8;
     c->tuning.visit = MLEM_VISIT_FILE;
     c->tuning.ms_per_iter = 0.0;
+    c->tile_follows = true;
 }
 
 // ---------------------------------------------------------------------------
@@ -200,6 +201,39 @@ int perm_scratch(mlem_ctx* c, size_t floats) {
     for (auto& p : c->pscratch) TRY(dev_alloc(c, &p, floats));
     c->pscratch_floats = floats;
     return MLEM_OK;
+}
+
+// Row scratch (and voxel scratch) of Bd floats each for the projections' padded
+// frames; false where they do not fit beside the matrix or would have to be
+// allocated while the caller's stream is being captured, and the caller's frame
+// count is walked as it is.
+bool room_for_padding(mlem_ctx* c, uint32_t Bd, cudaStream_t st) {
+    const size_t rows = (size_t)std::max<uint32_t>(c->R, 1) * Bd;
+    if (c->rscratch_floats < rows || c->pscratch_floats < (size_t)c->C * Bd) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    if (c->rscratch_floats < rows) {
+        if (c->rscratch) {
+            cudaFree(c->rscratch);
+            c->device_bytes -= c->rscratch_floats * 4;
+        }
+        c->rscratch = nullptr;
+        c->rscratch_floats = 0;
+        if (dev_alloc(c, &c->rscratch, rows) != MLEM_OK) {
+            c->err.clear();
+            return false;
+        }
+        c->rscratch_floats = rows;
+    }
+    if (perm_scratch(c, (size_t)c->C * Bd) != MLEM_OK) {
+        c->err.clear();
+        return false;
+    }
+    return true;
 }
 
 // Region-blocked copy for the tile size `frame_tile` (built once per tile
@@ -371,7 +405,7 @@ int build_long_rows(mlem_ctx* c) {
 // double sum).
 int norm_views(mlem_ctx* c) {
     if (c->bricked)
-        CK(c, permute_to_natural(c->norm, c->norm_nat, c->perm, c->C, 1, c->stream));
+        CK(c, permute_to_natural(c->norm, c->norm_nat, c->perm, c->C, 1, 1, c->stream));
     else if (c->C)
         CK(c, cudaMemcpyAsync(c->norm_nat, c->norm, (size_t)c->C * 4, cudaMemcpyDeviceToDevice,
                               c->stream));
@@ -552,7 +586,12 @@ int alloc_frames(mlem_ctx* c, uint32_t B) {
     CK(c, cudaMemsetAsync(c->x, 0, (size_t)c->C * Bp * 4, c->stream));
     CK(c, cudaMemsetAsync(c->correl, 0, (size_t)c->R * Bp * 4, c->stream));
     CK(c, cudaMemsetAsync(c->update, 0, (size_t)c->C * Bp * 4, c->stream));
-    c->tuning.frame_tile = std::min(c->tuning.frame_tile > 0 ? c->tuning.frame_tile : 16,
+    // the widest tile until a tuning is chosen: one walk over the matrix instead
+    // of one per frame (75 x 61 x 37 voxels, 120,007 rows, 5 frames: 372 us per
+    // iteration with tiles of 1, 115 with 8)
+    const bool follows = c->tile_follows && (c->tuning.bk_mode == MLEM_BK_CSC ||
+                                             c->tuning.bk_mode == MLEM_BK_ATOMIC);
+    c->tuning.frame_tile = std::min(c->tuning.frame_tile > 0 && !follows ? c->tuning.frame_tile : 16,
                                     default_tile(Bp));
     c->graph_dirty = true;
     return MLEM_OK;
@@ -1067,6 +1106,25 @@ LaunchCfg cfg_for_frames(const mlem_ctx* c, uint32_t B) {
     return cfg;
 }
 
+// Interleave stride of the device copies of B caller frames in the projections:
+// B, or the padded count whose passes cost least -- a frame count that is no
+// multiple of a wide tile otherwise walks the matrix once per one, two or four
+// frames.  Cost of a pass by its tile, forward + back projection of 1,048,576
+// rows: 490, 656, 890, 1340, 2100 us for 1, 2, 4, 8, 16 frames.
+uint32_t projection_stride(uint32_t B) {
+    auto cost = [](uint32_t n) {
+        for (auto t : {std::pair<uint32_t, double>{16, 2100.0}, {8, 1340.0}, {4, 890.0}, {2, 656.0}})
+            if (n % t.first == 0) return n / t.first * t.second;
+        return n * 490.0;
+    };
+    uint32_t best = B;
+    for (uint32_t t : {2u, 4u, 8u, 16u}) {
+        const uint32_t n = (B + t - 1) / t * t;
+        if (cost(n) < cost(best)) best = n;
+    }
+    return best;
+}
+
 // Mirrors applied in the kernels (MLEM_FLAG_MIRROR_KERNELS), set up on a
 // context that holds the stored matrix: the detector maps of the identity
 // and the header's mirrors (generateSyms order), the device voxel maps, and
@@ -1479,7 +1537,7 @@ void mlem_destroy(mlem_ctx* c) {
                     (void*)c->hist_zeros, (void*)c->hist_subn, (void*)c->tmp_r[0],
                     (void*)c->tmp_r[1], (void*)c->tmp_c[0], (void*)c->tmp_c[1], (void*)c->tmp_c[2],
                     (void*)c->tmp_sino, (void*)c->tmp_d, (void*)c->norm_nat, (void*)c->perm,
-                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->row_order,
+                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->rscratch, (void*)c->row_order,
                     (void*)c->row_ranges, (void*)c->counter, (void*)c->long_segs, (void*)c->f_long_d,
                     (void*)c->sub_norm,
                     (void*)c->sub_file, (void*)c->sub_file_ranges, (void*)c->sub_sorted,
@@ -1612,7 +1670,7 @@ int mlem_calc_fwproj(mlem_ctx* c, const float* image, float* out) {
     CK(c, cudaMemcpyAsync(c->tmp_c[0], image, (size_t)c->C * 4, cudaMemcpyHostToDevice, c->stream));
     const float* xd = c->tmp_c[0];
     if (c->bricked) {
-        CK(c, permute_to_device(c->tmp_c[0], c->tmp_c[1], c->perm, c->C, 1, c->stream));
+        CK(c, permute_to_device(c->tmp_c[0], c->tmp_c[1], c->perm, c->C, 1, 1, c->stream));
         xd = c->tmp_c[1];
     }
     if (c->flags & MLEM_FLAG_EXACT) {
@@ -1664,7 +1722,7 @@ int mlem_calc_bkproj(mlem_ctx* c, const float* correl, float* update) {
         CK(c, cudaMemsetAsync(ud, 0, (size_t)c->C * 4, c->stream));
         CK(c, bkproj_scatter(csr_visit(c, c->tuning), c->tmp_r[0], 1, 0, ud, cfg_for_frames(c, 1), c->stream));
     }
-    if (c->bricked) CK(c, permute_to_natural(ud, c->tmp_c[0], c->perm, c->C, 1, c->stream));
+    if (c->bricked) CK(c, permute_to_natural(ud, c->tmp_c[0], c->perm, c->C, 1, 1, c->stream));
     CK(c, cudaMemcpyAsync(update, c->tmp_c[0], (size_t)c->C * 4, cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     return MLEM_OK;
@@ -2137,6 +2195,7 @@ int mlem_set_tuning(mlem_ctx* c, const mlem_tuning* t) {
         }
     }
     c->tuning = n;
+    c->tile_follows = false;
     c->graph_dirty = true;
     return MLEM_OK;
 }
@@ -2236,6 +2295,7 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
     if (!csc_by_visit(c, best) && c->celems_vis)  // tried, not chosen: give the memory back
         free_csc_vis(c);
     c->tuning = best;
+    c->tile_follows = false;
     c->graph_dirty = true;
     if (best_out) *best_out = best;
     return MLEM_OK;
@@ -2368,13 +2428,17 @@ int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* strea
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
+    uint32_t Bd = c->mirrored ? B : projection_stride(B);
+    if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
     const float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, st));
+    float* yd = y;
+    if (c->bricked || Bd != B) {
+        TRY(perm_scratch(c, (size_t)c->C * Bd));
+        CK(c, permute_to_device(x, c->pscratch[0], c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
         xd = c->pscratch[0];
+        if (Bd != B) yd = c->rscratch;
     }
-    const LaunchCfg cfg = cfg_for_frames(c, B);
+    const LaunchCfg cfg = cfg_for_frames(c, Bd);
     if (c->mirrored) {
         CK(c, cudaMemsetAsync(y, 0, (size_t)c->R * B * 4, st));
         for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
@@ -2382,34 +2446,44 @@ int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* strea
                                 c->n_sm, c->tuning.blocks_per_sm, st));
         return MLEM_OK;
     }
-    for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
-        CK(c, fwproj(csr_visit(c, c->tuning), xd, B, f0, nullptr, nullptr, y, cfg, st));
+    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile)
+        CK(c, fwproj(csr_visit(c, c->tuning), xd, Bd, f0, nullptr, nullptr, yd, cfg, st));
+    if (Bd != B) CK(c, permute_to_natural(yd, y, nullptr, c->R, B, Bd, st));
     return MLEM_OK;
 }
 
 int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
-    const LaunchCfg cfg = cfg_for_frames(c, B);
     cudaStream_t st = (cudaStream_t)stream;
+    // only the gather pass takes padded frames
+    uint32_t Bd = c->mirrored || !c->has_csc ? B : projection_stride(B);
+    if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
+    const LaunchCfg cfg = cfg_for_frames(c, Bd);
+    const float* yd = y;
     float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
+    if (c->bricked || Bd != B) {
+        TRY(perm_scratch(c, (size_t)c->C * Bd));
         xd = c->pscratch[0];
     }
-    for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile) {
+    if (Bd != B) {
+        CK(c, permute_to_device(y, c->rscratch, nullptr, c->R, B, Bd, st));
+        yd = c->rscratch;
+    }
+    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile) {
         if (c->mirrored) {
             if (f0 == 0) CK(c, cudaMemsetAsync(xd, 0, (size_t)c->C * B * 4, st));
             CK(c, mirror_bkproj(csr_visit(c, c->tuning), c->mirror, y, nullptr, B, f0,
                                 cfg.frame_tile, xd, c->n_sm, c->tuning.blocks_per_sm, st));
         } else if (c->has_csc) {
-            CK(c, bkproj_csc(csc_view(c), y, B, f0, nullptr, nullptr, xd, cfg, st));
+            CK(c, bkproj_csc(csc_view(c), yd, Bd, f0, nullptr, nullptr, xd, cfg, st));
         } else {
             if (f0 == 0) CK(c, cudaMemsetAsync(xd, 0, (size_t)c->C * B * 4, st));
             CK(c, bkproj_scatter(csr_visit(c, c->tuning), y, B, f0, xd, cfg, st));
         }
     }
-    if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, st));
+    if (xd != x)
+        CK(c, permute_to_natural(xd, x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
     return MLEM_OK;
 }
 
@@ -2421,7 +2495,7 @@ int mlem_fwproj_correl_d(mlem_ctx* c, const float* x, const int32_t* sino, float
     const float* xd = x;
     if (c->bricked) {
         TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, st));
+        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
         xd = c->pscratch[0];
     }
     const LaunchCfg cfg = cfg_for_frames(c, B);
@@ -2461,7 +2535,7 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
         float* ud = u;
         if (c->bricked) {
             TRY(perm_scratch(c, (size_t)c->C * B));
-            CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, st));
+            CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
             xd = c->pscratch[0];
             ud = c->pscratch[1];
         }
@@ -2481,7 +2555,7 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
         for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
             CK(c, mirror_bkproj(v, c->mirror, c->f_mirror_d, sino, B, f0, cfg.frame_tile, ud,
                                 c->n_sm, c->tuning.blocks_per_sm, st));
-        if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, st));
+        if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, B, st));
         return MLEM_OK;
     }
     // the context's one-pass tuning when it has one, else sorted rows in chunks
@@ -2498,7 +2572,7 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
     float* ud = u;
     if (c->bricked) {
         TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, st));
+        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
         xd = c->pscratch[0];
         ud = c->pscratch[1];
     }
@@ -2523,7 +2597,7 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
     if (c->n_long)
         CK(c, long_rows_pass(csr_view(c), c->long_segs, c->n_long_segs, c->n_long, xd, B,
                              t.frame_tile, sino, c->f_long_d, ud, c->n_sm, st));
-    if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, st));
+    if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, B, st));
     return MLEM_OK;
 }
 
@@ -2543,7 +2617,7 @@ static int backward_pass(mlem_ctx* c, int op, const float* x, const int32_t* sin
     float* ud = u;
     if (c->bricked) {
         TRY(perm_scratch(c, (size_t)c->C));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, 1, st));
+        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, 1, 1, st));
         xd = c->pscratch[0];
         ud = c->pscratch[1];
     }
@@ -2551,7 +2625,7 @@ static int backward_pass(mlem_ctx* c, int op, const float* x, const int32_t* sin
     // the counter slot of mlem_fused_update_d: these calls, like it, must not
     // run concurrently with the context's own iterations
     CK(c, adjoint_pass(op, csr_view(c), xd, sino, rows, ud, c->counter + 8, c->n_sm, st));
-    if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, 1, st));
+    if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, 1, 1, st));
     return MLEM_OK;
 }
 
@@ -2574,13 +2648,13 @@ int mlem_bkproj_update_d(mlem_ctx* c, const float* correl, float* x, uint32_t B,
     float* xd = x;
     if (c->bricked) {
         TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, st));
+        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
         xd = c->pscratch[0];
     }
     const LaunchCfg cfg = cfg_for_frames(c, B);
     for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
         CK(c, bkproj_csc(csc_view(c), correl, B, f0, c->norm, xd, nullptr, cfg, st));
-    if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, st));
+    if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, B, st));
     return MLEM_OK;
 }
 
@@ -2603,7 +2677,7 @@ int mlem_set_norm_d(mlem_ctx* c, const float* norm, void* stream) {
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     CK(c, cudaMemcpyAsync(c->norm_nat, norm, (size_t)c->C * 4, cudaMemcpyDeviceToDevice, st));
-    if (c->bricked) CK(c, permute_to_device(c->norm_nat, c->norm, c->perm, c->C, 1, st));
+    if (c->bricked) CK(c, permute_to_device(c->norm_nat, c->norm, c->perm, c->C, 1, 1, st));
     else CK(c, cudaMemcpyAsync(c->norm, norm, (size_t)c->C * 4, cudaMemcpyDeviceToDevice, st));
     CK(c, cudaMemcpyAsync(c->norm_host.data(), c->norm_nat, (size_t)c->C * 4,
                           cudaMemcpyDeviceToHost, st));
@@ -2625,7 +2699,7 @@ int mlem_project_f64(mlem_ctx* c, const float* x, double* out) {
     CK(c, cudaMemcpyAsync(c->tmp_c[0], x, (size_t)c->C * 4, cudaMemcpyHostToDevice, c->stream));
     const float* xd = c->tmp_c[0];
     if (c->bricked) {
-        CK(c, permute_to_device(c->tmp_c[0], c->tmp_c[1], c->perm, c->C, 1, c->stream));
+        CK(c, permute_to_device(c->tmp_c[0], c->tmp_c[1], c->perm, c->C, 1, 1, c->stream));
         xd = c->tmp_c[1];
     }
     CK(c, project_f64(csr_view(c), xd, c->tmp_d, c->stream));

@@ -58,6 +58,8 @@ struct mlem_ctx {
     std::vector<uint32_t> perm_host, iperm_host;
     float* pscratch[2] = {nullptr, nullptr};
     size_t pscratch_floats = 0;
+    float* rscratch = nullptr;  // row vectors with padded frames (projections)
+    size_t rscratch_floats = 0;
 
     // Visiting order of the row kernels (row_order_build): rays with nearby
     // entry and exit voxels next to each other.  Null with MLEM_FLAG_NO_ROW_ORDER.
@@ -170,6 +172,7 @@ struct mlem_ctx {
     size_t rb_bytes = 0;
 
     mlem_tuning tuning{};
+    bool tile_follows = true;  // no tuning chosen yet: the frame tile follows the frame count
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     bool graph_stats = false;  // the graph holds the census

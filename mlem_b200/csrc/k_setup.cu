@@ -382,15 +382,14 @@ __global__ void k_deinterleave(const T* __restrict__ in, T* __restrict__ out, ui
     }
 }
 
-template <bool TO_DEVICE>
+template <bool TO_DEVICE, typename I>
 __global__ void k_permute(const float* __restrict__ in, float* __restrict__ out,
-                          const uint32_t* __restrict__ perm, uint64_t n, uint32_t B) {
-    const uint64_t total = n * B;
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < total;
-         j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = j / B, b = j - i * B;
-        const uint64_t d = (uint64_t)perm[i] * B + b;
-        if (TO_DEVICE) out[d] = in[j];
+                          const uint32_t* __restrict__ perm, I n, uint32_t B, uint32_t Bd) {
+    const I S = TO_DEVICE ? Bd : B, total = n * S;
+    for (I j = blockIdx.x * (I)blockDim.x + threadIdx.x; j < total; j += (I)gridDim.x * blockDim.x) {
+        const I i = j / S, b = j - i * S;
+        const uint64_t d = (uint64_t)(perm ? perm[i] : i) * Bd + b;
+        if (TO_DEVICE) out[d] = b < B ? in[(uint64_t)i * B + b] : 0.0f;
         else out[j] = in[d];
     }
 }
@@ -646,18 +645,31 @@ cudaError_t deinterleave_f32(const float* in, float* out, uint64_t n, uint32_t B
     return cudaGetLastError();
 }
 
-cudaError_t permute_to_device(const float* in, float* out, const uint32_t* perm, uint64_t n,
-                              uint32_t B, cudaStream_t st) {
+namespace {
+template <bool TO_DEVICE>
+cudaError_t run_permute(const float* in, float* out, const uint32_t* perm, uint64_t n, uint32_t B,
+                        uint32_t Bd, cudaStream_t st) {
     if (n * B == 0) return cudaSuccess;
-    k_permute<true><<<elementwise_grid(n * B), 256, 0, st>>>(in, out, perm, n, B);
+    const uint64_t total = n * Bd;
+    // 32-bit indexes (a 64-bit division per value costs several times the copy)
+    // while the last index plus a stride fits
+    if (total < 0xf0000000ull)
+        k_permute<TO_DEVICE, uint32_t><<<elementwise_grid(total), 256, 0, st>>>(in, out, perm,
+                                                                               (uint32_t)n, B, Bd);
+    else
+        k_permute<TO_DEVICE, uint64_t><<<elementwise_grid(total), 256, 0, st>>>(in, out, perm, n, B, Bd);
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t permute_to_device(const float* in, float* out, const uint32_t* perm, uint64_t n,
+                              uint32_t B, uint32_t Bd, cudaStream_t st) {
+    return run_permute<true>(in, out, perm, n, B, Bd, st);
 }
 
 cudaError_t permute_to_natural(const float* in, float* out, const uint32_t* perm, uint64_t n,
-                               uint32_t B, cudaStream_t st) {
-    if (n * B == 0) return cudaSuccess;
-    k_permute<false><<<elementwise_grid(n * B), 256, 0, st>>>(in, out, perm, n, B);
-    return cudaGetLastError();
+                               uint32_t B, uint32_t Bd, cudaStream_t st) {
+    return run_permute<false>(in, out, perm, n, B, Bd, st);
 }
 
 cudaError_t remap_columns(uint2* elems, uint64_t nnz, const uint32_t* perm, cudaStream_t st) {

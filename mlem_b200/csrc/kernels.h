@@ -214,12 +214,14 @@ cudaError_t interleave_f32(const float* in, float* out, uint64_t n, uint32_t B, 
                            const uint32_t* perm, cudaStream_t st);
 cudaError_t deinterleave_f32(const float* in, float* out, uint64_t n, uint32_t B, uint32_t Bp,
                              const uint32_t* perm, cudaStream_t st);
-// Interleaved [n][B] vectors between natural and device voxel order:
-// to_device: out[perm[i]*B + b] = in[i*B + b]; to_natural: out[i*B + b] = in[perm[i]*B + b].
+// Interleaved [n][B] vectors between natural and device voxel order, the device
+// vector with Bd >= B floats per voxel: to_device: out[p(i)*Bd + b] =
+// in[i*B + b] for b < B, 0 for the other b; to_natural: out[i*B + b] =
+// in[p(i)*Bd + b] for b < B.  p = perm, or the identity when perm is null.
 cudaError_t permute_to_device(const float* in, float* out, const uint32_t* perm, uint64_t n,
-                              uint32_t B, cudaStream_t st);
+                              uint32_t B, uint32_t Bd, cudaStream_t st);
 cudaError_t permute_to_natural(const float* in, float* out, const uint32_t* perm, uint64_t n,
-                               uint32_t B, cudaStream_t st);
+                               uint32_t B, uint32_t Bd, cudaStream_t st);
 // Relabel the column (voxel) index of every element: e.x = perm[e.x].
 cudaError_t remap_columns(uint2* elems, uint64_t nnz, const uint32_t* perm, cudaStream_t st);
 // x[i][b] = b < B ? vals[b] : 0 for the Bp-interleaved image (vals: device, B floats).

@@ -1,6 +1,6 @@
 """The gather passes (forward projection over rows, back projection over
-columns) at the sizes where their batches, lane groups and lane rule turn
-over: rows and columns of 0, 1 and batch +- 1 elements, few long columns, many
+columns) at the sizes where their batches, lane groups, lane rule and padded
+frames turn over: rows and columns of 0, 1 and batch +- 1 elements, few long columns, many
 short rows, one row far longer than the rest, and caller vectors on 4-, 8- and
 16-byte boundaries, for every group and frame tile.  Every sum must lie within
 the rounding of a float sum of its products: n 2^-23 sum |v x|."""
@@ -31,7 +31,7 @@ def matrix(kind, rng):
     if kind == "one-long":
         el["index"][rng.random(el.size) < 0.3] = 4
     el["value"] = rng.uniform(-1.0, 1.7, el.size)
-    return formats.Csr4(R, C, end, el)
+    return formats.Csr4(R, C, end, el, grid=(30, 40, 25) if kind == "many-rows" else (0, 0, 0))
 
 
 def sums(m, x, transpose):
@@ -53,14 +53,14 @@ def test_gather_passes_against_float64(kind):
     m = matrix(kind, rng)
     st = torch.cuda.current_stream().cuda_stream
     with api.Context.from_matrix(m) as ctx:
-        for B in (1, 2, 4, 8, 16, 3):
+        for B in (1, 2, 4, 8, 16, 3, 5, 12, 18):
             x, y = (rng.uniform(0.1, 1.0, (n, B)).astype(np.float32) for n in (m.n_cols, m.n_rows))
             want = {"fw": sums(m, x, False), "bk": sums(m, y, True)}
             for group in (4, 8, 16, 32):
                 ctx.set_tuning(bk_mode=api.BK_CSC, group=group, frame_tile=1, blocks_per_sm=8)
                 # the vectors `shift` floats past a 512-byte boundary: any float boundary at one
                 # frame, 8 bytes at two and 16 at more
-                for shift in (0, 1 if B in (1, 3) else 2 if B == 2 else 4):
+                for shift in (0, 1 if B % 2 else 2 if B % 4 else 4):
                     for way, src, n, call in (("fw", x, m.n_rows, ctx.fwproj_d), ("bk", y, m.n_cols, ctx.bkproj_d)):
                         a = torch.zeros(src.size + shift, device="cuda")
                         a[shift:] = torch.from_numpy(src.reshape(-1)).cuda()
@@ -69,3 +69,27 @@ def test_gather_passes_against_float64(kind):
                         got = o[shift:].cpu().numpy().reshape(n, B)
                         ref, mag, cnt = want[way]
                         assert np.all(np.abs(got - ref) <= 2.0 ** -23 * (cnt + 1) * mag), (way, B, group, shift)
+
+
+def test_default_frame_tile_follows_the_frames():
+    """Without a chosen tuning the frame tile is the widest one of the frame
+    count; a chosen one stays."""
+    rng = np.random.default_rng(3)
+    m = matrix("many-rows", rng)
+    m.elems["value"] = np.abs(m.elems["value"])
+    sino = rng.poisson(5, (5, m.n_rows)).astype(np.int32)
+    imgs = []
+    for tile in (None, 1):
+        with api.Context.from_matrix(m) as ctx:
+            ctx.set_sinograms(sino)
+            assert ctx.tuning()["frame_tile"] == 8
+            if tile:
+                ctx.set_tuning(api.BK_CSC, 32, tile, 8)
+            ctx.set_sinograms(sino[:1])
+            assert ctx.tuning()["frame_tile"] == 1
+            ctx.set_sinograms(sino)
+            assert ctx.tuning()["frame_tile"] == (tile or 8)
+            ctx.init_images()
+            ctx.iterate(4)
+            imgs.append(ctx.get_images().astype(np.float64))
+    assert np.linalg.norm(imgs[0] - imgs[1]) <= 1e-5 * np.linalg.norm(imgs[1])
