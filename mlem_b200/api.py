@@ -285,7 +285,7 @@ class Context:
         return sums, zeros, subn
 
     def get_images(self) -> np.ndarray:
-        out = np.zeros((self.n_frames, self.n_cols), np.float32)
+        out = np.empty((self.n_frames, self.n_cols), np.float32)  # written whole, or the call raises
         self._chk(core_lib().mlem_get_images(self._h, _p(out)))
         return out
 

@@ -540,6 +540,123 @@ int new_ctx(mlem_ctx** out, uint32_t R, uint32_t C, uint64_t Z, uint32_t flags, 
 }
 
 // ---------------------------------------------------------------------------
+// Host copies.  A copy between a caller's pageable array and the device goes,
+// from kStagedCopy bytes on, through page-locked slots of the context, kept
+// between calls: host threads, each with two slots, move 256 KiB pieces between
+// the slots and the array while the copy engine works on their other slots, so
+// the array's page faults (a result array is fresh memory) and copies run on
+// several cores: 16 images of 1,048,576 voxels into a fresh array 5.7 ms, 14.5
+// by one cudaMemcpyAsync.  Arrays below 32 MiB mostly come from memory the
+// process has touched before, where one copy is as fast (4 MiB 0.28 ms either way).
+// Page-locked arrays, small ones and hosts without page-locked memory to spare
+// take one plain cudaMemcpyAsync.  The caller synchronises the stream before it
+// lets go of the array.
+// ---------------------------------------------------------------------------
+constexpr size_t kSlotBytes = size_t(256) << 10;
+constexpr int kSlotThreads = 6, kSlots = 2 * kSlotThreads;
+constexpr size_t kStagedCopy = size_t(32) << 20;
+
+bool ensure_slots(mlem_ctx* c) {
+    if (c->slots) return true;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&c->slots), kSlots * kSlotBytes, cudaHostAllocDefault) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        c->slots = nullptr;
+        return false;
+    }
+    try {
+        c->slot_ev.assign(kSlots, nullptr);
+    } catch (...) {
+        c->slot_ev.clear();
+    }
+    bool ok = c->slot_ev.size() == kSlots;
+    for (cudaEvent_t& e : c->slot_ev)
+        if (ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) ok = false;
+    if (!ok) {
+        cudaGetLastError();
+        for (cudaEvent_t e : c->slot_ev)
+            if (e) cudaEventDestroy(e);
+        c->slot_ev.clear();
+        cudaFreeHost(c->slots);
+        c->slots = nullptr;
+    }
+    return ok;
+}
+
+cudaError_t copy_pageable(mlem_ctx* c, void* host, void* dev, size_t bytes, bool to_host) {
+    auto plain = [&]() {
+        return to_host ? cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream)
+                       : cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream);
+    };
+    const int T = (int)std::min<size_t>({(size_t)kSlotThreads, (size_t)std::thread::hardware_concurrency(),
+                                         bytes / (2 * kSlotBytes)});
+    if (bytes < kStagedCopy || T < 2) return plain();
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
+    else if (at.type != cudaMemoryTypeUnregistered) return plain();
+    if (!ensure_slots(c)) return plain();
+    const size_t n = (bytes + kSlotBytes - 1) / kSlotBytes;
+    unsigned char* h = static_cast<unsigned char*>(host);
+    unsigned char* d = static_cast<unsigned char*>(dev);
+    std::mutex enqueue;
+    std::atomic<int> bad{0};  // the first failure's cudaError_t
+    // thread t takes pieces t, t + T, ...; its j-th piece uses slot 2t + (j & 1)
+    auto worker = [&](int t) {
+        cudaError_t e = cudaSetDevice(c->device);
+        auto piece = [&](size_t i, size_t& off, size_t& len) {
+            off = i * kSlotBytes;
+            len = std::min(kSlotBytes, bytes - off);
+        };
+        size_t off = 0, len = 0, j = 0;
+        for (size_t i = (size_t)t; e == cudaSuccess && i < n && !bad.load(); i += (size_t)T, ++j) {
+            const int b = 2 * t + (int)(j & 1);
+            unsigned char* slot = c->slots + (size_t)b * kSlotBytes;
+            piece(i, off, len);
+            if (!to_host) {
+                if (j >= 2) e = cudaEventSynchronize(c->slot_ev[b]);  // the slot's last piece has left
+                if (e != cudaSuccess) break;
+                std::memcpy(slot, h + off, len);
+            }
+            {
+                std::lock_guard<std::mutex> g(enqueue);
+                e = to_host ? cudaMemcpyAsync(slot, d + off, len, cudaMemcpyDeviceToHost, c->stream)
+                            : cudaMemcpyAsync(d + off, slot, len, cudaMemcpyHostToDevice, c->stream);
+                if (e == cudaSuccess) e = cudaEventRecord(c->slot_ev[b], c->stream);
+            }
+            if (to_host && e == cudaSuccess && j >= 1) {  // the piece before, while this one arrives
+                const int pb = 2 * t + (int)((j - 1) & 1);
+                e = cudaEventSynchronize(c->slot_ev[pb]);
+                piece(i - (size_t)T, off, len);
+                if (e == cudaSuccess) std::memcpy(h + off, c->slots + (size_t)pb * kSlotBytes, len);
+            }
+        }
+        if (to_host && e == cudaSuccess && j >= 1 && !bad.load()) {  // the thread's last piece
+            const int pb = 2 * t + (int)((j - 1) & 1);
+            e = cudaEventSynchronize(c->slot_ev[pb]);
+            piece((size_t)t + (j - 1) * (size_t)T, off, len);
+            if (e == cudaSuccess) std::memcpy(h + off, c->slots + (size_t)pb * kSlotBytes, len);
+        }
+        if (e != cudaSuccess) {
+            int none = 0;
+            bad.compare_exchange_strong(none, (int)e);
+        }
+    };
+    std::vector<std::thread> pool;
+    int started = 1;  // the calling thread is worker 0
+    try {
+        pool.reserve((size_t)T);
+        for (; started < T; ++started) pool.emplace_back(worker, started);
+    } catch (...) {  // no more threads: the calling thread takes the rest
+    }
+    worker(0);
+    for (int t = started; t < T; ++t) worker(t);
+    for (std::thread& th : pool) th.join();
+    const cudaError_t e = static_cast<cudaError_t>(bad.load());
+    const cudaError_t es = cudaStreamSynchronize(c->stream);  // the slots are in use until here
+    return e != cudaSuccess ? e : es;
+}
+
+// ---------------------------------------------------------------------------
 // Frames.
 // ---------------------------------------------------------------------------
 int ensure_stage(mlem_ctx* c, size_t bytes) {
@@ -554,14 +671,14 @@ int ensure_stage(mlem_ctx* c, size_t bytes) {
 
 void free_frames(mlem_ctx* c) {
     for (void* p : {(void*)c->sino, (void*)c->x, (void*)c->correl, (void*)c->update,
-                    (void*)c->stats_scratch, (void*)c->inits_dev, (void*)c->f_long,
+                    (void*)c->stats_scratch, (void*)c->f_long,
                     (void*)c->sino_alt})
         dev_free(p);
     if (c->graph_alt) cudaGraphExecDestroy(c->graph_alt);
     c->graph_alt = nullptr;
     c->sino_alt = nullptr;
     c->sino = nullptr; c->x = nullptr; c->correl = nullptr; c->update = nullptr;
-    c->stats_scratch = nullptr; c->inits_dev = nullptr; c->f_long = nullptr;
+    c->stats_scratch = nullptr; c->f_long = nullptr;
     c->B = c->Bp = 0;
     c->images_ready = false;
     c->act_ready = false;
@@ -580,7 +697,6 @@ int alloc_frames(mlem_ctx* c, uint32_t B) {
     TRY(dev_alloc(c, &c->update, (size_t)c->C * Bp));
     TRY(dev_alloc(c, &c->stats_scratch, stats_scratch_bytes(Bp)));
     CK(c, cudaMemsetAsync(c->stats_scratch, 0, stats_scratch_bytes(Bp), c->stream));
-    TRY(dev_alloc(c, &c->inits_dev, Bp));
     if (c->n_long) TRY(dev_alloc(c, &c->f_long, (size_t)c->n_long * Bp));
     CK(c, cudaMemsetAsync(c->sino, 0, (size_t)c->R * Bp * 4, c->stream));
     CK(c, cudaMemsetAsync(c->x, 0, (size_t)c->C * Bp * 4, c->stream));
@@ -597,16 +713,28 @@ int alloc_frames(mlem_ctx* c, uint32_t B) {
     return MLEM_OK;
 }
 
+// mlem_ctx::pin and its parts (in words); null where no page-locked memory can
+// be had, and the results are copied one by one.
+constexpr size_t kPinActive = 128, kPinCensus = 136, kPinWords = kPinCensus + 3 * 64 * 64;
+unsigned long long* pinned(mlem_ctx* c) {
+    if (!c->pin &&
+        cudaHostAlloc(reinterpret_cast<void**>(&c->pin), kPinWords * 8, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->pin = nullptr;
+    }
+    return c->pin;
+}
+
 // Frame-major host [B][n] -> interleaved device [n][Bp] (pad frames untouched).
 template <typename T>
 int upload_frames(mlem_ctx* c, const T* host, T* dev, uint64_t n) {
     const bool voxels = std::is_same<T, float>::value && c->bricked;
     if (c->Bp == 1 && !voxels) {
-        CK(c, cudaMemcpyAsync(dev, host, n * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+        CK(c, copy_pageable(c, const_cast<T*>(host), dev, n * sizeof(T), false));
         return MLEM_OK;
     }
     TRY(ensure_stage(c, n * c->B * sizeof(T)));
-    CK(c, cudaMemcpyAsync(c->stage, host, n * c->B * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+    CK(c, copy_pageable(c, const_cast<T*>(host), c->stage, n * c->B * sizeof(T), false));
     if (std::is_same<T, int32_t>::value)
         CK(c, interleave_i32(reinterpret_cast<const int32_t*>(c->stage),
                              reinterpret_cast<int32_t*>(dev), n, c->B, c->Bp, c->stream));
@@ -619,13 +747,13 @@ int upload_frames(mlem_ctx* c, const T* host, T* dev, uint64_t n) {
 
 int download_images(mlem_ctx* c, float* host) {
     if (c->Bp == 1 && !c->bricked) {
-        CK(c, cudaMemcpyAsync(host, c->x, (size_t)c->C * 4, cudaMemcpyDeviceToHost, c->stream));
+        CK(c, copy_pageable(c, host, c->x, (size_t)c->C * 4, true));
         return MLEM_OK;
     }
     TRY(ensure_stage(c, (size_t)c->C * c->B * 4));
     float* st = static_cast<float*>(c->stage);
     CK(c, deinterleave_f32(c->x, st, c->C, c->B, c->Bp, c->bricked ? c->perm : nullptr, c->stream));
-    CK(c, cudaMemcpyAsync(host, st, (size_t)c->C * c->B * 4, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, copy_pageable(c, host, st, (size_t)c->C * c->B * 4, true));
     return MLEM_OK;
 }
 
@@ -661,13 +789,14 @@ int build_active_list(mlem_ctx* c, bool read_back, bool cut) {
                             c->act_tmp_bytes, c->act_order, c->act_ranges, c->act_n, c->act_z,
                             c->stream));
     if (read_back) {
-        uint32_t n = 0;
-        unsigned long long z = 0;
-        CK(c, cudaMemcpyAsync(&n, c->act_n, 4, cudaMemcpyDeviceToHost, c->stream));
-        CK(c, cudaMemcpyAsync(&z, c->act_z, 8, cudaMemcpyDeviceToHost, c->stream));
+        unsigned long long here[2] = {0, 0};
+        unsigned long long* to = pinned(c) ? c->pin + kPinActive : here;
+        to[0] = 0;
+        CK(c, cudaMemcpyAsync(to, c->act_n, 4, cudaMemcpyDeviceToHost, c->stream));
+        CK(c, cudaMemcpyAsync(to + 1, c->act_z, 8, cudaMemcpyDeviceToHost, c->stream));
         CK(c, cudaStreamSynchronize(c->stream));
-        c->act_rows = n;
-        c->act_nnz = z;
+        c->act_rows = (uint32_t)to[0];
+        c->act_nnz = to[1];
     }
     c->act_ready = true;
     return cut ? build_csc_act(c, c->tuning) : MLEM_OK;
@@ -1549,6 +1678,11 @@ void mlem_destroy(mlem_ctx* c) {
                     (void*)c->act_ranges_alt, (void*)c->act_n_alt, (void*)c->act_z_alt})
         dev_free(p);
     if (c->act_host) cudaFreeHost(c->act_host);
+    if (c->pin) cudaFreeHost(c->pin);
+    dev_free(c->count_sums);
+    for (cudaEvent_t e : c->slot_ev)
+        if (e) cudaEventDestroy(e);
+    if (c->slots) cudaFreeHost(c->slots);
     for (cudaStream_t q : {c->up_stream, c->down_stream})
         if (q) { cudaStreamSynchronize(q); cudaStreamDestroy(q); }
     for (int i = 0; i < 2; ++i) {
@@ -1747,17 +1881,30 @@ int mlem_set_sinograms(mlem_ctx* c, const int32_t* sino, uint32_t B) {
     if (!c || !sino) return fail(c, MLEM_ERR_INVALID, "null argument");
     TRY(set_device(c));
     TRY(alloc_frames(c, B));
+    TRY(upload_frames<int32_t>(c, sino, c->sino, c->R));
+    // initImage's sums of the counts (seqcsr4mlem.cpp:57-58: double, in row
+    // order).  Whole numbers whose magnitudes sum to at most 2^53 add exactly in
+    // any order, so the device adds them as integers; beyond that the host adds
+    // them as the reference does.
+    if (!c->count_sums) TRY(dev_alloc(c, &c->count_sums, 128));
+    CK(c, count_sums(c->sino, c->R, c->Bp, c->count_sums, c->count_sums + 64, c->stream));
+    unsigned long long here[128];
+    unsigned long long* sums = pinned(c) ? c->pin : here;
+    CK(c, cudaMemcpyAsync(sums, c->count_sums, sizeof(here), cudaMemcpyDeviceToHost, c->stream));
+    TRY(build_active(c, true, true));
+    ++c->sino_gen;
+    CK(c, cudaStreamSynchronize(c->stream));
     c->sumin.assign(B, 0.0);
     for (uint32_t b = 0; b < B; ++b) {
-        double s = 0.0;  // seqcsr4mlem.cpp:57-58
+        if (sums[64 + b] <= (1ull << 53)) {
+            c->sumin[b] = (double)(long long)sums[b];
+            continue;
+        }
+        double s = 0.0;
         const int32_t* p = sino + (size_t)b * c->R;
         for (uint32_t i = 0; i < c->R; ++i) s += p[i];
         c->sumin[b] = s;
     }
-    TRY(upload_frames<int32_t>(c, sino, c->sino, c->R));
-    TRY(build_active(c, true, true));
-    ++c->sino_gen;
-    CK(c, cudaStreamSynchronize(c->stream));
     c->images_ready = false;
     return MLEM_OK;
 }
@@ -1766,12 +1913,11 @@ int mlem_init_images(mlem_ctx* c, float* initial) {
     if (!c) return fail(nullptr, MLEM_ERR_INVALID, "null context");
     if (!c->B) return fail(c, MLEM_ERR_STATE, "mlem_set_sinograms must come first");
     TRY(set_device(c));
-    std::vector<float> init(c->Bp, 0.0f);
-    for (uint32_t b = 0; b < c->B; ++b) init[b] = (float)(c->sumin[b] / c->sumnorm);
-    CK(c, cudaMemcpyAsync(c->inits_dev, init.data(), c->Bp * 4, cudaMemcpyHostToDevice, c->stream));
-    CK(c, fill_frames(c->x, c->C, c->Bp, c->B, c->inits_dev, c->stream));
+    FrameValues init{};
+    for (uint32_t b = 0; b < c->B; ++b) init.v[b] = (float)(c->sumin[b] / c->sumnorm);
+    CK(c, fill_frames(c->x, c->C, c->Bp, init, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    if (initial) std::memcpy(initial, init.data(), c->B * 4);
+    if (initial) std::memcpy(initial, init.v, c->B * 4);
     c->images_ready = true;
     return MLEM_OK;
 }
@@ -1809,14 +1955,19 @@ int mlem_iterate(mlem_ctx* c, int n, double* sums, uint64_t* zeros, uint64_t* su
             if (stats) CK(c, cudaMemsetAsync(c->stats_slot, 0, 4, c->stream));
             for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, c->tuning, stats));
         }
-        const size_t cnt = (size_t)k * c->B;
-        if (sums) CK(c, cudaMemcpyAsync(sums + (size_t)done * c->B, c->hist_sums, cnt * 8,
-                                        cudaMemcpyDeviceToHost, c->stream));
-        if (zeros) CK(c, cudaMemcpyAsync(zeros + (size_t)done * c->B, c->hist_zeros, cnt * 8,
-                                         cudaMemcpyDeviceToHost, c->stream));
-        if (subn) CK(c, cudaMemcpyAsync(subn + (size_t)done * c->B, c->hist_subn, cnt * 8,
-                                        cudaMemcpyDeviceToHost, c->stream));
-        if (sums || zeros || subn) CK(c, cudaStreamSynchronize(c->stream));
+        // the census of the chunk: through page-locked memory, one wait for all of it
+        const size_t cnt = (size_t)k * c->B, part = (size_t)64 * 64;
+        struct { void* host; const void* dev; } out[3] = {{sums ? sums + (size_t)done * c->B : nullptr, c->hist_sums},
+                                                          {zeros ? zeros + (size_t)done * c->B : nullptr, c->hist_zeros},
+                                                          {subn ? subn + (size_t)done * c->B : nullptr, c->hist_subn}};
+        unsigned long long* pin = stats ? pinned(c) : nullptr;
+        for (int q = 0; q < 3; ++q)
+            if (out[q].host)
+                CK(c, cudaMemcpyAsync(pin ? (void*)(pin + kPinCensus + q * part) : out[q].host, out[q].dev,
+                                      cnt * 8, cudaMemcpyDeviceToHost, c->stream));
+        if (stats) CK(c, cudaStreamSynchronize(c->stream));
+        for (int q = 0; q < 3 && pin; ++q)
+            if (out[q].host) std::memcpy(out[q].host, pin + kPinCensus + q * part, cnt * 8);
         done += k;
     }
     CK(c, cudaStreamSynchronize(c->stream));

@@ -139,9 +139,16 @@ __device__ __forceinline__ void pdl_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Worth it where kernels are short.  After a long kernel the early blocks only
+// hold the SMs' free slots while its last blocks run, which another stream's
+// kernels could use (the streamed iterations build the next list of rows in that
+// time: 2,097,152 rows, 8 steps 7.89 ms with dependent launches, 7.74 without);
+// so rows, columns or values beyond kDependentMost are launched the plain way.
+constexpr uint64_t kDependentMost = 1ull << 18;
+
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
-                                    cudaStream_t st, A... args) {
+inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, int threads,
+                                    size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
@@ -151,7 +158,7 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 

@@ -120,6 +120,15 @@ struct mlem_ctx {
     float* x = nullptr;
     float* correl = nullptr;
     float* update = nullptr;
+    unsigned long long* count_sums = nullptr;  // 2 x 64: sums and magnitudes of the frames' counts
+    // Page-locked memory the small results of a call arrive in, so that one
+    // synchronisation waits for all of them: the frames' count sums (128 words),
+    // act_n and act_z, then the census of up to 64 iterations.
+    unsigned long long* pin = nullptr;
+    // Page-locked slots of the host copies (copy_pageable) and their events,
+    // made by the first large copy: kSlots x kSlotBytes.
+    unsigned char* slots = nullptr;
+    std::vector<cudaEvent_t> slot_ev;
     void* stage = nullptr;  // staging for frame-major <-> interleaved copies
     size_t stage_bytes = 0;
     // mlem_stream_host: an upload and a download stream, double-buffered
@@ -155,7 +164,6 @@ struct mlem_ctx {
     float* tmp_c[3] = {nullptr, nullptr, nullptr};
     int32_t* tmp_sino = nullptr;
     double* tmp_d = nullptr;
-    float* inits_dev = nullptr;
 
     // Mirrors applied in the kernels (MLEM_FLAG_MIRROR_KERNELS): the matrix
     // arrays hold the stored elements only; norm holds the full matrix's

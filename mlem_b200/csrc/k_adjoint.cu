@@ -122,7 +122,7 @@ cudaError_t adjoint_pass(int op, const SparseView& csr, const float* x, const in
     const auto kernel = op == kOpRatio
                             ? (sorted ? k_adjoint_chunked<kOpRatio, true> : k_adjoint_chunked<kOpRatio, false>)
                             : (sorted ? k_adjoint_chunked<kOpAdjoint, true> : k_adjoint_chunked<kOpAdjoint, false>);
-    return launch_dependent(kernel, grid, 256, 0, st, csr, x, sino, rows, u, chunk, counter);
+    return launch_dependent(csr.n <= kDependentMost, kernel, grid, 256, 0, st, csr, x, sino, rows, u, chunk, counter);
 }
 
 }  // namespace mlem

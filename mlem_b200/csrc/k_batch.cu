@@ -101,7 +101,7 @@ cudaError_t launch_batch_staged(const BatchTable& t, const BatchItem* items, uin
     cudaError_t e = cudaFuncSetAttribute(k_batch_staged<BT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_batch_staged<BT>, grid, kBatchThreads, smem, st, t, items, n_items,
+    return launch_dependent(true, k_batch_staged<BT>, grid, kBatchThreads, smem, st, t, items, n_items,
                             counter);
 }
 
@@ -177,22 +177,22 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
     // the resident CTAs: 64 registers x 1024 threads per SM, in 1, 2 or 4 CTAs
     const int grid = std::max(1, sm_count * ctas_per_sm), threads = 1024 / ctas_per_sm;
     switch (frame_tile) {
-        case 1: return launch_dependent(k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
-        case 2: return launch_dependent(k_fused_chunked<2>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
-        case 4: return launch_dependent(k_fused_chunked<4>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
-        case 8: return launch_dependent(k_fused_chunked<8>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
-        case 16: return launch_dependent(k_fused_chunked<16>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 1: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 2: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<2>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 4: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<4>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 8: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<8>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
+        case 16: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<16>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
         default: return cudaErrorInvalidValue;
     }
 }
 
 #define MLEM_BATCH_TILES(KERNEL, ...)                                                               \
     switch (frame_tile) {                                                                           \
-        case 1: return launch_dependent(sorted ? KERNEL<1, true> : KERNEL<1, false>, __VA_ARGS__);  \
-        case 2: return launch_dependent(sorted ? KERNEL<2, true> : KERNEL<2, false>, __VA_ARGS__);  \
-        case 4: return launch_dependent(sorted ? KERNEL<4, true> : KERNEL<4, false>, __VA_ARGS__);  \
-        case 8: return launch_dependent(sorted ? KERNEL<8, true> : KERNEL<8, false>, __VA_ARGS__);  \
-        case 16: return launch_dependent(sorted ? KERNEL<16, true> : KERNEL<16, false>, __VA_ARGS__); \
+        case 1: return launch_dependent(true, sorted ? KERNEL<1, true> : KERNEL<1, false>, __VA_ARGS__);  \
+        case 2: return launch_dependent(true, sorted ? KERNEL<2, true> : KERNEL<2, false>, __VA_ARGS__);  \
+        case 4: return launch_dependent(true, sorted ? KERNEL<4, true> : KERNEL<4, false>, __VA_ARGS__);  \
+        case 8: return launch_dependent(true, sorted ? KERNEL<8, true> : KERNEL<8, false>, __VA_ARGS__);  \
+        case 16: return launch_dependent(true, sorted ? KERNEL<16, true> : KERNEL<16, false>, __VA_ARGS__); \
         default: return cudaErrorInvalidValue;                                                      \
     }
 

@@ -277,15 +277,15 @@ MLEM_KERNEL_FUNCTOR(ScatterK, k_bkproj_scatter)
 template <int G, int BT>
 struct FusedK {  // file order
     template <typename... A>
-    static void run(int grid, cudaStream_t st, A... a) {
-        launch_dependent(k_fused_row<G, BT, false>, grid, 256, 0, st, a...);
+    static void run(int grid, cudaStream_t st, const SparseView& csr, A... a) {
+        launch_dependent(csr.n <= kDependentMost, k_fused_row<G, BT, false>, grid, 256, 0, st, csr, a...);
     }
 };
 template <int G, int BT>
 struct FusedSortedK {  // sorted visiting order (csr.order + csr.vrange)
     template <typename... A>
-    static void run(int grid, cudaStream_t st, A... a) {
-        launch_dependent(k_fused_row<G, BT, true>, grid, 256, 0, st, a...);
+    static void run(int grid, cudaStream_t st, const SparseView& csr, A... a) {
+        launch_dependent(csr.n <= kDependentMost, k_fused_row<G, BT, true>, grid, 256, 0, st, csr, a...);
     }
 };
 #undef MLEM_KERNEL_FUNCTOR
@@ -346,7 +346,7 @@ cudaError_t apply_update(float* x, float* u, const float* norm, uint32_t C, uint
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    return launch_dependent(B == 1 ? k_apply_update<true> : k_apply_update<false>, grid, 256, 0, st, x,
+    return launch_dependent(n <= kDependentMost, B == 1 ? k_apply_update<true> : k_apply_update<false>, grid, 256, 0, st, x,
                             u, norm, n, B, zero_u);
 }
 
@@ -355,7 +355,7 @@ cudaError_t apply_update_subset(float* x, float* u, const float* norm_s, const f
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    return launch_dependent(B == 1 ? k_apply_update_subset<true> : k_apply_update_subset<false>, grid,
+    return launch_dependent(true, B == 1 ? k_apply_update_subset<true> : k_apply_update_subset<false>, grid,
                             256, 0, st, x, u, norm_s, norm, n, B);
 }
 

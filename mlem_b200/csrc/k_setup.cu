@@ -341,14 +341,14 @@ __global__ void k_stats_final(const double* __restrict__ ps, const unsigned long
     stats_finish(ps, pz, pn, nblocks, B, n_out, out);
 }
 
-__global__ void k_fill_frames(float* __restrict__ x, uint64_t n, uint32_t Bp, uint32_t B,
-                              const float* __restrict__ vals) {
-    const uint64_t total = n * Bp;
+__global__ void k_fill_frames(float* __restrict__ x, uint64_t total, uint32_t Bp,
+                              const FrameValues vals) {
+    __shared__ float v[64];
+    if (threadIdx.x < 64) v[threadIdx.x] = vals.v[threadIdx.x];
+    __syncthreads();
     for (uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; o < total;
-         o += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = (uint32_t)(o % Bp);
-        x[o] = b < B ? vals[b] : 0.0f;
-    }
+         o += (uint64_t)gridDim.x * blockDim.x)
+        x[o] = v[o % Bp];
 }
 
 __global__ void k_correl(const float* __restrict__ f, const int32_t* __restrict__ s,
@@ -356,6 +356,47 @@ __global__ void k_correl(const float* __restrict__ f, const int32_t* __restrict_
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
         c[i] = correl_of(s[i], f[i]);
+}
+
+// Whole-number sums of every frame's counts, and of their magnitudes, over the
+// interleaved sinogram: a thread keeps to one frame (the grid's threads are a
+// multiple of Bp), blocks add in shared memory, then one atomic per block and
+// frame.  Integer sums, so their order does not matter.
+__global__ void k_count_sums(const int32_t* __restrict__ s, uint64_t total, uint32_t Bp,
+                             unsigned long long* __restrict__ sums,
+                             unsigned long long* __restrict__ mags) {
+    __shared__ unsigned long long ss[64], sm[64];
+    for (uint32_t f = threadIdx.x; f < Bp; f += blockDim.x) ss[f] = sm[f] = 0ull;
+    __syncthreads();
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    long long a = 0;
+    unsigned long long m = 0;
+#pragma unroll 4
+    for (uint64_t i = t; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const long long v = s[i];
+        a += v;
+        m += (unsigned long long)(v < 0 ? -v : v);
+    }
+    // lanes of one frame first where a warp holds them
+    const uint32_t f = (uint32_t)(t % Bp);
+    if (Bp <= 16) {
+        for (uint32_t o = 16; o >= Bp; o >>= 1) {
+            a += __shfl_xor_sync(MLEM_FULL_MASK, a, o);
+            m += __shfl_xor_sync(MLEM_FULL_MASK, m, o);
+        }
+        if ((threadIdx.x & 31) < Bp) {
+            atomicAdd(&ss[f], (unsigned long long)a);
+            atomicAdd(&sm[f], m);
+        }
+    } else {
+        atomicAdd(&ss[f], (unsigned long long)a);
+        atomicAdd(&sm[f], m);
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < Bp; k += blockDim.x) {
+        if (ss[k]) atomicAdd(&sums[k], ss[k]);
+        if (sm[k]) atomicAdd(&mags[k], sm[k]);
+    }
 }
 
 template <typename T>
@@ -594,13 +635,14 @@ cudaError_t run_stats(const float* x, uint32_t C, uint32_t B, uint32_t n_out, bo
     const uint32_t nb = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>(kStatsBlocks, ceil_div(items, (uint64_t)kStatsThreads * 4)));
     const dim3 grid(nb, B / V);
+    const bool early = (uint64_t)C * B <= kDependentMost;
     if (one_launch)
-        return launch_dependent(k_stats<V, true>, grid, kStatsThreads, 0, st, x, C, B, ps, pz, pn,
+        return launch_dependent(early, k_stats<V, true>, grid, kStatsThreads, 0, st, x, C, B, ps, pz, pn,
                                 ticket, n_out, out);
-    cudaError_t e = launch_dependent(k_stats<V, false>, grid, kStatsThreads, 0, st, x, C, B, ps, pz, pn,
+    cudaError_t e = launch_dependent(early, k_stats<V, false>, grid, kStatsThreads, 0, st, x, C, B, ps, pz, pn,
                                      ticket, n_out, out);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_stats_final, 1, 512, 0, st, ps, pz, pn, nb, B, n_out, out);
+    return launch_dependent(early, k_stats_final, 1, 512, 0, st, ps, pz, pn, nb, B, n_out, out);
 }
 }  // namespace
 
@@ -622,6 +664,18 @@ cudaError_t image_stats(const float* x, uint32_t C, uint32_t B, uint32_t n_out, 
 
 static unsigned elementwise_grid(uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 256), kB200SMs * 16));
+}
+
+cudaError_t count_sums(const int32_t* sino, uint64_t R, uint32_t Bp, unsigned long long* sums,
+                       unsigned long long* mags, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(sums, 0, Bp * 8, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(mags, 0, Bp * 8, st);
+    if (e != cudaSuccess || R == 0) return e;
+    const unsigned threads = Bp == 48 ? 192 : 256;  // a multiple of every padded frame count
+    const uint64_t total = R * Bp;
+    const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(total, threads * 4ull), kB200SMs * 8);
+    k_count_sums<<<grid, threads, 0, st>>>(sino, total, Bp, sums, mags);
+    return cudaGetLastError();
 }
 
 cudaError_t interleave_i32(const int32_t* in, int32_t* out, uint64_t n, uint32_t B, uint32_t Bp,
@@ -678,10 +732,10 @@ cudaError_t remap_columns(uint2* elems, uint64_t nnz, const uint32_t* perm, cuda
     return cudaGetLastError();
 }
 
-cudaError_t fill_frames(float* x, uint64_t n, uint32_t Bp, uint32_t B, const float* vals,
-                        cudaStream_t st) {
+cudaError_t fill_frames(float* x, uint64_t n, uint32_t Bp, const FrameValues& vals, cudaStream_t st) {
     if (n * Bp == 0) return cudaSuccess;
-    k_fill_frames<<<elementwise_grid(n * Bp), 256, 0, st>>>(x, n, Bp, B, vals);
+    if (Bp > 64) return cudaErrorInvalidValue;
+    k_fill_frames<<<elementwise_grid(n * Bp), 256, 0, st>>>(x, n * Bp, Bp, vals);
     return cudaGetLastError();
 }
 

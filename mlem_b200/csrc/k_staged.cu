@@ -66,7 +66,7 @@ cudaError_t launch_staged(const SparseView& csr, const float* x, uint32_t B, con
     cudaError_t e = cudaFuncSetAttribute(k_fused_staged<BT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_fused_staged<BT>, grid, kStagedThreads, smem, st, csr, x, B, sino, u,
+    return launch_dependent(csr.n <= kDependentMost, k_fused_staged<BT>, grid, kStagedThreads, smem, st, csr, x, B, sino, u,
                             chunk_rows, counter);
 }
 

@@ -204,6 +204,11 @@ cudaError_t image_stats(const float* x, uint32_t C, uint32_t B, uint32_t n_out, 
                         unsigned int* slot, double* sums, unsigned long long* zeros,
                         unsigned long long* subnormals, bool one_launch, cudaStream_t st);
 
+// Per frame f < Bp (a padded frame count) of the interleaved sinogram [R][Bp]:
+// the sum of its counts (two's complement) and of their magnitudes.
+cudaError_t count_sums(const int32_t* sino, uint64_t R, uint32_t Bp, unsigned long long* sums,
+                       unsigned long long* mags, cudaStream_t st);
+
 // ---- layout helpers -------------------------------------------------------
 // out[p(i)*Bp + b] = in[b*n + i] for b < B (n items per frame; pad frames
 // untouched), and back: out[b*n + i] = in[p(i)*Bp + b], where p = perm
@@ -224,9 +229,11 @@ cudaError_t permute_to_natural(const float* in, float* out, const uint32_t* perm
                                uint32_t B, uint32_t Bd, cudaStream_t st);
 // Relabel the column (voxel) index of every element: e.x = perm[e.x].
 cudaError_t remap_columns(uint2* elems, uint64_t nnz, const uint32_t* perm, cudaStream_t st);
-// x[i][b] = b < B ? vals[b] : 0 for the Bp-interleaved image (vals: device, B floats).
-cudaError_t fill_frames(float* x, uint64_t n, uint32_t Bp, uint32_t B, const float* vals,
-                        cudaStream_t st);
+// x[i][b] = vals.v[b] for the Bp-interleaved image (Bp <= 64).
+struct FrameValues {
+    float v[64];
+};
+cudaError_t fill_frames(float* x, uint64_t n, uint32_t Bp, const FrameValues& vals, cudaStream_t st);
 // c[i] = calcCorrel(s[i], f[i]).
 cudaError_t correl_elementwise(const float* f, const int32_t* s, float* c, uint64_t n,
                                cudaStream_t st);
