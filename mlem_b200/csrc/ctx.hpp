@@ -151,6 +151,13 @@ struct mlem_ctx {
     cudaEvent_t ev_img[2] = {nullptr, nullptr}, ev_dfree[2] = {nullptr, nullptr};
     bool images_ready = false;
 
+    // The census of an iteration runs on a stream of its own beside the next
+    // iteration's forward pass, which like it only reads the image; what writes
+    // the image waits for it (join_census).
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_image = nullptr, ev_census = nullptr;
+    bool census_out = false;  // a census the stream has not waited for
+
     // statistics history
     void* stats_scratch = nullptr;
     unsigned int* stats_slot = nullptr;

@@ -430,9 +430,9 @@ struct FwRun {
         const int grid = gather_grid<G, BT>(cfg, csr.n);
         if constexpr (BT <= 4)
             if (c && !y && !csr.n_dev)
-                return launch_dependent(csr.n <= kDependentMost, k_fwproj<G, BT, true>, grid, kGatherThreads, 0, st, csr, x, B,
+                return launch_dependent(cfg.dependent && csr.n <= kDependentMost, k_fwproj<G, BT, true>, grid, kGatherThreads, 0, st, csr, x, B,
                                         f0, sino, c, y);
-        return launch_dependent(csr.n <= kDependentMost, k_fwproj<G, BT, false>, grid, kGatherThreads, 0, st, csr, x, B, f0,
+        return launch_dependent(cfg.dependent && csr.n <= kDependentMost, k_fwproj<G, BT, false>, grid, kGatherThreads, 0, st, csr, x, B, f0,
                                 sino, c, y);
     }
 };
@@ -442,7 +442,7 @@ struct BkRun {
     static cudaError_t run(const LaunchCfg& cfg, cudaStream_t st, const SparseView& csc,
                            const float* c, uint32_t B, uint32_t f0, const float* norm, float* x,
                            float* u) {
-        return launch_dependent(csc.n <= kDependentMost, k_bkproj_csc<G, BT>, gather_grid<G, BT>(cfg, csc.n), kGatherThreads, 0,
+        return launch_dependent(cfg.dependent && csc.n <= kDependentMost, k_bkproj_csc<G, BT>, gather_grid<G, BT>(cfg, csc.n), kGatherThreads, 0,
                                 st, csc, c, B, f0, norm, x, u);
     }
 };

@@ -342,20 +342,20 @@ cudaError_t fused_row(const SparseView& csr, const float* x, uint32_t B, uint32_
 }
 
 cudaError_t apply_update(float* x, float* u, const float* norm, uint32_t C, uint32_t B,
-                         bool zero_u, cudaStream_t st) {
+                         bool zero_u, cudaStream_t st, bool dependent) {
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    return launch_dependent(n <= kDependentMost, B == 1 ? k_apply_update<true> : k_apply_update<false>, grid, 256, 0, st, x,
+    return launch_dependent(dependent && n <= kDependentMost, B == 1 ? k_apply_update<true> : k_apply_update<false>, grid, 256, 0, st, x,
                             u, norm, n, B, zero_u);
 }
 
 cudaError_t apply_update_subset(float* x, float* u, const float* norm_s, const float* norm,
-                                uint32_t C, uint32_t B, cudaStream_t st) {
+                                uint32_t C, uint32_t B, cudaStream_t st, bool dependent) {
     const uint64_t n = (uint64_t)C * B;
     if (n == 0) return cudaSuccess;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)kB200SMs * 16);
-    return launch_dependent(true, B == 1 ? k_apply_update_subset<true> : k_apply_update_subset<false>, grid,
+    return launch_dependent(dependent, B == 1 ? k_apply_update_subset<true> : k_apply_update_subset<false>, grid,
                             256, 0, st, x, u, norm_s, norm, n, B);
 }
 

@@ -69,6 +69,7 @@ struct LaunchCfg {
     int frame_tile = 1;   // frames per pass over the matrix: 1, 2, 4, 8 or 16
     int blocks_per_sm = 8;
     int sm_count = 148;
+    bool dependent = true;  // small launches may be programmatic dependents
 };
 
 // Valid launch configuration (group 4..32, frame tile 1..16, 1..8 blocks/SM).
@@ -169,12 +170,12 @@ cudaError_t long_rows_pass(const SparseView& csr, const LongSeg* segs, uint32_t 
 
 // x[i] *= factor(u[i], norm[i/B]); u[i] = 0 when zero_u.
 cudaError_t apply_update(float* x, float* u, const float* norm, uint32_t C, uint32_t B,
-                         bool zero_u, cudaStream_t st);
+                         bool zero_u, cudaStream_t st, bool dependent = true);
 
 // ---- ordered subsets (row r in subset r % S) -------------------------------
 // x *= norm_s != 0 ? u / norm_s : (norm != 0 ? 1 : u); u = 0.
 cudaError_t apply_update_subset(float* x, float* u, const float* norm_s, const float* norm,
-                                uint32_t C, uint32_t B, cudaStream_t st);
+                                uint32_t C, uint32_t B, cudaStream_t st, bool dependent = true);
 // Column sums of subset s over the CSC, in ascending row order (bit-exact
 // with calcColumnSums over the subset's rows).
 cudaError_t subset_column_sums_exact(const SparseView& csc, uint32_t S, uint32_t s, float* norm,
