@@ -164,6 +164,31 @@ __global__ void __launch_bounds__(1024, 1) k_fused_chunked(SparseView csr,
     }
 }
 
+// The same at one frame, each warp's rows pipelined (one_pass_rows).
+__global__ void __launch_bounds__(1024, 1) k_fused_chunked_one(SparseView csr, const float* __restrict__ x,
+                                                              const int32_t* __restrict__ sino,
+                                                              float* __restrict__ u, uint32_t chunk,
+                                                              unsigned int* __restrict__ counter) {
+    __shared__ uint32_t s_chunk;
+    const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    pdl_wait();
+    pdl_release();
+    for (;;) {
+        if (threadIdx.x == 0) s_chunk = work_grab(counter);
+        __syncthreads();
+        const uint64_t ci = s_chunk;
+        __syncthreads();  // s_chunk is rewritten by the next grab
+        // re-read per chunk (a cached load) rather than held in a register
+        const uint64_t n = visit_count(csr);
+        if (ci >= (n + chunk - 1) / chunk) {  // block-uniform
+            if (threadIdx.x == 0) work_leave(counter);
+            return;
+        }
+        const uint64_t r0 = ci * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
+        one_pass_rows(csr, x, sino, u, (uint32_t)r0 + warp, (uint32_t)r1, nwarps);
+    }
+}
+
 }  // namespace
 
 cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int frame_tile,
@@ -176,6 +201,8 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
     if (!csr.order || !csr.vrange) return cudaErrorInvalidValue;  // a sorted visit
     // the resident CTAs: 64 registers x 1024 threads per SM, in 1, 2 or 4 CTAs
     const int grid = std::max(1, sm_count * ctas_per_sm), threads = 1024 / ctas_per_sm;
+    if (B == 1 && csr.max_len != ~0u)
+        return launch_dependent(csr.n <= kDependentMost, k_fused_chunked_one, grid, threads, 0, st, csr, x, sino, u, chunk_rows, counter);
     switch (frame_tile) {
         case 1: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
         case 2: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<2>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);

@@ -32,17 +32,6 @@ namespace {
 
 constexpr int kGatherThreads = 256;
 
-// One element when `in`, else {0, 0} (value 0).
-__device__ __forceinline__ uint2 ld_elem_if(const uint2* p, bool in, uint64_t pol) {
-    uint2 r;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
-        "@p ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;\n\t}"
-        : "=r"(r.x), "=r"(r.y)
-        : "l"(p), "l"(pol), "r"((uint32_t)in));
-    return r;
-}
-
 // Frame tile split: VW <= 8 floats (a 32-byte sector) per lane.
 template <int BT>
 struct GLanes {

@@ -90,6 +90,17 @@ __global__ void __launch_bounds__(256) k_fused_row(SparseView csr, const float* 
 }
 
 
+// The sorted walk at one frame and a warp per row, pipelined (one_pass_rows).
+__global__ void __launch_bounds__(256, 4) k_fused_row_one(SparseView csr, const float* __restrict__ x,
+                                                         const int32_t* __restrict__ sino,
+                                                         float* __restrict__ u) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    pdl_wait();
+    pdl_release();
+    one_pass_rows(csr, x, sino, u, warp, (uint32_t)visit_count(csr), nwarps);
+}
+
 #undef MLEM_WARP_LOOP_SETUP
 
 template <bool ONE_FRAME>
@@ -337,6 +348,11 @@ cudaError_t fused_row(const SparseView& csr, const float* x, uint32_t B, uint32_
     if (!cfg_valid(cfg) || (B % cfg.frame_tile) || (f0 % cfg.frame_tile)) return cudaErrorInvalidValue;
     if (csr.n == 0) return cudaSuccess;
     if (csr.order && !csr.vrange) return cudaErrorInvalidValue;  // sorted visits carry vrange
+    if (csr.vrange && B == 1 && cfg.group == 32 && csr.max_len != ~0u) {
+        // the resident CTAs: rows in flight from the first to the last
+        const int grid = std::min(cfg.blocks_per_sm, 4) * cfg.sm_count;
+        return launch_dependent(csr.n <= kDependentMost, k_fused_row_one, grid, 256, 0, st, csr, x, sino, u);
+    }
     if (csr.vrange) return dispatch<FusedSortedK>(cfg, st, csr, x, B, f0, sino, u);
     return dispatch<FusedK>(cfg, st, csr, x, B, f0, sino, u);
 }

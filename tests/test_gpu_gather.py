@@ -93,3 +93,39 @@ def test_default_frame_tile_follows_the_frames():
             ctx.iterate(4)
             imgs.append(ctx.get_images().astype(np.float64))
     assert np.linalg.norm(imgs[0] - imgs[1]) <= 1e-5 * np.linalg.norm(imgs[1])
+
+
+@pytest.mark.parametrize("visit", [api.VISIT_SORTED, api.VISIT_SORTED_CHUNKED])
+@pytest.mark.parametrize("rows", [2, 33, 12000])
+def test_pipelined_one_pass_against_float64(visit, rows):
+    """The one-frame sorted one-pass walk at the edges of its 256-element batch,
+    with fewer and more rows than warps: u = A^T (s / A x), each entry within the
+    rounding of its terms."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(rows)
+    edges = np.array([0, 1, 31, 32, 33, 255, 256, 257, 287, 288, 511, 512, 513, 900, 4096])
+    lens = edges[rng.integers(0, edges.size, rows)] if rows > 100 else edges[np.arange(rows) % edges.size]
+    lens[-1] = 257
+    end = np.cumsum(lens).astype(np.uint64)
+    C = 5000
+    el = np.zeros(int(end[-1]), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, C, el.size)
+    el["value"] = rng.uniform(0.05, 1.7, el.size)
+    m = formats.Csr4(rows, C, end, el)
+    s = rng.poisson(3, rows).astype(np.int32)
+    x = rng.uniform(0.1, 2.0, C).astype(np.float32)
+    f = sums(m, x[:, None], False)[0][:, 0]
+    c = np.where(f != 0, s / np.where(f != 0, f, 1.0), 0.0)
+    ref, mag, cnt = sums(m, c[:, None], True)
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_tuning(api.BK_FUSED, 32, 1, 4, visit)
+        xd, sd = torch.from_numpy(x).cuda(), torch.from_numpy(s).cuda()
+        for own in (False, True):  # the caller's sinogram over every row, the context's over its list
+            u = torch.full((C,), np.nan, device="cuda")
+            if own:
+                ctx.set_sinograms(s)
+            ctx.fused_update_d(xd.data_ptr(), 0 if own else sd.data_ptr(), u.data_ptr(), 1,
+                               torch.cuda.current_stream().cuda_stream)
+            got = u.cpu().numpy().astype(np.float64)
+            # n terms, each with its factor's error: a sum of at most 4096 products and a division
+            assert np.all(np.abs(got - ref[:, 0]) <= 2.0 ** -23 * (cnt[:, 0] + 4096 + 4) * mag[:, 0])
