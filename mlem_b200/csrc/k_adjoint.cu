@@ -33,7 +33,7 @@ __device__ __forceinline__ void adjoint_row_range(const SparseView& csr, const f
                                                   float* __restrict__ rows, float* __restrict__ u,
                                                   uint64_t r_begin, uint64_t r_end, uint64_t warp,
                                                   uint64_t nwarps) {
-    constexpr int kBatch = batch_depth<32>();
+    constexpr int kBatch = batch_depth<32, 1>();
     const int lane = threadIdx.x & 31;
     const uint64_t ps = l2_evict_first(), ph = l2_evict_last();
     const uint2* el = reinterpret_cast<const uint2*>(csr.pairs);

@@ -39,43 +39,6 @@ struct GLanes {
     static constexpr int FL = BT / VW;
 };
 
-// VW floats when `in`, else zeros.  Not the .nc form: the kernel before this one
-// (which it may overlap up to pdl_wait) writes the vector.
-template <int VW>
-__device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW], uint64_t pol) {
-    if constexpr (VW == 8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %10, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-            "mov.f32 %4, 0f00000000;\n\tmov.f32 %5, 0f00000000;\n\tmov.f32 %6, 0f00000000;\n\t"
-            "mov.f32 %7, 0f00000000;\n\t"
-            "@p ld.global.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;\n\t}"
-            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
-              "=f"(v[7])
-            : "l"(p), "l"(pol), "r"((uint32_t)in));
-    } else if constexpr (VW == 4) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-            "@p ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n\t}"
-            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-            : "l"(p), "l"(pol), "r"((uint32_t)in));
-    } else if constexpr (VW == 2) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "mov.f32 %1, 0f00000000;\n\t"
-            "@p ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;\n\t}"
-            : "=f"(v[0]), "=f"(v[1])
-            : "l"(p), "l"(pol), "r"((uint32_t)in));
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "@p ld.global.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
-            : "=f"(v[0])
-            : "l"(p), "l"(pol), "r"((uint32_t)in));
-    }
-}
-
 // VW <= 8 values as 16-byte (or narrower) accesses: the outputs and the counts
 // need no more alignment than a tile of four frames does.
 template <int VW>

@@ -102,12 +102,75 @@ __device__ __forceinline__ void red_vec(float* __restrict__ p, float w, const fl
         atomicAdd(p, w * c[0]);
 }
 
+// Predicated loads: the value when `in`, else zeros.  Volatile, so that a batch of
+// them goes out before anything waits: as conditional expressions the compiler
+// put most of them behind one another (16 frames in chunks 2,996 -> 2,639 us per
+// iteration of 1,048,576 rows with these and batches of 4, sorted 3,994 -> 3,481,
+// staged 2,615 -> 2,529; 8 frames of 120,007 rows 79 -> 63 us).
+// One element of the stream, past L1.
+__device__ __forceinline__ uint2 ld_elem_if(const uint2* p, bool in, uint64_t pol) {
+    uint2 r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
+        "@p ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;\n\t}"
+        : "=r"(r.x), "=r"(r.y)
+        : "l"(p), "l"(pol), "r"((uint32_t)in));
+    return r;
+}
+// One element through L1 (a row that is read again).
+__device__ __forceinline__ uint2 ld_elem_keep_if(const uint2* p, bool in, uint64_t pol) {
+    uint2 r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
+        "@p ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;\n\t}"
+        : "=r"(r.x), "=r"(r.y)
+        : "l"(p), "l"(pol), "r"((uint32_t)in));
+    return r;
+}
+// VW floats when `in`, else zeros.  Not the .nc form: the kernel before this one
+// (which it may overlap up to pdl_wait) writes the vector.
+template <int VW>
+__device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW], uint64_t pol) {
+    if constexpr (VW == 8) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %10, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+            "mov.f32 %4, 0f00000000;\n\tmov.f32 %5, 0f00000000;\n\tmov.f32 %6, 0f00000000;\n\t"
+            "mov.f32 %7, 0f00000000;\n\t"
+            "@p ld.global.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;\n\t}"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+              "=f"(v[7])
+            : "l"(p), "l"(pol), "r"((uint32_t)in));
+    } else if constexpr (VW == 4) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "mov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+            "@p ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n\t}"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+            : "l"(p), "l"(pol), "r"((uint32_t)in));
+    } else if constexpr (VW == 2) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "mov.f32 %1, 0f00000000;\n\t"
+            "@p ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;\n\t}"
+            : "=f"(v[0]), "=f"(v[1])
+            : "l"(p), "l"(pol), "r"((uint32_t)in));
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "@p ld.global.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
+            : "=f"(v[0])
+            : "l"(p), "l"(pol), "r"((uint32_t)in));
+    }
+}
+
 // Elements a lane loads before it gathers (memory-level parallelism).  A
-// full-warp group takes 8 (a 150-250-element row is one batch); narrower
-// groups take 4, which keeps their registers, and so their occupancy, lower
+// full-warp group takes 8 (a 150-250-element row is one batch) at one and two
+// frames; with four floats per lane 8 gathers and the kept elements would spill,
+// and narrower groups keep their registers, and so their occupancy, lower with 4
 // (measured on the plain-full workload).
-template <int G>
-constexpr int batch_depth() { return G == 32 ? 8 : 4; }
+template <int G, int BT>
+constexpr int batch_depth() { return G == 32 && BT < 4 ? 8 : 4; }
 
 // acc[0..VW) = sum over the row's elements of value * vec[col*B + off + ...].
 // Each batch issues all of its (predicated) element loads, then all of its
@@ -121,7 +184,7 @@ __device__ __forceinline__ bool row_dot(const uint2* __restrict__ el, uint64_t b
                                         uint32_t off, float (&acc)[Lanes<BT>::VW], uint64_t ps,
                                         uint64_t ph, uint2* keep = nullptr) {
     constexpr int VW = Lanes<BT>::VW, FL = Lanes<BT>::FL, EPS = G / FL;
-    constexpr int kBatch = batch_depth<G>();
+    constexpr int kBatch = batch_depth<G, BT>();
     const float* base = vec + off;
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[i] = 0.0f;
@@ -138,19 +201,12 @@ __device__ __forceinline__ bool row_dot(const uint2* __restrict__ el, uint64_t b
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const uint64_t k = k0 + (uint64_t)u * EPS;
-            q[u] = make_uint2(0u, 0u);  // value 0: contributes nothing
-            if (k < e) q[u] = kL1 ? ld_keep2(el + k, ps) : ld_stream2(el + k, ps);
+            q[u] = kL1 ? ld_elem_keep_if(el + k, k < e, ps) : ld_elem_if(el + k, k < e, ps);
         }
         float xv[kBatch][VW];
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            if (k0 + (uint64_t)u * EPS < e) {
-                ld_vec<VW>(base + (size_t)q[u].x * B, xv[u], ph);
-            } else {
-#pragma unroll
-                for (int i = 0; i < VW; ++i) xv[u][i] = 0.0f;
-            }
-        }
+        for (int u = 0; u < kBatch; ++u)
+            ld_vec_if<VW>(base + (size_t)q[u].x * B, k0 + (uint64_t)u * EPS < e, xv[u], ph);
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const float v = __uint_as_float(q[u].y);
@@ -193,7 +249,7 @@ __device__ __forceinline__ void fused_row_range(const SparseView& csr, const flo
     // [r_begin, r_end) are visiting positions (rows in csr.order when set)
     constexpr int RPW = 32 / G;
     constexpr int VW = Lanes<BT>::VW, FL = Lanes<BT>::FL, EPS = G / FL;
-    constexpr int kBatch = batch_depth<G>();
+    constexpr int kBatch = batch_depth<G, BT>();
     const int lw = threadIdx.x & 31;
     const int lane = lw & (G - 1);
     const int sub = lane % FL;
@@ -260,27 +316,6 @@ __device__ __forceinline__ void fused_row_range(const SparseView& csr, const flo
     }
 }
 
-// One element when `in`, else {0, 0} (value 0); volatile, so that a batch of
-// them goes out before anything waits.
-__device__ __forceinline__ uint2 ld_elem_if(const uint2* p, bool in, uint64_t pol) {
-    uint2 r;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
-        "@p ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;\n\t}"
-        : "=r"(r.x), "=r"(r.y)
-        : "l"(p), "l"(pol), "r"((uint32_t)in));
-    return r;
-}
-__device__ __forceinline__ float ld_hot_if(const float* p, bool in, uint64_t pol) {
-    float r;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-        "@p ld.global.L2::cache_hint.f32 %0, [%1], %2;\n\t}"
-        : "=f"(r)
-        : "l"(p), "l"(pol), "r"((uint32_t)in));
-    return r;
-}
-
 // One pass over the sorted visiting positions v, v + S, ... < end at one frame, a
 // warp per row: forward sum, calcCorrel, scatter.  What the whole machine waits
 // for is the L2's float reductions (plain-full: 299 M sector reductions, 1.63 ms
@@ -328,12 +363,12 @@ __device__ __forceinline__ void one_pass_rows(const SparseView& csr, const float
 #pragma unroll
         for (int t = 0; t < D; ++t) qn[t] = ld_elem_if(nx.b + t * 32, t * 32 < mn, ps);
         const int32_t sn = sino[nx.r];
-        float xv[D];
+        float xv[D][1];
 #pragma unroll
-        for (int t = 0; t < D; ++t) xv[t] = ld_hot_if(x + q[t].x, t * 32 < m, ph);
+        for (int t = 0; t < D; ++t) ld_vec_if<1>(x + q[t].x, t * 32 < m, xv[t], ph);
         float acc = 0.0f;
 #pragma unroll
-        for (int t = 0; t < D; ++t) acc = fmaf(__uint_as_float(q[t].y), xv[t], acc);
+        for (int t = 0; t < D; ++t) acc = fmaf(__uint_as_float(q[t].y), xv[t][0], acc);
         for (uint32_t k = kBatch; k + lane < cur.n; k += 32) {
             const uint2 e = ld_keep2(cur.b + k, ps);
             acc = fmaf(__uint_as_float(e.y), ld_hot(x + e.x, ph), acc);

@@ -91,14 +91,8 @@ __device__ __forceinline__ void staged_row(const uint2* __restrict__ el, const u
             e[t] = j < n ? row[j] : make_uint2(0u, 0u);
         }
 #pragma unroll
-        for (int t = 0; t < kBatch; ++t) {
-            if (j0 + t * EPS < n) {
-                ld_vec<VW>(x + off + (size_t)e[t].x * B, xv[t], ph);
-            } else {
-#pragma unroll
-                for (int i = 0; i < VW; ++i) xv[t][i] = 0.0f;
-            }
-        }
+        for (int t = 0; t < kBatch; ++t)
+            ld_vec_if<VW>(x + off + (size_t)e[t].x * B, j0 + t * EPS < n, xv[t], ph);
 #pragma unroll
         for (int t = 0; t < kBatch; ++t) {
             const float v = __uint_as_float(e[t].y);
