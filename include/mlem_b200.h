@@ -363,6 +363,20 @@ int mlem_ratio_rows_d(mlem_ctx* ctx, const float* x, const int32_t* sino, float*
                       float* update, void* stream);
 int mlem_adjoint_update_d(mlem_ctx* ctx, const float* du, const int32_t* sino, const float* rows,
                           float* update, void* stream);
+/* The voxel-wise steps of the unrolled relaxed MLEM around those two (one frame,
+ * device pointers, natural voxel order, norm[C]; omega: one float on the device):
+ *   mlem_relax_step_d: ratio = norm != 0 ? update / norm : update and
+ *                      x_next = x * (ratio > 0 ? max(ratio, 1e-38) ** omega : 0);
+ *   mlem_relax_grad_d: for the gradient g + g2 of x_next (g2 may be NULL), gx =
+ *                      the part with respect to x at a fixed ratio, du = the one
+ *                      with respect to update, and omega's gradient in
+ *                      MLEM_RELAX_PARTIALS parts.  gx may be g. */
+#define MLEM_RELAX_PARTIALS 592
+int mlem_relax_step_d(mlem_ctx* ctx, const float* x, const float* update, const float* norm,
+                      const float* omega, float* ratio, float* x_next, void* stream);
+int mlem_relax_grad_d(mlem_ctx* ctx, const float* g, const float* g2, const float* x,
+                      const float* ratio, const float* norm, const float* omega, float* gx,
+                      float* du, double* partial, void* stream);
 /* Device pointer of the context's column sums (float[C]). */
 int mlem_norm_d(mlem_ctx* ctx, const float** norm);
 /* Replace the column sums with norm[C] (device pointer): a row shard uses the

@@ -51,6 +51,8 @@ BATCH_NAMES = {BATCH_INTERLEAVED: "interleaved", BATCH_ITEMS: "items"}
 BK_NAMES = {BK_CSC: "csc", BK_ATOMIC: "atomic", BK_FUSED: "fused", BK_REGION: "region",
             BK_MIRRORED: "mirrored"}
 
+RELAX_PARTIALS = 592  # MLEM_RELAX_PARTIALS
+
 ELEM_DTYPE = np.dtype([("index", "<u4"), ("value", "<f4")])
 
 
@@ -415,6 +417,20 @@ class Context:
         nonzero, in one pass (one frame)."""
         self._chk(core_lib().mlem_adjoint_update_d(self._h, du_ptr, sino_ptr, rows_ptr, update_ptr,
                                                    stream))
+
+    def relax_step_d(self, x_ptr, update_ptr, norm_ptr, omega_ptr, ratio_ptr, next_ptr,
+                     stream=0) -> None:
+        """ratio = calcUpdate's factor of update, next = x * ratio ** omega (0 where
+        ratio <= 0); omega is one float on the device."""
+        self._chk(core_lib().mlem_relax_step_d(self._h, x_ptr, update_ptr, norm_ptr, omega_ptr,
+                                               ratio_ptr, next_ptr, stream))
+
+    def relax_grad_d(self, g_ptr, g2_ptr, x_ptr, ratio_ptr, norm_ptr, omega_ptr, gx_ptr, du_ptr,
+                     partial_ptr, stream=0) -> None:
+        """The gradient of relax_step_d for g + g2 (g2_ptr None: g alone); partial:
+        RELAX_PARTIALS doubles whose sum is omega's."""
+        self._chk(core_lib().mlem_relax_grad_d(self._h, g_ptr, g2_ptr, x_ptr, ratio_ptr, norm_ptr,
+                                               omega_ptr, gx_ptr, du_ptr, partial_ptr, stream))
 
     def bkproj_update_d(self, correl_ptr, x_ptr, n_frames=1, stream=0) -> None:
         self._chk(core_lib().mlem_bkproj_update_d(self._h, correl_ptr, x_ptr, n_frames, stream))

@@ -41,6 +41,8 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
                      "-ftz=true", "-prec-div=true", "-prec-sqrt=true",
                      "--expt-relaxed-constexpr", "-ccbin", CXX,
                      f"-I{INCLUDE}", f"-I{CSRC}", f"-I{GEN}"]
+# Sources that replace tensor expressions of the same arithmetic keep subnormals.
+KEEP_SUBNORMALS = {"k_relax.cu"}
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wextra", f"-I{INCLUDE}", f"-I{CSRC}"]
 
 
@@ -82,7 +84,10 @@ def _compile(src, jobs_verbose=False):
     obj = os.path.join(OBJ, rel + ".o")
     if _newer(obj, [src] + _headers()):
         if src.endswith(".cu"):
-            _run([NVCC] + NVCC_FLAGS + ["-c", src, "-o", obj])
+            flags = NVCC_FLAGS
+            if rel in KEEP_SUBNORMALS:
+                flags = ["-ftz=false" if f == "-ftz=true" else f for f in flags]
+            _run([NVCC] + flags + ["-c", src, "-o", obj])
         else:
             _run([CXX] + CXX_FLAGS + ["-c", src, "-o", obj])
         if jobs_verbose:

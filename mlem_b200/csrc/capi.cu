@@ -2846,6 +2846,27 @@ int mlem_adjoint_update_d(mlem_ctx* c, const float* du, const int32_t* sino, con
     return backward_pass(c, kOpAdjoint, du, sino, const_cast<float*>(rows), update, stream);
 }
 
+static_assert(MLEM_RELAX_PARTIALS == kRelaxPartials, "the header's count is the kernel's grid");
+
+int mlem_relax_step_d(mlem_ctx* c, const float* x, const float* update, const float* norm,
+                      const float* omega, float* ratio, float* x_next, void* stream) {
+    if (!c || !x || !update || !norm || !omega || !ratio || !x_next)
+        return fail(c, MLEM_ERR_INVALID, "null argument");
+    TRY(set_device(c));
+    CK(c, relax_step(x, update, norm, omega, c->C, ratio, x_next, (cudaStream_t)stream));
+    return MLEM_OK;
+}
+
+int mlem_relax_grad_d(mlem_ctx* c, const float* g, const float* g2, const float* x,
+                      const float* ratio, const float* norm, const float* omega, float* gx,
+                      float* du, double* partial, void* stream) {
+    if (!c || !g || !x || !ratio || !norm || !omega || !gx || !du || !partial)
+        return fail(c, MLEM_ERR_INVALID, "null argument");
+    TRY(set_device(c));
+    CK(c, relax_grad(g, g2, x, ratio, norm, omega, c->C, gx, du, partial, (cudaStream_t)stream));
+    return MLEM_OK;
+}
+
 int mlem_bkproj_update_d(mlem_ctx* c, const float* correl, float* x, uint32_t B, void* stream) {
     if (!c || !x || !correl || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     if (!c->has_csc || c->mirrored)

@@ -454,4 +454,17 @@ cudaError_t fused_staged(const SparseView& csr, const float* x, uint32_t B, int 
 cudaError_t batch_interleaved(const BatchTable& t, int frame_tile, bool sorted, int sm_count,
                               int blocks_per_sm, cudaStream_t st);
 
+// ---- voxel-wise steps of the unrolled relaxed MLEM (k_relax.cu) ------------
+// Natural voxel order, one frame; omega: one device float.  r = calcUpdate's
+// factor of u, x_next = x * (r > 0 ? max(r, 1e-38) ** omega : 0).
+cudaError_t relax_step(const float* x, const float* u, const float* norm, const float* omega,
+                       uint32_t C, float* r, float* x_next, cudaStream_t st);
+// The gradient of that step with respect to x (gx) and u (du) for the incoming
+// gradient g + g2 (g2 may be null), and omega's in kRelaxPartials parts.  gx may
+// be g.
+constexpr int kRelaxPartials = 592;
+cudaError_t relax_grad(const float* g, const float* g2, const float* x, const float* r,
+                       const float* norm, const float* omega, uint32_t C, float* gx, float* du,
+                       double* partial, cudaStream_t st);
+
 }  // namespace mlem

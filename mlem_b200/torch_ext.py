@@ -105,90 +105,91 @@ def _mirrored(ctx) -> bool:
     return bool(ctx.info.flags & api.FLAG_MIRROR_KERNELS)
 
 
-def _ratio_rows(ctx, x, sino_i, norm):
-    """calcUpdate factor of A^T (s / A x) and the row sums f = A x (0 for the
-    rows without a count), in one pass over the matrix (mlem_ratio_rows_d).
-    A mirrored context takes the fused update and a separate forward
-    projection instead (f is then A x on every row)."""
-    u = torch.empty_like(x)
+def _ratio_numerator(ctx, x, sino_i, u, f):
+    """u = A^T (s / A x) and the row sums f = A x (0 for the rows without a
+    count), in one pass over the matrix (mlem_ratio_rows_d).  A mirrored context
+    takes the fused update and a separate forward projection instead (f is then
+    A x on every row)."""
     if _mirrored(ctx):
         ctx.fused_update_d(x.data_ptr(), sino_i.data_ptr(), u.data_ptr(), 1, _stream())
-        f = _fw(ctx, x)
+        ctx.fwproj_d(x.data_ptr(), f.data_ptr(), 1, _stream())
     else:
-        f = torch.empty(ctx.n_rows, dtype=torch.float32, device=x.device)
         ctx.ratio_rows_d(x.data_ptr(), sino_i.data_ptr(), f.data_ptr(), u.data_ptr(), _stream())
-    r = torch.where(norm != 0, u / torch.where(norm != 0, norm, torch.ones_like(norm)), u)
-    return r, f
 
 
-def _adjoint(ctx, du, sino_i, f):
-    """A^T df with df = -(A du) s / f^2 where the row has a count and f != 0:
+def _adjoint(ctx, du, sino_i, f, out):
+    """out = A^T df with df = -(A du) s / f^2 where the row has a count and f != 0:
     the adjoint of calcCorrel and both projections, in one pass
     (mlem_adjoint_update_d; a mirrored context: a forward and a back
     projection with df formed between them)."""
-    du = du.contiguous()
     if _mirrored(ctx):
-        dc = _fw(ctx, du)
+        dc = _fw(ctx, du.view(-1))
         live = (sino_i != 0) & (f != 0)
         fs = torch.where(live, f, torch.ones_like(f))
+        # formed as -(dc (s / f)) / f so that a tiny f never squares to 0
         df = torch.where(live, -(dc * (sino_i.to(torch.float32) / fs)) / fs, torch.zeros_like(f))
-        return _bk(ctx, df)
-    out = torch.empty_like(du)
-    ctx.adjoint_update_d(du.data_ptr(), sino_i.data_ptr(), f.data_ptr(), out.data_ptr(), _stream())
-    return out
+        out.copy_(_bk(ctx, df).view(out.shape))
+    else:
+        ctx.adjoint_update_d(du.data_ptr(), sino_i.data_ptr(), f.data_ptr(), out.data_ptr(), _stream())
+
+
+def _step(ctx, x, u, norm, w, r, x_next):
+    ctx.relax_step_d(x.data_ptr(), u.data_ptr(), norm.data_ptr(), w.data_ptr(), r.data_ptr(),
+                     x_next.data_ptr(), _stream())
 
 
 class _UnrolledMLEM(torch.autograd.Function):
+    """Every iteration is one pass over the matrix and one over the voxels
+    (mlem_ratio_rows_d, mlem_relax_step_d), forward and backward alike
+    (mlem_relax_grad_d, mlem_adjoint_update_d)."""
+
     @staticmethod
-    def forward(fctx, x0, omega, sino_f, norm, ctx, sino_i, keep):
+    def forward(fctx, x0, omega, norm, ctx, sino_i, keep):
         K = omega.shape[0]
-        xs = [x0.detach()]
-        rs, fs = [], []
-        x = x0.detach().contiguous()
+        x0 = x0.detach()
+        xs = x0.new_empty((K,) + x0.shape)  # the images the iterations start from
+        xs[0].copy_(x0)
+        final, u = torch.empty_like(xs[0]), torch.empty_like(xs[0])
+        kept = (torch.empty_like(xs), x0.new_empty((K, ctx.n_rows))) if keep else ()
+        r, f = (None, None) if keep else (torch.empty_like(u), x0.new_empty(ctx.n_rows))
         for k in range(K):
-            r, f = _ratio_rows(ctx, x, sino_i, norm)
-            if keep:
-                rs.append(r)
-                fs.append(f)
-            x = x * torch.where(r > 0, r.clamp_min(1e-38) ** omega[k], torch.zeros_like(r))
-            xs.append(x)
+            rk, fk = (kept[0][k], kept[1][k]) if keep else (r, f)
+            _ratio_numerator(ctx, xs[k], sino_i, u, fk)
+            _step(ctx, xs[k], u, norm, omega[k], rk, xs[k + 1] if k + 1 < K else final)
         fctx.mctx = ctx
         fctx.sino_i = sino_i
         fctx.keep = keep
-        saved = [torch.stack(xs[:-1]), omega, sino_f, norm, x]
-        if keep:
-            saved += [torch.stack(rs), torch.stack(fs)]
-        fctx.save_for_backward(*saved)
-        return x
+        fctx.save_for_backward(xs, omega, norm, *kept)
+        return final
 
     @staticmethod
     def backward(fctx, g):
         ctx = fctx.mctx
         saved = fctx.saved_tensors
-        xs, omega, sino_f, norm = saved[:4]
+        xs, omega, norm = saved[:3]
         K = omega.shape[0]
         g = g.contiguous()
-        d_omega = torch.zeros_like(omega)
+        gx, du, out = (torch.empty_like(g) for _ in range(3))
+        partial = torch.empty((K, api.RELAX_PARTIALS), dtype=torch.float64, device=g.device)
+        if not fctx.keep:
+            u, r, f = torch.empty_like(g), torch.empty_like(g), g.new_empty(ctx.n_rows)
+        g2 = None
         for k in range(K - 1, -1, -1):
-            xk = xs[k].contiguous()
+            xk = xs[k]
             if fctx.keep:  # kept by the forward pass
-                r, f = saved[5][k], saved[6][k]
-            else:  # recomputed from the checkpoint
-                r, f = _ratio_rows(ctx, xk, fctx.sino_i, norm)
-            pos = r > 0
-            rs = torch.where(pos, r, torch.ones_like(r))
-            p = torch.where(pos, rs ** omega[k], torch.zeros_like(r))  # r^w
-            x_next = xk * p
-            d_omega[k] = torch.sum(g * x_next * torch.where(pos, torch.log(rs), torch.zeros_like(r)))
-            gx = g * p                                          # direct path
-            dr = torch.where(pos, g * xk * omega[k] * rs ** (omega[k] - 1), torch.zeros_like(r))
-            du = torch.where(norm != 0, dr / torch.where(norm != 0, norm, torch.ones_like(norm)), dr)
-            # adjoint of A^T, of calcCorrel (c = s / f where f != 0: dc/df = -s / f^2,
-            # formed as -(dc (s / f)) / f so that a tiny f never squares to 0; a row
-            # with zero counts has c = 0 whatever f is: no gradient) and of A
-            gx = gx + _adjoint(ctx, du, fctx.sino_i, f)
-            g = gx
-        return g, d_omega, None, None, None, None, None
+                r, f = saved[3][k], saved[4][k]
+            else:  # recomputed from the checkpoint (du holds the unused next image)
+                _ratio_numerator(ctx, xk, fctx.sino_i, u, f)
+                _step(ctx, xk, u, norm, omega[k], r, du)
+            # the direct path (gx) and omega's gradient, then the adjoint of A^T, of
+            # calcCorrel (a row with zero counts has c = 0 whatever f is: no gradient)
+            # and of A, added to the direct path by the next step
+            ctx.relax_grad_d(g.data_ptr(), g2.data_ptr() if g2 is not None else None, xk.data_ptr(),
+                             r.data_ptr(), norm.data_ptr(), omega[k].data_ptr(), gx.data_ptr(),
+                             du.data_ptr(), partial[k].data_ptr(), _stream())
+            _adjoint(ctx, du, fctx.sino_i, f, out)
+            g, g2 = gx, out
+        return gx + out, partial.sum(1).to(omega.dtype), None, None, None, None
 
 
 def unrolled_mlem(x0: torch.Tensor, omega: torch.Tensor, sino: torch.Tensor,
@@ -202,8 +203,11 @@ def unrolled_mlem(x0: torch.Tensor, omega: torch.Tensor, sino: torch.Tensor,
     if norm is None:
         norm = norm_tensor(ctx, x0.device)
     sino_i = sino.to(device=x0.device, dtype=torch.int32).contiguous()
-    sino_f = sino_i.to(torch.float32)
     K = int(omega.shape[0])
+    if K == 0:
+        raise RuntimeError("unrolled_mlem: omega holds no iteration")
+    # one float per voxel, as the voxel-wise kernels read it
+    norm = norm.to(device=x0.device, dtype=torch.float32).expand(x0.shape).contiguous()
     keep = K * (ctx.n_rows + ctx.n_cols) * 4 <= keep_bytes
-    return _UnrolledMLEM.apply(x0, omega.to(device=x0.device, dtype=torch.float32), sino_f, norm,
+    return _UnrolledMLEM.apply(x0, omega.to(device=x0.device, dtype=torch.float32).contiguous(), norm,
                                ctx, sino_i, keep)

@@ -195,3 +195,49 @@ def test_backward_pass_kernels_on_an_odd_matrix():
     ok = live & (f64 != 0)
     df = np.where(ok, -(dc * (s / np.where(ok, f64, 1.0))) / np.where(ok, f64, 1.0), 0.0)
     assert ob.rel_l2(a_got, ob.bkproj(m, df.astype(np.float32))) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 257, 300007])
+def test_relax_steps_match_tensor_expressions(n):
+    """mlem_relax_step_d and mlem_relax_grad_d against the same arithmetic in
+    float64: zero, negative and subnormal ratios, zero norms, one and two incoming
+    gradients.  powf and logf are within 8 ulp, the products round four times:
+    2^-20 relative."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    u, norm, x, g, g2 = (torch.rand(n, generator=gen, device="cuda") * 3 + 0.01 for _ in range(5))
+    pick = torch.randint(0, 12, (n,), generator=gen, device="cuda")
+    u[pick == 0] = 0.0
+    u[pick == 1] *= -1
+    norm[pick == 2] = 0.0
+    u[pick == 3], norm[pick == 3] = 3e-39, 1.0
+    g = g - 1.5
+    el = np.zeros(1, api.ELEM_DTYPE)
+    with api.Context(np.array([1], np.uint64), el, 1, n) as ctx:
+        st = torch.cuda.current_stream().cuda_stream
+        for w in (1.0, 0.37, 0.0):
+            om = torch.tensor([w], device="cuda")
+            r, xn, gx, du = (torch.empty(n, device="cuda") for _ in range(4))
+            part = torch.empty(api.RELAX_PARTIALS, dtype=torch.float64, device="cuda")
+            ctx.relax_step_d(x.data_ptr(), u.data_ptr(), norm.data_ptr(), om.data_ptr(), r.data_ptr(),
+                             xn.data_ptr(), st)
+            d = lambda t: t.double()  # noqa: E731
+            rw = torch.where(norm != 0, u / torch.where(norm != 0, norm, 1.0), u)
+            assert torch.equal(r, rw)
+            pos = rw > 0
+            want = d(x) * torch.where(pos, d(rw).clamp_min(float(np.float32(1e-38))) ** w, 0.0)
+            assert torch.all((d(xn) - want).abs() <= 2.0 ** -20 * want.abs() + 1e-45)
+            for second in (None, g2):
+                ctx.relax_grad_d(g.data_ptr(), second.data_ptr() if second is not None else None,
+                                 x.data_ptr(), r.data_ptr(), norm.data_ptr(), om.data_ptr(), gx.data_ptr(),
+                                 du.data_ptr(), part.data_ptr(), st)
+                gt = d(g if second is None else g + g2)
+                rs = torch.where(pos, d(rw), 1.0)
+                p = torch.where(pos, rs ** w, 0.0)
+                dr = torch.where(pos, gt * d(x) * w * rs ** (w - 1), 0.0)
+                wdu = torch.where(norm != 0, dr / torch.where(norm != 0, d(norm), 1.0), dr)
+                terms = gt * d(x) * p * torch.log(rs)
+                assert torch.all((d(gx) - gt * p).abs() <= 2.0 ** -20 * (gt * p).abs() + 1e-45)
+                # the exponent w - 1 is rounded: log(r) 2^-24 more
+                slack = 2.0 ** -20 + 2.0 ** -23 * torch.log(rs).abs()
+                assert torch.all((d(du) - wdu).abs() <= slack * wdu.abs() + 1e-45)
+                assert abs(float(part.sum() - terms.sum())) <= 2.0 ** -19 * float(terms.abs().sum()) + 1e-45
