@@ -93,6 +93,7 @@ namespace {
 SparseView csc_view(const mlem_ctx* c) {
     SparseView v{c->col_ptr, reinterpret_cast<const uint4*>(c->celems), c->C, c->Z};
     v.max_len = c->max_col_len;
+    v.by_line = false;
     return v;
 }
 
@@ -993,6 +994,7 @@ int enqueue_iteration(mlem_ctx* c, const mlem_tuning& t, bool stats,
                 if (by_visit) {
                     fw.out_by_visit = true;
                     bk.pairs = reinterpret_cast<const uint4*>(c->celems_vis);
+                    bk.by_line = true;
                     if (c->csc_act_ready) {
                         // only the rows with counts: the cut copy has no entry of another
                         // row, so the others' correlations are not read

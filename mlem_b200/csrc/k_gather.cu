@@ -117,6 +117,7 @@ struct FwOp {
         int32_t s[VW < 8 ? VW : 1];      // the counts, a row ahead
     };
     __device__ __forceinline__ uint64_t count() const { return visit_count(csr); }
+    __device__ __forceinline__ bool by_line() const { return csr.by_line; }
     // Row of visiting position v: loaded two rows ahead, so that its counts
     // (SKIP) can load beside its range.
     __device__ __forceinline__ uint32_t id(uint32_t v) const { return (uint32_t)row_at(csr, v); }
@@ -206,6 +207,7 @@ struct BkOp {
         float x[VW < 8 ? VW : 1];
     };
     __device__ __forceinline__ uint64_t count() const { return csc.n; }
+    __device__ __forceinline__ bool by_line() const { return csc.by_line; }
     __device__ __forceinline__ uint32_t id(uint32_t v) const { return v; }
     __device__ __forceinline__ Row row(uint32_t v, uint32_t) const {
         const uint2* el = reinterpret_cast<const uint2*>(csc.pairs);
@@ -251,69 +253,83 @@ __device__ __forceinline__ void gather_walk(const Op& op, const float* __restric
     constexpr int VW = GLanes<BT>::VW, FL = GLanes<BT>::FL, EPS = G / FL;
     constexpr int D = gather_depth<BT>();
     constexpr uint32_t kBatch = D * EPS;
-    const int slot = (threadIdx.x & (G - 1)) / FL;
+    const uint32_t slot = (threadIdx.x & (G - 1)) / FL;
     const uint64_t ps = l2_evict_first(), ph = l2_evict_last();
     pdl_wait();
     pdl_release();
     const uint32_t n = (uint32_t)op.count();
     if (v >= n) return;
     uint32_t rows = (n - v - 1) / stride;  // rows after the current one
-    // batches of the row (at least one, an empty one for an empty row) and
-    // the elements of the last
-    auto batches = [](uint64_t len, uint32_t& nb, uint32_t& tail) {
-        nb = len == 0 ? 1u : (uint32_t)((len + kBatch - 1) / kBatch);
-        tail = (uint32_t)(len - (uint64_t)(nb - 1) * kBatch);
+    // A row is walked from the last line (or the last multiple of a load's span)
+    // before it, `head` elements masked off.  At one frame the pass is bound by the
+    // L1's wavefronts (79 % busy), one for each 128-byte line that an instruction
+    // touches, and a third of them were a load's 64-byte pieces crossing lines:
+    // plain-full forward + back projection 1.93 -> 1.82 ms, 1,048,576 rows at 2 and 4
+    // frames 669 -> 635 and 912 -> 882; at 8 and 16
+    // frames the gathers' own lines leave nothing to gain (loading 16 bytes a lane
+    // there changed nothing either).  Batches of the row from there (at least one,
+    // an empty one for an empty row) and the elements of the last.
+    constexpr uint32_t kAlign = EPS < 16 ? EPS : 16;
+    auto enter = [&](const typename Op::Row& q, const uint2*& p, uint32_t& nb, uint32_t& tail) {
+        const uint64_t len = op.take(q);
+        const uint32_t head =
+            len && op.by_line() ? (uint32_t)(reinterpret_cast<uintptr_t>(q.b) >> 3) & (kAlign - 1) : 0u;
+        p = q.b + (int)(slot - head);
+        nb = len == 0 ? 1u : (uint32_t)((len + head + kBatch - 1) / kBatch);
+        tail = (uint32_t)(len + head - (uint64_t)(nb - 1) * kBatch);
+        return head;
     };
     typename Op::Row nx = op.row(v, op.id(v));
     typename Op::Pre pre = op.pre(nx, v);
-    const uint2* p = nx.b + slot;
+    const uint2* p;
     uint32_t nb, tail;  // of the current row, from the loaded batch q on
-    batches(op.take(nx), nb, tail);
+    uint32_t head = enter(nx, p, nb, tail);
     if (rows) nx = op.row(v + stride, op.id(v + stride));
     uint32_t id2 = rows > 1 ? op.id(v + 2 * stride) : 0u;
+    // element t of this lane is in the batch when t * EPS + s0 < m (unsigned)
     uint2 q[D];
-    int m0 = (int)(nb == 1 ? tail : kBatch) - slot;
+    uint32_t s0 = slot - head, m0 = (nb == 1 ? tail : kBatch) - head;
 #pragma unroll
-    for (int t = 0; t < D; ++t) q[t] = ld_elem_if(p + t * EPS, t * EPS < m0, ps);
+    for (int t = 0; t < D; ++t) q[t] = ld_elem_if(p + t * EPS, t * EPS + s0 < m0, ps);
     float acc[VW];
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[i] = 0.0f;
     for (;;) {
         // the next batch: the rest of this row, else the group's next row
         const bool last = nb == 1;
+        head = 0;
         if (!last) {
             p += kBatch;
             --nb;
         } else if (rows) {
-            p = nx.b + slot;
-            batches(op.take(nx), nb, tail);
+            head = enter(nx, p, nb, tail);
         } else {
             tail = 0;
         }
-        const int m = (int)(nb == 1 ? tail : kBatch) - slot;
+        const uint32_t s = slot - head, m = (nb == 1 ? tail : kBatch) - head;
         uint2 qn[D];
 #pragma unroll
-        for (int t = 0; t < D; ++t) qn[t] = ld_elem_if(p + t * EPS, t * EPS < m, ps);
+        for (int t = 0; t < D; ++t) qn[t] = ld_elem_if(p + t * EPS, t * EPS + s < m, ps);
         // this batch's gathers
         float xv[D][VW];
 #pragma unroll
         for (int t = 0; t < D; ++t)
-            ld_vec_if<VW>(vec + off + (size_t)q[t].x * B, t * EPS < m0, xv[t], ph);
+            ld_vec_if<VW>(vec + off + (size_t)q[t].x * B, t * EPS + s0 < m0, xv[t], ph);
         // the batch's products by pairs, then as a tree, into the running sum: a
         // chain of len / (D x G) additions instead of len / G
 #pragma unroll
         for (int i = 0; i < VW; ++i) {
-            float s[(D + 1) / 2];
+            float sum[(D + 1) / 2];
 #pragma unroll
             for (int t = 0; t < D; t += 2) {
-                s[t / 2] = __uint_as_float(q[t].y) * xv[t][i];
-                if (t + 1 < D) s[t / 2] = fmaf(__uint_as_float(q[t + 1].y), xv[t + 1][i], s[t / 2]);
+                sum[t / 2] = __uint_as_float(q[t].y) * xv[t][i];
+                if (t + 1 < D) sum[t / 2] = fmaf(__uint_as_float(q[t + 1].y), xv[t + 1][i], sum[t / 2]);
             }
 #pragma unroll
             for (int h = 1; h < (D + 1) / 2; h <<= 1)
 #pragma unroll
-                for (int t = 0; t + h < (D + 1) / 2; t += 2 * h) s[t] += s[t + h];
-            acc[i] += s[0];
+                for (int t = 0; t + h < (D + 1) / 2; t += 2 * h) sum[t] += sum[t + h];
+            acc[i] += sum[0];
         }
         if (last) {
 #pragma unroll
@@ -330,6 +346,7 @@ __device__ __forceinline__ void gather_walk(const Op& op, const float* __restric
 #pragma unroll
             for (int i = 0; i < VW; ++i) acc[i] = 0.0f;
         }
+        s0 = s;
         m0 = m;
 #pragma unroll
         for (int t = 0; t < D; ++t) q[t] = qn[t];

@@ -50,6 +50,10 @@ struct SparseView {
     // The longest row (column), for the gather passes' choice of lanes; ~0 when
     // unknown.
     uint32_t max_len = ~0u;
+    // The gather passes walk a row from the memory line it starts in, so that the
+    // grouping of its sum depends on where it is stored.  Not with the CSC in file
+    // order, whose sums do not depend on the voxel layout.
+    bool by_line = true;
 };
 
 // Entry range of column (or row) i: [ptr[i], ptr[i + 1]), or len[i] entries from ptr[i].
