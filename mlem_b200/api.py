@@ -397,6 +397,14 @@ class Context:
     def bkproj_d(self, y_ptr: int, x_ptr: int, n_frames: int = 1, stream: int = 0) -> None:
         self._chk(core_lib().mlem_bkproj_d(self._h, y_ptr, x_ptr, n_frames, stream))
 
+    def fwproj_frames_d(self, x_ptr: int, y_ptr: int, n_frames: int, stream: int = 0) -> None:
+        """fwproj_d on frame-major vectors, x[B][C] and y[B][R]."""
+        self._chk(core_lib().mlem_fwproj_frames_d(self._h, x_ptr, y_ptr, n_frames, stream))
+
+    def bkproj_frames_d(self, y_ptr: int, x_ptr: int, n_frames: int, stream: int = 0) -> None:
+        """bkproj_d on frame-major vectors, y[B][R] and x[B][C]."""
+        self._chk(core_lib().mlem_bkproj_frames_d(self._h, y_ptr, x_ptr, n_frames, stream))
+
     def fwproj_correl_d(self, x_ptr, sino_ptr, correl_ptr, n_frames=1, stream=0) -> None:
         self._chk(core_lib().mlem_fwproj_correl_d(self._h, x_ptr, sino_ptr, correl_ptr, n_frames,
                                                   stream))

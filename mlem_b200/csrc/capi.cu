@@ -996,15 +996,21 @@ int enqueue_iteration(mlem_ctx* c, const mlem_tuning& t, bool stats,
                     bk.pairs = reinterpret_cast<const uint4*>(c->celems_vis);
                     bk.by_line = true;
                     if (c->csc_act_ready) {
-                        // only the rows with counts: the cut copy has no entry of another
-                        // row, so the others' correlations are not read
-                        fw.order = c->act_order;
-                        fw.vrange = c->act_ranges;
-                        fw.n_dev = c->act_n;
-                        fw.out_pos = c->row_pos;
                         bk.pairs = reinterpret_cast<const uint4*>(c->csc_act);
                         bk.len = c->csc_act_len;
                     }
+                }
+                // The list of rows with counts: where the cut copy has no entry of
+                // another row, and for wide tiles, whose forward pass does not skip
+                // rows by their counts -- the other rows' correlations are zeroed then
+                // (narrow tiles skip and write the zeros themselves).
+                const bool cut = by_visit && c->csc_act_ready;
+                if (c->act_ready && (cut || T >= 8) && (!by_visit || c->row_pos)) {
+                    fw.order = c->act_order;
+                    fw.vrange = c->act_ranges;
+                    fw.n_dev = c->act_n;
+                    if (by_visit) fw.out_pos = c->row_pos;
+                    if (!cut) CK(c, cudaMemsetAsync(c->correl, 0, (size_t)c->R * Bp * 4, st));
                 }
                 for (uint32_t f0 = 0; f0 < Bp; f0 += T)
                     CK(c, fwproj(fw, c->x, Bp, f0, c->sino, c->correl, nullptr, cfg, st));
@@ -2633,31 +2639,58 @@ int mlem_subset_column_sums(mlem_ctx* c, uint32_t s, float* out) {
 // ---- device-pointer entry points ---------------------------------------------
 // Caller vectors are in natural voxel order; with the brick layout they are
 // converted through the context's scratch buffers.
+namespace {
+// yd[R][Bd] = A xd[C][Bd], both in the device's order.
+int project_rows(mlem_ctx* c, const float* xd, float* yd, uint32_t Bd, cudaStream_t st) {
+    const LaunchCfg cfg = cfg_for_frames(c, Bd);
+    if (c->mirrored) CK(c, cudaMemsetAsync(yd, 0, (size_t)c->R * Bd * 4, st));
+    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile) {
+        if (c->mirrored)
+            CK(c, mirror_fwproj(csr_visit(c, c->tuning), c->mirror, xd, Bd, f0, cfg.frame_tile, yd,
+                                c->n_sm, c->tuning.blocks_per_sm, st));
+        else
+            CK(c, fwproj(csr_view(c), xd, Bd, f0, nullptr, nullptr, yd, cfg, st));
+    }
+    return MLEM_OK;
+}
+
+// xd[C][Bd] = A^T yd[R][Bd], both in the device's order.
+int project_columns(mlem_ctx* c, const float* yd, float* xd, uint32_t Bd, cudaStream_t st) {
+    const LaunchCfg cfg = cfg_for_frames(c, Bd);
+    if (c->mirrored || !c->has_csc) CK(c, cudaMemsetAsync(xd, 0, (size_t)c->C * Bd * 4, st));
+    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile) {
+        if (c->mirrored)
+            CK(c, mirror_bkproj(csr_visit(c, c->tuning), c->mirror, yd, nullptr, Bd, f0,
+                                cfg.frame_tile, xd, c->n_sm, c->tuning.blocks_per_sm, st));
+        else if (c->has_csc)
+            CK(c, bkproj_csc(csc_view(c), yd, Bd, f0, nullptr, nullptr, xd, cfg, st));
+        else
+            CK(c, bkproj_scatter(csr_visit(c, c->tuning), yd, Bd, f0, xd, cfg, st));
+    }
+    return MLEM_OK;
+}
+
+// Only the gather passes take padded frames.
+uint32_t fw_stride(const mlem_ctx* c, uint32_t B) { return c->mirrored ? B : projection_stride(B); }
+uint32_t bk_stride(const mlem_ctx* c, uint32_t B) {
+    return c->mirrored || !c->has_csc ? B : projection_stride(B);
+}
+}  // namespace
+
 int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* stream) {
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t Bd = c->mirrored ? B : projection_stride(B);
+    uint32_t Bd = fw_stride(c, B);
     if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
     const float* xd = x;
-    float* yd = y;
     if (c->bricked || Bd != B) {
         TRY(perm_scratch(c, (size_t)c->C * Bd));
         CK(c, permute_to_device(x, c->pscratch[0], c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
         xd = c->pscratch[0];
-        if (Bd != B) yd = c->rscratch;
     }
-    const LaunchCfg cfg = cfg_for_frames(c, Bd);
-    if (c->mirrored) {
-        CK(c, cudaMemsetAsync(y, 0, (size_t)c->R * B * 4, st));
-        for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
-            CK(c, mirror_fwproj(csr_visit(c, c->tuning), c->mirror, xd, B, f0, cfg.frame_tile, y,
-                                c->n_sm, c->tuning.blocks_per_sm, st));
-        return MLEM_OK;
-    }
-    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile)
-        CK(c, fwproj(csr_view(c), xd, Bd, f0, nullptr, nullptr, yd, cfg, st));
-    if (Bd != B) CK(c, permute_to_natural(yd, y, nullptr, c->R, B, Bd, st));
+    TRY(project_rows(c, xd, Bd != B ? c->rscratch : y, Bd, st));
+    if (Bd != B) CK(c, permute_to_natural(c->rscratch, y, nullptr, c->R, B, Bd, st));
     return MLEM_OK;
 }
 
@@ -2665,10 +2698,8 @@ int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* strea
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    // only the gather pass takes padded frames
-    uint32_t Bd = c->mirrored || !c->has_csc ? B : projection_stride(B);
+    uint32_t Bd = bk_stride(c, B);
     if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
-    const LaunchCfg cfg = cfg_for_frames(c, Bd);
     const float* yd = y;
     float* xd = x;
     if (c->bricked || Bd != B) {
@@ -2679,20 +2710,35 @@ int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* strea
         CK(c, permute_to_device(y, c->rscratch, nullptr, c->R, B, Bd, st));
         yd = c->rscratch;
     }
-    for (uint32_t f0 = 0; f0 < Bd; f0 += (uint32_t)cfg.frame_tile) {
-        if (c->mirrored) {
-            if (f0 == 0) CK(c, cudaMemsetAsync(xd, 0, (size_t)c->C * B * 4, st));
-            CK(c, mirror_bkproj(csr_visit(c, c->tuning), c->mirror, y, nullptr, B, f0,
-                                cfg.frame_tile, xd, c->n_sm, c->tuning.blocks_per_sm, st));
-        } else if (c->has_csc) {
-            CK(c, bkproj_csc(csc_view(c), yd, Bd, f0, nullptr, nullptr, xd, cfg, st));
-        } else {
-            if (f0 == 0) CK(c, cudaMemsetAsync(xd, 0, (size_t)c->C * B * 4, st));
-            CK(c, bkproj_scatter(csr_visit(c, c->tuning), y, B, f0, xd, cfg, st));
-        }
-    }
+    TRY(project_columns(c, yd, xd, Bd, st));
     if (xd != x)
         CK(c, permute_to_natural(xd, x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+    return MLEM_OK;
+}
+
+int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* stream) {
+    if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
+    TRY(set_device(c));
+    cudaStream_t st = (cudaStream_t)stream;
+    const uint32_t Bd = fw_stride(c, B);
+    if (!room_for_padding(c, Bd, st))
+        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
+    CK(c, interleave_f32(x, c->pscratch[0], c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
+    TRY(project_rows(c, c->pscratch[0], c->rscratch, Bd, st));
+    CK(c, deinterleave_f32(c->rscratch, y, c->R, B, Bd, nullptr, st));
+    return MLEM_OK;
+}
+
+int mlem_bkproj_frames_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
+    if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
+    TRY(set_device(c));
+    cudaStream_t st = (cudaStream_t)stream;
+    const uint32_t Bd = bk_stride(c, B);
+    if (!room_for_padding(c, Bd, st))
+        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
+    CK(c, interleave_f32(y, c->rscratch, c->R, B, Bd, nullptr, st));
+    TRY(project_columns(c, c->rscratch, c->pscratch[0], Bd, st));
+    CK(c, deinterleave_f32(c->pscratch[0], x, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
     return MLEM_OK;
 }
 

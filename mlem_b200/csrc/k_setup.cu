@@ -2,6 +2,7 @@
 // deterministic CSR -> CSC transpose, matrix validation, image statistics,
 // frame-layout transposes, and the synthetic Siddon generator on the device.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -399,27 +400,41 @@ __global__ void k_count_sums(const int32_t* __restrict__ s, uint64_t total, uint
     }
 }
 
-template <typename T>
+// Frame-major [B][n] <-> interleaved [n][Bp], V frames per access on the
+// interleaved side; a thread keeps to one item, so the frame-major side is
+// coalesced and no thread divides an index.  Pad frames are written as 0.
+template <typename T, int V>
+struct alignas(V * sizeof(T)) FrameVec {
+    T v[V];
+};
+
+template <typename T, int V>
 __global__ void k_interleave(const T* __restrict__ in, T* __restrict__ out, uint64_t n, uint32_t B,
                              uint32_t Bp, const uint32_t* __restrict__ perm) {
-    const uint64_t total = n * B;
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < total;
-         j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = j / n, i = j - b * n;
-        const uint64_t d = perm ? perm[i] : i;
-        out[d * Bp + b] = in[j];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        T* to = out + (perm ? (uint64_t)perm[i] : i) * Bp;
+        for (uint32_t b0 = 0; b0 < Bp; b0 += V) {
+            FrameVec<T, V> f;
+#pragma unroll
+            for (int k = 0; k < V; ++k) f.v[k] = b0 + k < B ? in[(uint64_t)(b0 + k) * n + i] : T(0);
+            *reinterpret_cast<FrameVec<T, V>*>(to + b0) = f;
+        }
     }
 }
 
-template <typename T>
+template <typename T, int V>
 __global__ void k_deinterleave(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
                                uint32_t B, uint32_t Bp, const uint32_t* __restrict__ perm) {
-    const uint64_t total = n * B;
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < total;
-         j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = j / n, i = j - b * n;
-        const uint64_t d = perm ? perm[i] : i;
-        out[j] = in[d * Bp + b];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const T* from = in + (perm ? (uint64_t)perm[i] : i) * Bp;
+        for (uint32_t b0 = 0; b0 < B; b0 += V) {
+            const FrameVec<T, V> f = *reinterpret_cast<const FrameVec<T, V>*>(from + b0);
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                if (b0 + k < B) out[(uint64_t)(b0 + k) * n + i] = f.v[k];
+        }
     }
 }
 
@@ -678,25 +693,37 @@ cudaError_t count_sums(const int32_t* sino, uint64_t R, uint32_t Bp, unsigned lo
     return cudaGetLastError();
 }
 
+namespace {
+template <typename T, bool TO_FRAMES>
+cudaError_t run_interleave(const T* in, T* out, uint64_t n, uint32_t B, uint32_t Bp,
+                           const uint32_t* perm, cudaStream_t st) {
+    if (n * B == 0) return cudaSuccess;
+    const unsigned grid = elementwise_grid(n);
+    auto go = [&](auto v) {
+        constexpr int V = decltype(v)::value;
+        if (TO_FRAMES) k_deinterleave<T, V><<<grid, 256, 0, st>>>(in, out, n, B, Bp, perm);
+        else k_interleave<T, V><<<grid, 256, 0, st>>>(in, out, n, B, Bp, perm);
+        return cudaGetLastError();
+    };
+    if (Bp % 4 == 0) return go(std::integral_constant<int, 4>{});
+    if (Bp % 2 == 0) return go(std::integral_constant<int, 2>{});
+    return go(std::integral_constant<int, 1>{});
+}
+}  // namespace
+
 cudaError_t interleave_i32(const int32_t* in, int32_t* out, uint64_t n, uint32_t B, uint32_t Bp,
                            cudaStream_t st) {
-    if (n * B == 0) return cudaSuccess;
-    k_interleave<int32_t><<<elementwise_grid(n * B), 256, 0, st>>>(in, out, n, B, Bp, nullptr);
-    return cudaGetLastError();
+    return run_interleave<int32_t, false>(in, out, n, B, Bp, nullptr, st);
 }
 
 cudaError_t interleave_f32(const float* in, float* out, uint64_t n, uint32_t B, uint32_t Bp,
                            const uint32_t* perm, cudaStream_t st) {
-    if (n * B == 0) return cudaSuccess;
-    k_interleave<float><<<elementwise_grid(n * B), 256, 0, st>>>(in, out, n, B, Bp, perm);
-    return cudaGetLastError();
+    return run_interleave<float, false>(in, out, n, B, Bp, perm, st);
 }
 
 cudaError_t deinterleave_f32(const float* in, float* out, uint64_t n, uint32_t B, uint32_t Bp,
                              const uint32_t* perm, cudaStream_t st) {
-    if (n * B == 0) return cudaSuccess;
-    k_deinterleave<float><<<elementwise_grid(n * B), 256, 0, st>>>(in, out, n, B, Bp, perm);
-    return cudaGetLastError();
+    return run_interleave<float, true>(in, out, n, B, Bp, perm, st);
 }
 
 namespace {

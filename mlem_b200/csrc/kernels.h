@@ -215,8 +215,8 @@ cudaError_t count_sums(const int32_t* sino, uint64_t R, uint32_t Bp, unsigned lo
                        unsigned long long* mags, cudaStream_t st);
 
 // ---- layout helpers -------------------------------------------------------
-// out[p(i)*Bp + b] = in[b*n + i] for b < B (n items per frame; pad frames
-// untouched), and back: out[b*n + i] = in[p(i)*Bp + b], where p = perm
+// out[p(i)*Bp + b] = in[b*n + i] for b < B (n items per frame), 0 in the pad
+// frames, and back: out[b*n + i] = in[p(i)*Bp + b], where p = perm
 // (natural -> device order) or the identity when perm is null.
 cudaError_t interleave_i32(const int32_t* in, int32_t* out, uint64_t n, uint32_t B, uint32_t Bp,
                            cudaStream_t st);

@@ -51,18 +51,31 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+def _projected(ctx, v, n_out, frames_call, call):
+    """A projection of v, [n] or [B, n], by the frame-major entry point; where its
+    scratch finds no room, through interleaved copies."""
+    if v.dim() == 2 and v.shape[0] > 1:
+        src = v.contiguous()
+        out = torch.empty((v.shape[0], n_out), dtype=torch.float32, device=v.device)
+        try:
+            frames_call(src.data_ptr(), out.data_ptr(), v.shape[0], _stream())
+            return out
+        except api.MlemError as e:
+            if e.status != api.MLEM_ERR_NOMEM:
+                raise
+    vi, B = _frames(v)
+    out = torch.empty((n_out, B), dtype=torch.float32, device=v.device)
+    call(vi.data_ptr(), out.data_ptr(), B, _stream())
+    return _unframes(out, B, v.dim() > 1)
+
+
 def _fw(ctx: "api.Context", x: torch.Tensor) -> torch.Tensor:
-    xi, B = _frames(_check(x, ctx.n_cols, "image"))
-    y = torch.empty((ctx.n_rows, B), dtype=torch.float32, device=x.device)
-    ctx.fwproj_d(xi.data_ptr(), y.data_ptr(), B, _stream())
-    return _unframes(y, B, x.dim() > 1)
+    return _projected(ctx, _check(x, ctx.n_cols, "image"), ctx.n_rows, ctx.fwproj_frames_d, ctx.fwproj_d)
 
 
 def _bk(ctx: "api.Context", y: torch.Tensor) -> torch.Tensor:
-    yi, B = _frames(_check(y, ctx.n_rows, "projection"))
-    x = torch.empty((ctx.n_cols, B), dtype=torch.float32, device=y.device)
-    ctx.bkproj_d(yi.data_ptr(), x.data_ptr(), B, _stream())
-    return _unframes(x, B, y.dim() > 1)
+    return _projected(ctx, _check(y, ctx.n_rows, "projection"), ctx.n_cols, ctx.bkproj_frames_d,
+                      ctx.bkproj_d)
 
 
 class _ForwardProject(torch.autograd.Function):

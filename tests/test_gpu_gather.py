@@ -129,3 +129,28 @@ def test_pipelined_one_pass_against_float64(visit, rows):
             got = u.cpu().numpy().astype(np.float64)
             # n terms, each with its factor's error: a sum of at most 4096 products and a division
             assert np.all(np.abs(got - ref[:, 0]) <= 2.0 ** -23 * (cnt[:, 0] + 4096 + 4) * mag[:, 0])
+
+
+@pytest.mark.parametrize("flags", [0, api.FLAG_NATURAL_LAYOUT, api.FLAG_NO_CSC])
+def test_frame_major_projections(flags):
+    """mlem_fwproj_frames_d / mlem_bkproj_frames_d against the interleaved entry
+    points, padded and unpadded frame counts: the same kernels over the same
+    device vectors, so the same bits (within rounding where rows are scattered)."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(5)
+    m = matrix("many-rows", rng)
+    st = torch.cuda.current_stream().cuda_stream
+    with api.Context.from_matrix(m, flags=flags) as ctx:
+        for B in (1, 2, 3, 6, 16, 19):
+            for n_in, n_out, frames, inter in ((m.n_cols, m.n_rows, ctx.fwproj_frames_d, ctx.fwproj_d),
+                                               (m.n_rows, m.n_cols, ctx.bkproj_frames_d, ctx.bkproj_d)):
+                v = torch.from_numpy(rng.uniform(0.1, 1.0, (B, n_in)).astype(np.float32)).cuda()
+                a = torch.full((B, n_out), np.nan, device="cuda")
+                b = torch.full((n_out, B), np.nan, device="cuda")
+                frames(v.data_ptr(), a.data_ptr(), B, st)
+                vi = v.t().contiguous()
+                inter(vi.data_ptr(), b.data_ptr(), B, st)
+                if flags & api.FLAG_NO_CSC and n_in == m.n_rows:
+                    assert torch.allclose(a, b.t(), rtol=1e-4, atol=1e-5)
+                else:
+                    assert torch.equal(a, b.t())
