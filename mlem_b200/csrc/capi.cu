@@ -85,6 +85,8 @@ SparseView csr_view(const mlem_ctx* c) {
     SparseView v{c->row_ptr, reinterpret_cast<const uint4*>(c->elems), c->R, c->Z,
                  c->row_order, c->row_order ? c->row_ranges : nullptr};
     v.max_len = c->max_row_len;
+    // every row in one batch, or nearly all of them
+    v.short_rows = c->max_row_len <= 256 || (c->Z <= 128ull * c->R && c->max_row_len <= 4096);
     return v;
 }
 }  // namespace mlem
@@ -710,6 +712,7 @@ int alloc_frames(mlem_ctx* c, uint32_t B) {
                                              c->tuning.bk_mode == MLEM_BK_ATOMIC);
     c->tuning.frame_tile = std::min(c->tuning.frame_tile > 0 && !follows ? c->tuning.frame_tile : 16,
                                     default_tile(Bp));
+    c->one_pass.frame_tile = std::min(c->one_pass.frame_tile, default_tile(Bp));
     c->graph_dirty = true;
     return MLEM_OK;
 }
@@ -906,6 +909,17 @@ int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, const f
 }
 int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, cudaStream_t st) {
     return fused_pass(c, t, csr, c->x, c->sino, c->update, c->Bp, c->counter, st);
+}
+
+// The tuning a run takes: the context's, or the autotuner's one-pass tuning
+// (mlem_ctx::one_pass) where it chose the CSC method in visiting order: for ordered
+// subsets, and while there is no cut copy of the current sinograms -- in steps of
+// one iteration per sinogram (plain-full: 2.24 ms a streamed step against 2.57 for
+// the CSC method over every entry) and in what follows them.
+const mlem_tuning& tuning_for(const mlem_ctx* c, bool steps) {
+    const bool instead = c->has_one_pass && csc_by_visit(c, c->tuning) &&
+                         (steps || c->n_subsets > 1 || (c->tuned_cut && !c->csc_act_ready));
+    return instead ? c->one_pass : c->tuning;
 }
 
 // The census is one launch in the two-pass methods without an update kernel of
@@ -1173,14 +1187,14 @@ void phase_bytes_for(const mlem_ctx* c, int bk_mode, int frame_tile, double* byt
         const double S = (double)c->n_subsets;
         bytes[0] = tiles * csr_pass + B * 4.0 * R + S * B * 8.0 * C +
                    S * (8.0 * C + B * 16.0 * C);
-        launches[0] = (int)S * ((chunk_visit(c->tuning.visit) ? 1 : nt) + 1);
+        launches[0] = (int)S * ((chunk_visit(tuning_for(c, false).visit) ? 1 : nt) + 1);
         bytes[3] = 4.0 * C * B;
         launches[3] = 2;
         return;
     }
     if (mode == MLEM_BK_FUSED) {
         bytes[0] = tiles * csr_pass + B * (4.0 * C + 4.0 * R + 4.0 * C);  // x, sino, update
-        launches[0] = (!exact && chunk_visit(c->tuning.visit)) ? 1 : nt;
+        launches[0] = (!exact && chunk_visit(tuning_for(c, false).visit)) ? 1 : nt;
         if (!exact && c->n_long) launches[0] += 2;  // the long-row kernels
     } else {
         bytes[0] = tiles * csr_pass + B * (4.0 * C + 4.0 * R + 4.0 * R);  // x, sino, correl
@@ -1211,8 +1225,8 @@ void voxel_permutation(uint32_t nx, uint32_t ny, uint32_t nz, std::vector<uint32
 namespace {
 
 void phase_bytes(const mlem_ctx* c, double* bytes, int* launches) {
-    phase_bytes_for(c, c->tuning.bk_mode, c->tuning.frame_tile, bytes, launches,
-                    c->tuning.visit != MLEM_VISIT_FILE);
+    const mlem_tuning& t = tuning_for(c, false);
+    phase_bytes_for(c, t.bk_mode, t.frame_tile, bytes, launches, t.visit != MLEM_VISIT_FILE);
 }
 
 }  // namespace
@@ -1247,14 +1261,14 @@ void drop_graph(mlem_ctx* c) {
 
 // Capture `n` iterations (slot reset + n x (iteration + statistics), or the
 // iterations alone) into *out.
-int capture_into(mlem_ctx* c, int n, bool stats, cudaGraphExec_t* out) {
+int capture_into(mlem_ctx* c, const mlem_tuning& t, int n, bool stats, cudaGraphExec_t* out) {
     CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int s = MLEM_OK;
     cudaError_t e = stats ? cudaMemsetAsync(c->stats_slot, 0, sizeof(unsigned int), c->stream)
                           : cudaSuccess;
     if (e != cudaSuccess) s = fail(c, MLEM_ERR_CUDA, "capture memset: %s", cudaGetErrorString(e));
     c->census_out = false;
-    for (int i = 0; i < n && s == MLEM_OK; ++i) s = enqueue_iteration(c, c->tuning, stats);
+    for (int i = 0; i < n && s == MLEM_OK; ++i) s = enqueue_iteration(c, t, stats);
     if (s == MLEM_OK) s = join_census(c);
     c->census_out = false;
     cudaGraph_t g = nullptr;
@@ -1270,13 +1284,20 @@ int capture_into(mlem_ctx* c, int n, bool stats, cudaGraphExec_t* out) {
     return MLEM_OK;
 }
 
-int capture(mlem_ctx* c, int n, bool stats) {
+int capture(mlem_ctx* c, const mlem_tuning& t, int n, bool stats) {
     drop_graph(c);
-    TRY(capture_into(c, n, stats, &c->graph));
+    TRY(capture_into(c, t, n, stats, &c->graph));
     c->graph_iters = n;
     c->graph_stats = stats;
+    c->graph_one_pass = &t == &c->one_pass;
     c->graph_dirty = false;
     return MLEM_OK;
+}
+
+// Whether the captured graph is n iterations of tuning t (with the census or not).
+bool graph_is(const mlem_ctx* c, const mlem_tuning& t, int n, bool stats) {
+    return !c->graph_dirty && c->graph && c->graph_iters == n && c->graph_stats == stats &&
+           c->graph_one_pass == (&t == &c->one_pass);
 }
 
 int ensure_tmp(mlem_ctx* c) {
@@ -1788,16 +1809,17 @@ int mlem_set_stream(mlem_ctx* c, void* stream) {
 int mlem_kernels_per_iteration(const mlem_ctx* c, int* n) {
     if (!c || !n) return fail(nullptr, MLEM_ERR_INVALID, "null argument");
     if (!c->Bp) return fail(const_cast<mlem_ctx*>(c), MLEM_ERR_STATE, "no frames");
-    const int tiles = (int)(c->Bp / (uint32_t)c->tuning.frame_tile);
-    int k = stats_in_one(c, c->tuning.bk_mode) ? 1 : 2;  // image statistics
+    const mlem_tuning& t = tuning_for(c, false);
+    const int tiles = (int)(c->Bp / (uint32_t)t.frame_tile);
+    int k = stats_in_one(c, t.bk_mode) ? 1 : 2;  // image statistics
     if (c->flags & MLEM_FLAG_EXACT) k += 2;
-    else if (c->tuning.bk_mode == MLEM_BK_CSC) k += 2 * tiles;
-    else if (c->tuning.bk_mode == MLEM_BK_ATOMIC) k += 2 * tiles + 1;
-    else if (c->tuning.bk_mode == MLEM_BK_REGION) k += 2 * tiles + 1;  // + correl
-    else if (c->tuning.bk_mode == MLEM_BK_MIRRORED) k += 2 * tiles + 1;  // + update
+    else if (t.bk_mode == MLEM_BK_CSC) k += 2 * tiles;
+    else if (t.bk_mode == MLEM_BK_ATOMIC) k += 2 * tiles + 1;
+    else if (t.bk_mode == MLEM_BK_REGION) k += 2 * tiles + 1;  // + correl
+    else if (t.bk_mode == MLEM_BK_MIRRORED) k += 2 * tiles + 1;  // + update
     else if (c->n_subsets > 1)  // per subset: the one-pass launch(es) and the update
-        k += (int)c->n_subsets * ((chunk_visit(c->tuning.visit) ? 1 : tiles) + 1);
-    else if (chunk_visit(c->tuning.visit)) k += 2 + (c->n_long ? 2 : 0);  // all tiles in one launch
+        k += (int)c->n_subsets * ((chunk_visit(t.visit) ? 1 : tiles) + 1);
+    else if (chunk_visit(t.visit)) k += 2 + (c->n_long ? 2 : 0);  // all tiles in one launch
     else k += tiles + 1 + (c->n_long ? 2 : 0);
     *n = k;
     return MLEM_OK;
@@ -2001,14 +2023,14 @@ int mlem_iterate(mlem_ctx* c, int n, double* sums, uint64_t* zeros, uint64_t* su
     if (!c->images_ready) return fail(c, MLEM_ERR_STATE, "images not initialised");
     if (n == 0) return MLEM_OK;
     TRY(set_device(c));
-    if (c->tuning.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
-        TRY(ensure_region(c, c->tuning.frame_tile));
+    const mlem_tuning& t = tuning_for(c, false);
+    if (t.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
+        TRY(ensure_region(c, t.frame_tile));
     // Chunks of up to 64 iterations, each one graph launch.
     const int chunk = std::min(n, 64);
     const bool stats = sums || zeros || subn;  // the census only when the caller takes it
     TRY(ensure_history(c, chunk));
-    if (c->graph_dirty || !c->graph || c->graph_iters != chunk || c->graph_stats != stats)
-        TRY(capture(c, chunk, stats));
+    if (!graph_is(c, t, chunk, stats)) TRY(capture(c, t, chunk, stats));
     int done = 0;
     while (done < n) {
         const int k = std::min(chunk, n - done);
@@ -2016,7 +2038,7 @@ int mlem_iterate(mlem_ctx* c, int n, double* sums, uint64_t* zeros, uint64_t* su
             CK(c, cudaGraphLaunch(c->graph, c->stream));
         } else {
             if (stats) CK(c, cudaMemsetAsync(c->stats_slot, 0, 4, c->stream));
-            for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, c->tuning, stats));
+            for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, t, stats));
             TRY(join_census(c));
         }
         // the census of the chunk: through page-locked memory, one wait for all of it
@@ -2068,11 +2090,12 @@ int mlem_step_host(mlem_ctx* c, const int32_t* sino, float* images, uint32_t B) 
     }
     TRY(upload_frames<float>(c, images, c->x, c->C));
     c->images_ready = true;
-    if (c->tuning.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
-        TRY(ensure_region(c, c->tuning.frame_tile));
-    if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
+    const mlem_tuning& t = tuning_for(c, true);
+    if (t.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
+        TRY(ensure_region(c, t.frame_tile));
+    if (!graph_is(c, t, 1, false)) {
         TRY(ensure_history(c, 1));
-        TRY(capture(c, 1, false));
+        TRY(capture(c, t, 1, false));
     }
     CK(c, cudaGraphLaunch(c->graph, c->stream));
     TRY(download_images(c, images));
@@ -2133,9 +2156,10 @@ static int stream_steps(mlem_ctx* c, const int32_t* const* sinos, float* const* 
         CK(c, cudaEventRecord(c->ev_sfree[cur], c->stream));
         TRY(build_active(c, false, false));
         ++c->sino_gen;
-        if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
+        const mlem_tuning& t = tuning_for(c, true);
+        if (!graph_is(c, t, 1, false)) {
             TRY(ensure_history(c, 1));
-            TRY(capture(c, 1, false));
+            TRY(capture(c, t, 1, false));
         }
         CK(c, cudaGraphLaunch(c->graph, c->stream));
         if (images && images[k]) {  // this iteration's images, once the buffer's last download is done
@@ -2209,13 +2233,14 @@ static int stream_steps_overlap(mlem_ctx* c, const int32_t* const* sinos, float*
         c->csc_act_ready = false;
         c->graph_dirty = true;
     }
-    if (c->graph_dirty || !c->graph || c->graph_iters != 1 || c->graph_stats) {
+    const mlem_tuning& t = tuning_for(c, true);
+    if (!graph_is(c, t, 1, false)) {
         TRY(ensure_history(c, 1));
-        TRY(capture(c, 1, false));
+        TRY(capture(c, t, 1, false));
     }
     if (!c->graph_alt) {
         swap_sets(c);
-        const int s = capture_into(c, 1, false, &c->graph_alt);
+        const int s = capture_into(c, t, 1, false, &c->graph_alt);
         swap_sets(c);
         TRY(s);
     }
@@ -2280,8 +2305,9 @@ int mlem_stream_host(mlem_ctx* c, const int32_t* const* sinos, float* const* ima
     if (!c->images_ready) return fail(c, MLEM_ERR_STATE, "images not initialised");
     TRY(set_device(c));
     TRY(ensure_streaming(c));
-    if (c->tuning.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
-        TRY(ensure_region(c, c->tuning.frame_tile));
+    const mlem_tuning& t = tuning_for(c, true);
+    if (t.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
+        TRY(ensure_region(c, t.frame_tile));
     if (c->act_ready && !c->act_host &&
         cudaHostAlloc(reinterpret_cast<void**>(&c->act_host), 16, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
@@ -2317,8 +2343,9 @@ int mlem_profile_phases(mlem_ctx* c, int n, double* ms, double* bytes, int* laun
     if (!c->images_ready) return fail(c, MLEM_ERR_STATE, "images not initialised");
     TRY(set_device(c));
     TRY(ensure_history(c, 1));
-    if (c->tuning.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
-        TRY(ensure_region(c, c->tuning.frame_tile));
+    const mlem_tuning& t = tuning_for(c, false);
+    if (t.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
+        TRY(ensure_region(c, t.frame_tile));
     std::vector<PhaseEvents> evs((size_t)n);
     for (auto& pe : evs)
         for (auto& e : pe.ev) CK(c, cudaEventCreate(&e));
@@ -2327,7 +2354,7 @@ int mlem_profile_phases(mlem_ctx* c, int n, double* ms, double* bytes, int* laun
         if (cudaMemsetAsync(c->stats_slot, 0, 4, c->stream) != cudaSuccess)
             s = fail(c, MLEM_ERR_CUDA, "memset");
         else
-            s = enqueue_iteration(c, c->tuning, true, &evs[(size_t)i]);
+            s = enqueue_iteration(c, t, true, &evs[(size_t)i]);
     }
     if (s == MLEM_OK && cudaStreamSynchronize(c->stream) != cudaSuccess)
         s = fail(c, MLEM_ERR_CUDA, "synchronize");
@@ -2410,6 +2437,7 @@ int mlem_set_tuning(mlem_ctx* c, const mlem_tuning* t) {
         }
     }
     c->tuning = n;
+    c->has_one_pass = false;
     c->tile_follows = false;
     c->graph_dirty = true;
     return MLEM_OK;
@@ -2454,6 +2482,7 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
     CK(c, cudaEventCreate(&e1));
     mlem_tuning best = c->tuning;
     best.ms_per_iter = 1e30;
+    mlem_tuning one_pass = best;
     const mlem_tuning orig = c->tuning;
     for (int mode : modes)
         for (int group : {8, 16, 32})
@@ -2496,6 +2525,7 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
                     CK(c, cudaEventElapsedTime(&ms, e0, e1));
                     t.ms_per_iter = ms / 2.0;
                     if (t.ms_per_iter < best.ms_per_iter) best = t;
+                    if (mode == MLEM_BK_FUSED && t.ms_per_iter < one_pass.ms_per_iter) one_pass = t;
                     CK(c, cudaMemcpyAsync(c->x, saved, xb, cudaMemcpyDeviceToDevice, c->stream));
                 }
             }
@@ -2510,6 +2540,9 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
     if (!csc_by_visit(c, best) && c->celems_vis)  // tried, not chosen: give the memory back
         free_csc_vis(c);
     c->tuning = best;
+    c->one_pass = one_pass;
+    c->tuned_cut = c->csc_act_ready;
+    c->has_one_pass = one_pass.bk_mode == MLEM_BK_FUSED && one_pass.ms_per_iter < 1e30;
     c->tile_follows = false;
     c->graph_dirty = true;
     if (best_out) *best_out = best;
@@ -2814,7 +2847,7 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
         return MLEM_OK;
     }
     // the context's one-pass tuning when it has one, else sorted rows in chunks
-    mlem_tuning t = c->tuning;
+    mlem_tuning t = c->has_one_pass ? c->one_pass : c->tuning;
     if (t.bk_mode != MLEM_BK_FUSED) {
         t.visit = c->row_order ? MLEM_VISIT_SORTED_CHUNKED : MLEM_VISIT_FILE;
         t.blocks_per_sm = c->row_order ? 4 : 8;

@@ -187,10 +187,17 @@ struct mlem_ctx {
     size_t rb_bytes = 0;
 
     mlem_tuning tuning{};
+    // The best one-pass tuning the autotuner saw, where it chose the CSC method in
+    // visiting order: what runs where that method cannot (ordered subsets) or pays
+    // for a cut copy it cannot use (one iteration per sinogram).
+    mlem_tuning one_pass{};
+    bool has_one_pass = false;
+    bool tuned_cut = false;  // the chosen method was timed over the cut copy
     bool tile_follows = true;  // no tuning chosen yet: the frame tile follows the frame count
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     bool graph_stats = false;  // the graph holds the census
+    bool graph_one_pass = false;  // the graph was captured with one_pass, not tuning
     bool graph_dirty = true;
 
     std::string err;

@@ -201,7 +201,7 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
     if (!csr.order || !csr.vrange) return cudaErrorInvalidValue;  // a sorted visit
     // the resident CTAs: 64 registers x 1024 threads per SM, in 1, 2 or 4 CTAs
     const int grid = std::max(1, sm_count * ctas_per_sm), threads = 1024 / ctas_per_sm;
-    if (B == 1 && csr.max_len != ~0u)
+    if (B == 1 && csr.short_rows)
         return launch_dependent(csr.n <= kDependentMost, k_fused_chunked_one, grid, threads, 0, st, csr, x, sino, u, chunk_rows, counter);
     switch (frame_tile) {
         case 1: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);

@@ -348,7 +348,7 @@ cudaError_t fused_row(const SparseView& csr, const float* x, uint32_t B, uint32_
     if (!cfg_valid(cfg) || (B % cfg.frame_tile) || (f0 % cfg.frame_tile)) return cudaErrorInvalidValue;
     if (csr.n == 0) return cudaSuccess;
     if (csr.order && !csr.vrange) return cudaErrorInvalidValue;  // sorted visits carry vrange
-    if (csr.vrange && B == 1 && cfg.group == 32 && csr.max_len != ~0u) {
+    if (csr.vrange && B == 1 && cfg.group == 32 && csr.short_rows) {
         // the resident CTAs: rows in flight from the first to the last
         const int grid = std::min(cfg.blocks_per_sm, 4) * cfg.sm_count;
         return launch_dependent(csr.n <= kDependentMost, k_fused_row_one, grid, 256, 0, st, csr, x, sino, u);

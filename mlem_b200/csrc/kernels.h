@@ -50,6 +50,9 @@ struct SparseView {
     // The longest row (column), for the gather passes' choice of lanes; ~0 when
     // unknown.
     uint32_t max_len = ~0u;
+    // The rows fit the pipelined one-frame one-pass walk (one_pass_rows), which
+    // handles 256 elements of a row at once and the rest one load at a time.
+    bool short_rows = false;
     // The gather passes walk a row from the memory line it starts in, so that the
     // grouping of its sum depends on where it is stored.  Not with the CSC in file
     // order, whose sums do not depend on the voxel layout.

@@ -1,0 +1,70 @@
+"""An autotuned context that chose the CSC method in visiting order: what that
+method cannot run, or has no cut copy for, runs on the best one-pass tuning the
+autotuner saw -- streamed and single host steps, the iterations after them, and
+ordered subsets -- and a tuning chosen by the caller is left alone."""
+import numpy as np
+import pytest
+
+from mlem_b200 import api, synth
+
+import oracle_bind as ob
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-4
+
+
+def test_autotuned_context_streams_steps_and_subsets():
+    # frames enough for the two-pass method to win the autotuner's comparison
+    g = synth.Geometry(64, 64, 32, 60000, 40, 200, seed=9)
+    m = synth.host_matrix(g)
+    rng = np.random.default_rng(2)
+    sinos = [rng.poisson(4, (4, g.n_rows)).astype(np.int32) for _ in range(3)]
+    for s in sinos:
+        s[:, rng.random(g.n_rows) < 0.3] = 0
+
+    def want(chain, n_after=0, subsets=1):
+        out = []
+        for b in range(4):
+            x = None
+            for s in chain:
+                x = ob.mlem(m, s[b], 1, start_image=x)[0]
+            if n_after:
+                x = (ob.mlem(m, chain[-1][b], n_after, start_image=x)[0] if subsets == 1 else
+                     ob.osem(m, chain[-1][b], n_after, subsets, start_image=x)[0])
+            out.append(x)
+        return out
+
+    def close(got, ref):
+        for b in range(4):
+            assert ob.rel_l2(got[b], ref[b]) <= TOL
+
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_sinograms(sinos[0])
+        ctx.init_images()
+        chosen = ctx.autotune()
+        ctx.init_images()
+        ctx.iterate(2)
+        close(ctx.get_images(), want([sinos[0]], 1))
+        ctx.set_sinograms(sinos[0])
+        ctx.init_images()
+        ctx.stream_host(sinos)
+        close(ctx.get_images(), want(sinos))
+        ctx.iterate(2)  # no cut copy of the last sinograms
+        close(ctx.get_images(), want(sinos, 2))
+        x = np.ascontiguousarray(want(sinos[:1]), np.float32)
+        ctx.step_host(sinos[1], x)
+        close(x, want(sinos[:2]))
+        ctx.set_sinograms(sinos[0])
+        ctx.init_images()
+        ctx.iterate(1)
+        if chosen["bk_mode"] in (api.BK_CSC, api.BK_FUSED):
+            ctx.set_subsets(3)
+            assert ctx.kernels_per_iteration() >= 6
+            ctx.iterate(2)
+            close(ctx.get_images(), want(sinos[:1], 2, 3))
+            ctx.set_subsets(1)
+        ctx.set_tuning(api.BK_CSC, 32, 4, 8, api.VISIT_SORTED)
+        ctx.set_subsets(3)
+        with pytest.raises(api.MlemError):  # the caller's own choice is refused, as before
+            ctx.iterate(1)
