@@ -74,13 +74,6 @@ namespace mlem {
 void dev_free(void* p) {
     if (p) cudaFree(p);
 }
-}  // namespace mlem
-
-namespace {
-
-}  // namespace
-
-namespace mlem {
 SparseView csr_view(const mlem_ctx* c) {
     SparseView v{c->row_ptr, reinterpret_cast<const uint4*>(c->elems), c->R, c->Z,
                  c->row_order, c->row_order ? c->row_ranges : nullptr};

@@ -33,7 +33,7 @@ __device__ __forceinline__ void adjoint_row_range(const SparseView& csr, const f
                                                   float* __restrict__ rows, float* __restrict__ u,
                                                   uint64_t r_begin, uint64_t r_end, uint64_t warp,
                                                   uint64_t nwarps) {
-    constexpr int kBatch = batch_depth<32, 1>();
+    constexpr int kBatch = batch_depth<32, 1, true>();
     const int lane = threadIdx.x & 31;
     const uint64_t ps = l2_evict_first(), ph = l2_evict_last();
     const uint2* el = reinterpret_cast<const uint2*>(csr.pairs);
@@ -56,7 +56,7 @@ __device__ __forceinline__ void adjoint_row_range(const SparseView& csr, const f
         }
         float acc[1];
         uint2 kept[kBatch];
-        const bool in_regs = row_dot<32, 1, true>(el, b, e, lane, x, 1, 0, acc, ps, ph, kept);
+        const bool in_regs = row_dot<32, 1, true, true, kBatch>(el, b, e, lane, x, 1, 0, acc, ps, ph, kept);
         slot_allreduce<32, 1>(acc);
         float h;
         if constexpr (OP == kOpRatio) {

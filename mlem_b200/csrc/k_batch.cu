@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch_interleaved(const Ba
 
 // One matrix in dynamically scheduled chunks of consecutive visiting
 // positions (the items schedule with uniform items and no item list).
-template <int BT>
+// kBatch: elements a lane holds at once (fused_row_range).
+template <int BT, int kBatch = batch_depth<32, BT, true>()>
 __global__ void __launch_bounds__(1024, 1) k_fused_chunked(SparseView csr,
                                                                      const float* __restrict__ x,
                                                                      uint32_t B,
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(1024, 1) k_fused_chunked(SparseView csr,
         const uint64_t r0 = ci * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
 #pragma unroll 1
         for (uint32_t f0 = 0; f0 < B; f0 += BT)
-            fused_row_range<32, BT, true>(csr, x, B, f0, sino, u, r0, r1, warp, nwarps);
+            fused_row_range<32, BT, true, kBatch>(csr, x, B, f0, sino, u, r0, r1, warp, nwarps);
     }
 }
 
@@ -203,6 +204,12 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
     const int grid = std::max(1, sm_count * ctas_per_sm), threads = 1024 / ctas_per_sm;
     if (B == 1 && csr.short_rows)
         return launch_dependent(csr.n <= kDependentMost, k_fused_chunked_one, grid, threads, 0, st, csr, x, sino, u, chunk_rows, counter);
+    // Four frames a pass, rows that eight elements a lane hold and four do not: eight, so
+    // that the row stays in registers for its scatter (1,048,576 rows of 200 elements
+    // 1,038 -> 1,005 to 1,018 us per iteration).  Other rows lose with eight (120,007 of
+    // odd lengths 84.7 -> 88.3 us, 400,000 of up to 470 1,068 -> 1,137).
+    if (frame_tile == 4 && csr.max_len <= 256 && csr.nnz > 128ull * csr.n)
+        return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<4, 8>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
     switch (frame_tile) {
         case 1: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
         case 2: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<2>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);

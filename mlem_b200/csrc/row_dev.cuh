@@ -164,13 +164,24 @@ __device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW
     }
 }
 
+// How a row's elements and gathers are loaded.  In a sorted visit neighbouring rows
+// share image lines and the loads are latency-bound: batches of volatile predicated
+// loads (eager).  In file order at four and more frames the rows share nothing and
+// the L2 is the limit: all of a batch at once made it 12 % slower than conditional
+// loads, which the compiler spaces out (1,048,576 rows: 16 frames 4,499 us eager,
+// 3,864 conditional; 4 frames 1,322 and 1,127).  At one frame, and at two with a
+// warp per row, eager is at least as fast in either order (two frames, 16 lanes: 992
+// and 963).
+template <int G, int BT, bool SORTED>
+constexpr bool eager_loads() { return SORTED || BT == 1 || (BT == 2 && G == 32); }
+
 // Elements a lane loads before it gathers (memory-level parallelism).  A
 // full-warp group takes 8 (a 150-250-element row is one batch) at one and two
-// frames; with four floats per lane 8 gathers and the kept elements would spill,
-// and narrower groups keep their registers, and so their occupancy, lower with 4
-// (measured on the plain-full workload).
-template <int G, int BT>
-constexpr int batch_depth() { return G == 32 && BT < 4 ? 8 : 4; }
+// frames and of conditional loads; with four floats per lane, and in narrower
+// groups, 4 eager ones keep the registers, and so the occupancy.  Kernels whose
+// rows want another depth at four frames pass their own.
+template <int G, int BT, bool EAGER>
+constexpr int batch_depth() { return G == 32 && (BT < 4 || !EAGER) ? 8 : 4; }
 
 // acc[0..VW) = sum over the row's elements of value * vec[col*B + off + ...].
 // Each batch issues all of its (predicated) element loads, then all of its
@@ -178,13 +189,12 @@ constexpr int batch_depth() { return G == 32 && BT < 4 ? 8 : 4; }
 // two per element.  When `keep` is non-null and the whole row fits in one
 // batch, the lane's elements are left in keep[] (fused kernel) and true is
 // returned.
-template <int G, int BT, bool KEEP>
+template <int G, int BT, bool KEEP, bool EAGER, int kBatch>
 __device__ __forceinline__ bool row_dot(const uint2* __restrict__ el, uint64_t b, uint64_t e,
                                         int lane, const float* __restrict__ vec, uint32_t B,
                                         uint32_t off, float (&acc)[Lanes<BT>::VW], uint64_t ps,
                                         uint64_t ph, uint2* keep = nullptr) {
     constexpr int VW = Lanes<BT>::VW, FL = Lanes<BT>::FL, EPS = G / FL;
-    constexpr int kBatch = batch_depth<G, BT>();
     const float* base = vec + off;
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[i] = 0.0f;
@@ -201,12 +211,26 @@ __device__ __forceinline__ bool row_dot(const uint2* __restrict__ el, uint64_t b
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const uint64_t k = k0 + (uint64_t)u * EPS;
-            q[u] = kL1 ? ld_elem_keep_if(el + k, k < e, ps) : ld_elem_if(el + k, k < e, ps);
+            if constexpr (EAGER) {
+                q[u] = kL1 ? ld_elem_keep_if(el + k, k < e, ps) : ld_elem_if(el + k, k < e, ps);
+            } else {
+                q[u] = make_uint2(0u, 0u);  // value 0: contributes nothing
+                if (k < e) q[u] = kL1 ? ld_keep2(el + k, ps) : ld_stream2(el + k, ps);
+            }
         }
         float xv[kBatch][VW];
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-            ld_vec_if<VW>(base + (size_t)q[u].x * B, k0 + (uint64_t)u * EPS < e, xv[u], ph);
+        for (int u = 0; u < kBatch; ++u) {
+            const bool in = k0 + (uint64_t)u * EPS < e;
+            if constexpr (EAGER) {
+                ld_vec_if<VW>(base + (size_t)q[u].x * B, in, xv[u], ph);
+            } else if (in) {
+                ld_vec<VW>(base + (size_t)q[u].x * B, xv[u], ph);
+            } else {
+#pragma unroll
+                for (int i = 0; i < VW; ++i) xv[u][i] = 0.0f;
+            }
+        }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
             const float v = __uint_as_float(q[u].y);
@@ -240,7 +264,8 @@ __device__ __forceinline__ void slot_allreduce(float (&acc)[Lanes<BT>::VW]) {
 // (csr.vrange); otherwise rows are visited in file order (csr.order null).
 // A compile-time choice: the file-order loop measured 2.49 vs 3.15 ms on the
 // plain-full matrix when the sorted path was a runtime branch inside it.
-template <int G, int BT, bool SORTED>
+// kBatch: elements a lane holds at once.
+template <int G, int BT, bool SORTED, int kBatch = batch_depth<G, BT, eager_loads<G, BT, SORTED>()>()>
 __device__ __forceinline__ void fused_row_range(const SparseView& csr, const float* __restrict__ x,
                                                 uint32_t B, uint32_t f0,
                                                 const int32_t* __restrict__ sino,
@@ -249,7 +274,6 @@ __device__ __forceinline__ void fused_row_range(const SparseView& csr, const flo
     // [r_begin, r_end) are visiting positions (rows in csr.order when set)
     constexpr int RPW = 32 / G;
     constexpr int VW = Lanes<BT>::VW, FL = Lanes<BT>::FL, EPS = G / FL;
-    constexpr int kBatch = batch_depth<G, BT>();
     const int lw = threadIdx.x & 31;
     const int lane = lw & (G - 1);
     const int sub = lane % FL;
@@ -286,7 +310,8 @@ __device__ __forceinline__ void fused_row_range(const SparseView& csr, const flo
         float acc[VW];
         uint2 kept[kBatch];
         const bool in_regs =
-            row_dot<G, BT, true>(el, b, e, lane, x, B, f0 + sub * VW, acc, ps, ph, kept);
+            row_dot<G, BT, true, eager_loads<G, BT, SORTED>(), kBatch>(el, b, e, lane, x, B,
+                                                                    f0 + sub * VW, acc, ps, ph, kept);
         slot_allreduce<G, BT>(acc);
         if (!active) continue;
         const uint64_t idx = r * B + f0 + sub * VW;

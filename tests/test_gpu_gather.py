@@ -131,6 +131,38 @@ def test_pipelined_one_pass_against_float64(visit, rows):
             assert np.all(np.abs(got - ref[:, 0]) <= 2.0 ** -23 * (cnt[:, 0] + 4096 + 4) * mag[:, 0])
 
 
+@pytest.mark.parametrize("visit", [api.VISIT_FILE, api.VISIT_SORTED, api.VISIT_SORTED_CHUNKED])
+@pytest.mark.parametrize("long_rows", [False, True])
+def test_four_frame_one_pass_against_float64(visit, long_rows):
+    """The one-pass walks at four frames at the edges of their 4-, 6- and 8-element
+    batches (128, 192 and 256 elements a row), with mean row lengths on both sides of
+    128: u = A^T (s / A x), each entry within the rounding of its terms."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(5)
+    R, C, B = 4000, 5000, 4
+    lens = rng.choice([0, 1, 31, 33, 127, 128, 129] + [191, 192, 193, 255, 256] * (2 * long_rows), R)
+    assert (lens.mean() > 128) == long_rows
+    end = np.cumsum(lens).astype(np.uint64)
+    el = np.zeros(int(end[-1]), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, C, el.size)
+    el["value"] = rng.uniform(0.05, 1.7, el.size)
+    m = formats.Csr4(R, C, end, el)
+    s = rng.poisson(3, (R, B)).astype(np.int32)
+    x = rng.uniform(0.1, 2.0, (C, B)).astype(np.float32)
+    f = sums(m, x, False)[0]
+    c = np.where(f != 0, s / np.where(f != 0, f, 1.0), 0.0)
+    ref, mag, cnt = sums(m, c, True)
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_tuning(api.BK_FUSED, 32, 4, 4, visit)
+        xd, sd = torch.from_numpy(x).cuda(), torch.from_numpy(s).cuda()
+        u = torch.full((C, B), np.nan, device="cuda")
+        ctx.fused_update_d(xd.data_ptr(), sd.data_ptr(), u.data_ptr(), B,
+                           torch.cuda.current_stream().cuda_stream)
+        got = u.cpu().numpy().astype(np.float64)
+    # n terms, each with its factor's error: a sum of at most 256 products and a division
+    assert np.all(np.abs(got - ref) <= 2.0 ** -23 * (cnt + 256 + 4) * mag)
+
+
 @pytest.mark.parametrize("flags", [0, api.FLAG_NATURAL_LAYOUT, api.FLAG_NO_CSC])
 def test_frame_major_projections(flags):
     """mlem_fwproj_frames_d / mlem_bkproj_frames_d against the interleaved entry
