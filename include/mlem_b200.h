@@ -348,9 +348,10 @@ int mlem_apply_update_d(mlem_ctx* ctx, const float* update, float* x, uint32_t n
                         void* stream);
 /* mlem_fwproj_d and mlem_bkproj_d on frame-major device vectors, x[B][C] and
  * y[B][R]: the frames are interleaved (and padded) on the way to the device
- * order and back, in one kernel each way.  Rows of scratch are kept in the
- * context; MLEM_ERR_NOMEM when they do not fit, or would have to be allocated
- * while the stream is being captured. */
+ * order and back, in one kernel each way.  The interleaved vectors are scratch
+ * kept in the context, and calls on several streams take turns with it;
+ * MLEM_ERR_NOMEM when it does not fit or the stream is being captured
+ * (mlem_fwproj_d and mlem_bkproj_d can be captured). */
 int mlem_fwproj_frames_d(mlem_ctx* ctx, const float* x, float* y, uint32_t n_frames, void* stream);
 int mlem_bkproj_frames_d(mlem_ctx* ctx, const float* y, float* x, uint32_t n_frames, void* stream);
 /* The two one-pass kernels of the unrolled MLEM's backward pass (one frame,

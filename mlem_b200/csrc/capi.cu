@@ -199,37 +199,48 @@ int perm_scratch(mlem_ctx* c, size_t floats) {
     return MLEM_OK;
 }
 
-// Row scratch (and voxel scratch) of Bd floats each for the projections' padded
-// frames; false where they do not fit beside the matrix or would have to be
-// allocated while the caller's stream is being captured, and the caller's frame
-// count is walked as it is.
-bool room_for_padding(mlem_ctx* c, uint32_t Bd, cudaStream_t st) {
-    const size_t rows = (size_t)std::max<uint32_t>(c->R, 1) * Bd;
-    if (c->rscratch_floats < rows || c->pscratch_floats < (size_t)c->C * Bd) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return false;
-        }
+// Voxel and row vectors of Bd frames for one projection of B caller frames on `st`
+// (frame_voxels, frame_rows); false where they do not fit beside the matrix or where the
+// stream is being captured (a graph may be replayed beside, or after, a call that
+// uses or replaces them), and the caller's frame count is walked as it is.  Calls
+// on several streams take turns: each waits for the last one's frame_room_done.
+bool frame_room(mlem_ctx* c, uint32_t B, uint32_t Bd, cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
     }
-    if (c->rscratch_floats < rows) {
-        if (c->rscratch) {
-            cudaFree(c->rscratch);
-            c->device_bytes -= c->rscratch_floats * 4;
-        }
-        c->rscratch = nullptr;
-        c->rscratch_floats = 0;
-        if (dev_alloc(c, &c->rscratch, rows) != MLEM_OK) {
-            c->err.clear();
-            return false;
-        }
-        c->rscratch_floats = rows;
-    }
-    if (perm_scratch(c, (size_t)c->C * Bd) != MLEM_OK) {
+    // what a later capture of the same call needs
+    if (c->bricked && perm_scratch(c, (size_t)c->C * B) != MLEM_OK) {
         c->err.clear();
         return false;
     }
+    const size_t voxels = (((size_t)c->C * Bd + 63) & ~(size_t)63), floats = voxels + (size_t)c->R * Bd;
+    if (c->fscratch_floats < floats) {
+        if (c->fscratch) {
+            cudaFree(c->fscratch);
+            c->device_bytes -= c->fscratch_floats * 4;
+        }
+        c->fscratch = nullptr;
+        c->fscratch_floats = 0;
+        if (dev_alloc(c, &c->fscratch, floats) != MLEM_OK) {
+            c->err.clear();
+            return false;
+        }
+        c->fscratch_floats = floats;
+    }
+    if ((!c->ev_frames && cudaEventCreateWithFlags(&c->ev_frames, cudaEventDisableTiming) != cudaSuccess) ||
+        cudaStreamWaitEvent(st, c->ev_frames, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     return true;
+}
+float* frame_voxels(mlem_ctx* c) { return c->fscratch; }
+float* frame_rows(mlem_ctx* c, uint32_t Bd) { return c->fscratch + (((size_t)c->C * Bd + 63) & ~(size_t)63); }
+int frame_room_done(mlem_ctx* c, cudaStream_t st) {
+    CK(c, cudaEventRecord(c->ev_frames, st));
+    return MLEM_OK;
 }
 
 // Region-blocked copy for the tile size `frame_tile` (built once per tile
@@ -1741,7 +1752,7 @@ void mlem_destroy(mlem_ctx* c) {
                     (void*)c->hist_zeros, (void*)c->hist_subn, (void*)c->tmp_r[0],
                     (void*)c->tmp_r[1], (void*)c->tmp_c[0], (void*)c->tmp_c[1], (void*)c->tmp_c[2],
                     (void*)c->tmp_sino, (void*)c->tmp_d, (void*)c->norm_nat, (void*)c->perm,
-                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->rscratch, (void*)c->row_order,
+                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->fscratch, (void*)c->row_order,
                     (void*)c->row_ranges, (void*)c->counter, (void*)c->long_segs, (void*)c->f_long_d,
                     (void*)c->sub_norm,
                     (void*)c->sub_file, (void*)c->sub_file_ranges, (void*)c->sub_sorted,
@@ -1760,7 +1771,7 @@ void mlem_destroy(mlem_ctx* c) {
     if (c->slots) cudaFreeHost(c->slots);
     for (cudaStream_t q : {c->up_stream, c->down_stream, c->side})
         if (q) { cudaStreamSynchronize(q); cudaStreamDestroy(q); }
-    for (cudaEvent_t e : {c->ev_image, c->ev_census})
+    for (cudaEvent_t e : {c->ev_image, c->ev_census, c->ev_frames})
         if (e) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) {
         dev_free(c->sstage[i]);
@@ -2707,38 +2718,40 @@ int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* strea
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t Bd = fw_stride(c, B);
-    if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
+    const uint32_t Bd = fw_stride(c, B);
+    if (Bd != B && frame_room(c, B, Bd, st)) {
+        CK(c, permute_to_device(x, frame_voxels(c), c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+        TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
+        CK(c, permute_to_natural(frame_rows(c, Bd), y, nullptr, c->R, B, Bd, st));
+        return frame_room_done(c, st);
+    }
     const float* xd = x;
-    if (c->bricked || Bd != B) {
-        TRY(perm_scratch(c, (size_t)c->C * Bd));
-        CK(c, permute_to_device(x, c->pscratch[0], c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+    if (c->bricked) {
+        TRY(perm_scratch(c, (size_t)c->C * B));
+        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
         xd = c->pscratch[0];
     }
-    TRY(project_rows(c, xd, Bd != B ? c->rscratch : y, Bd, st));
-    if (Bd != B) CK(c, permute_to_natural(c->rscratch, y, nullptr, c->R, B, Bd, st));
-    return MLEM_OK;
+    return project_rows(c, xd, y, B, st);
 }
 
 int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t Bd = bk_stride(c, B);
-    if (Bd != B && !room_for_padding(c, Bd, st)) Bd = B;
-    const float* yd = y;
+    const uint32_t Bd = bk_stride(c, B);
+    if (Bd != B && frame_room(c, B, Bd, st)) {
+        CK(c, permute_to_device(y, frame_rows(c, Bd), nullptr, c->R, B, Bd, st));
+        TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
+        CK(c, permute_to_natural(frame_voxels(c), x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+        return frame_room_done(c, st);
+    }
     float* xd = x;
-    if (c->bricked || Bd != B) {
-        TRY(perm_scratch(c, (size_t)c->C * Bd));
+    if (c->bricked) {
+        TRY(perm_scratch(c, (size_t)c->C * B));
         xd = c->pscratch[0];
     }
-    if (Bd != B) {
-        CK(c, permute_to_device(y, c->rscratch, nullptr, c->R, B, Bd, st));
-        yd = c->rscratch;
-    }
-    TRY(project_columns(c, yd, xd, Bd, st));
-    if (xd != x)
-        CK(c, permute_to_natural(xd, x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+    TRY(project_columns(c, y, xd, B, st));
+    if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, B, st));
     return MLEM_OK;
 }
 
@@ -2747,12 +2760,12 @@ int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = fw_stride(c, B);
-    if (!room_for_padding(c, Bd, st))
+    if (!frame_room(c, B, Bd, st))
         return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
-    CK(c, interleave_f32(x, c->pscratch[0], c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
-    TRY(project_rows(c, c->pscratch[0], c->rscratch, Bd, st));
-    CK(c, deinterleave_f32(c->rscratch, y, c->R, B, Bd, nullptr, st));
-    return MLEM_OK;
+    CK(c, interleave_f32(x, frame_voxels(c), c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
+    TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
+    CK(c, deinterleave_f32(frame_rows(c, Bd), y, c->R, B, Bd, nullptr, st));
+    return frame_room_done(c, st);
 }
 
 int mlem_bkproj_frames_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
@@ -2760,12 +2773,12 @@ int mlem_bkproj_frames_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = bk_stride(c, B);
-    if (!room_for_padding(c, Bd, st))
+    if (!frame_room(c, B, Bd, st))
         return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
-    CK(c, interleave_f32(y, c->rscratch, c->R, B, Bd, nullptr, st));
-    TRY(project_columns(c, c->rscratch, c->pscratch[0], Bd, st));
-    CK(c, deinterleave_f32(c->pscratch[0], x, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
-    return MLEM_OK;
+    CK(c, interleave_f32(y, frame_rows(c, Bd), c->R, B, Bd, nullptr, st));
+    TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
+    CK(c, deinterleave_f32(frame_voxels(c), x, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
+    return frame_room_done(c, st);
 }
 
 int mlem_fwproj_correl_d(mlem_ctx* c, const float* x, const int32_t* sino, float* correl,

@@ -58,8 +58,11 @@ struct mlem_ctx {
     std::vector<uint32_t> perm_host, iperm_host;
     float* pscratch[2] = {nullptr, nullptr};
     size_t pscratch_floats = 0;
-    float* rscratch = nullptr;  // row vectors with padded frames (projections)
-    size_t rscratch_floats = 0;
+    // Voxel and row vectors of the projections' interleaved, padded frames
+    // (frame_room); ev_frames: the last call that used them.
+    float* fscratch = nullptr;
+    size_t fscratch_floats = 0;
+    cudaEvent_t ev_frames = nullptr;
 
     // Visiting order of the row kernels (row_order_build): rays with nearby
     // entry and exit voxels next to each other.  Null with MLEM_FLAG_NO_ROW_ORDER.

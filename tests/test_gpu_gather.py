@@ -186,3 +186,35 @@ def test_frame_major_projections(flags):
                     assert torch.allclose(a, b.t(), rtol=1e-4, atol=1e-5)
                 else:
                     assert torch.equal(a, b.t())
+
+
+def test_frame_scratch_on_two_streams_and_under_capture():
+    """Projections of several frames on two streams take turns with the context's
+    scratch, and a captured one does not use it: replayed after a call that replaces
+    the scratch it still gives its own result."""
+    torch = pytest.importorskip("torch")
+    from mlem_b200 import torch_ext
+    rng = np.random.default_rng(6)
+    m = matrix("many-rows", rng)
+    m = formats.Csr4(m.n_rows, m.n_cols, m.row_end, m.elems)  # no grid: no voxel scratch either
+    with api.Context.from_matrix(m) as ctx:
+        v = [torch.from_numpy(rng.uniform(0.1, 1.0, (3, m.n_cols)).astype(np.float32)).cuda() for _ in range(2)]
+        ref = [torch_ext.forward_project(t, ctx) for t in v]
+        side = [torch.cuda.Stream() for _ in v]
+        torch.cuda.synchronize()
+        got = [[], []]
+        for _ in range(20):
+            for i, s in enumerate(side):
+                with torch.cuda.stream(s):
+                    got[i].append(torch_ext.forward_project(v[i], ctx))
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, ref[i]) for i in (0, 1) for g in got[i])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = torch_ext.forward_project(v[0], ctx)
+        torch_ext.forward_project(torch.rand((16, m.n_cols), device="cuda"), ctx)  # a larger scratch
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        # rows of at most 4 products below 1.7: n 2^-23 sum |v x|
+        assert torch.allclose(out, ref[0], rtol=0, atol=4 * 6.8 * 2.0 ** -23)
