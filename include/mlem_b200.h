@@ -119,9 +119,10 @@ typedef struct {
  * the copy, as does selecting the method; mlem_step_host and
  * mlem_stream_host, one iteration per sinogram, walk the whole CSC in
  * visiting order instead (the copy takes about as long as the back
- * projection saves in six iterations).  Either way the sums are a fixed
- * function of the matrix, the sinograms and the entry point, the same from
- * run to run. */
+ * projection saves in six iterations), or run the one-pass method where
+ * mlem_autotune chose the CSC method over it.  The CSC method's sums
+ * are a fixed function of the matrix, the sinograms and the entry point, the
+ * same from run to run. */
 typedef struct {
     int bk_mode;        /* MLEM_BK_CSC, MLEM_BK_ATOMIC, MLEM_BK_FUSED or MLEM_BK_REGION */
     int group;          /* lanes per row/column: 4, 8, 16 or 32 */
@@ -295,8 +296,11 @@ int mlem_measure_l2_rates(int device, double* rates);
 int mlem_get_tuning(const mlem_ctx* ctx, mlem_tuning* out);
 int mlem_set_tuning(mlem_ctx* ctx, const mlem_tuning* t);
 /* Time every valid configuration for the current B on the device and keep
- * the fastest (deterministic_only != 0 restricts to MLEM_BK_CSC).  The
- * image state is restored afterwards. */
+ * the fastest (deterministic_only != 0 restricts to MLEM_BK_CSC).  Where
+ * that is MLEM_BK_CSC with MLEM_VISIT_SORTED among all methods, the fastest
+ * one-pass configuration is kept beside it for mlem_step_host,
+ * mlem_stream_host and ordered subsets.  The image state is restored
+ * afterwards. */
 int mlem_autotune(mlem_ctx* ctx, int deterministic_only, mlem_tuning* best);
 
 /* ---- ordered subsets (OSEM) ---------------------------------------------
