@@ -205,13 +205,65 @@ class _UnrolledMLEM(torch.autograd.Function):
         return gx + out, partial.sum(1).to(omega.dtype), None, None, None, None
 
 
+class _UnrolledTensors(torch.autograd.Function):
+    """The same iterations with the voxel-wise steps as tensor expressions, for
+    factors and relaxations of other shapes than one float a voxel and one an
+    iteration (omega[k] and norm broadcast against the image)."""
+
+    @staticmethod
+    def _ratio(ctx, x, sino_i, norm):
+        x = x.to(torch.float32)  # the kernels' type, whatever the expressions' types promote to
+        u, f = torch.empty_like(x), torch.empty(ctx.n_rows, dtype=torch.float32, device=x.device)
+        _ratio_numerator(ctx, x, sino_i, u, f)
+        return torch.where(norm != 0, u / torch.where(norm != 0, norm, torch.ones_like(norm)), u), f
+
+    @staticmethod
+    def forward(fctx, x0, omega, norm, ctx, sino_i, keep):
+        xs, rs, fs = [x0.detach()], [], []
+        x = x0.detach().contiguous()
+        for w in omega:
+            r, f = _UnrolledTensors._ratio(ctx, x, sino_i, norm)
+            if keep:
+                rs.append(r)
+                fs.append(f)
+            x = x * torch.where(r > 0, r.clamp_min(1e-38) ** w, torch.zeros_like(r))
+            xs.append(x)
+        fctx.mctx, fctx.sino_i, fctx.keep = ctx, sino_i, keep
+        fctx.save_for_backward(torch.stack(xs[:-1]), omega, norm,
+                               *([torch.stack(rs), torch.stack(fs)] if keep else []))
+        return x
+
+    @staticmethod
+    def backward(fctx, g):
+        ctx = fctx.mctx
+        xs, omega, norm, *kept = fctx.saved_tensors
+        g = g.contiguous()
+        d_omega = torch.zeros_like(omega)
+        for k in range(omega.shape[0] - 1, -1, -1):
+            xk, w = xs[k].contiguous(), omega[k]
+            r, f = (kept[0][k], kept[1][k]) if kept else _UnrolledTensors._ratio(ctx, xk, fctx.sino_i, norm)
+            pos = r > 0
+            rs = torch.where(pos, r, torch.ones_like(r))
+            p = torch.where(pos, rs ** w, torch.zeros_like(r))
+            term = g * (xk * p) * torch.where(pos, torch.log(rs), torch.zeros_like(r))
+            d_omega[k] = term.sum_to_size(w.shape)
+            dr = torch.where(pos, g * xk * w * rs ** (w - 1), torch.zeros_like(r))
+            du = torch.where(norm != 0, dr / torch.where(norm != 0, norm, torch.ones_like(norm)), dr)
+            du = du.to(torch.float32).contiguous()
+            out = torch.empty_like(du)
+            _adjoint(ctx, du, fctx.sino_i, f, out)
+            g = g * p + out
+        return g, d_omega, None, None, None, None
+
+
 def unrolled_mlem(x0: torch.Tensor, omega: torch.Tensor, sino: torch.Tensor,
                   ctx: "api.Context", norm: torch.Tensor | None = None,
                   keep_bytes: int = 2 << 30) -> torch.Tensor:
     """K = len(omega) relaxed MLEM iterations from x0 (float32 [C] CUDA).
-    The forward pass keeps each iteration's row sums and update factor for
-    the backward pass when they take at most keep_bytes (0: always
-    recompute them)."""
+    omega is [K], or [K, ...] whose omega[k] broadcasts against the image: [K, C]
+    holds a relaxation per voxel.  The forward pass keeps each iteration's row
+    sums and update factor for the backward pass when they take at most
+    keep_bytes (0: always recompute them)."""
     _check(x0, ctx.n_cols, "x0")
     if norm is None:
         norm = norm_tensor(ctx, x0.device)
@@ -219,8 +271,14 @@ def unrolled_mlem(x0: torch.Tensor, omega: torch.Tensor, sino: torch.Tensor,
     K = int(omega.shape[0])
     if K == 0:
         raise RuntimeError("unrolled_mlem: omega holds no iteration")
-    # one float per voxel, as the voxel-wise kernels read it
-    norm = norm.to(device=x0.device, dtype=torch.float32).expand(x0.shape).contiguous()
     keep = K * (ctx.n_rows + ctx.n_cols) * 4 <= keep_bytes
-    return _UnrolledMLEM.apply(x0, omega.to(device=x0.device, dtype=torch.float32).contiguous(), norm,
-                               ctx, sino_i, keep)
+    omega = omega.to(device=x0.device, dtype=torch.float32)
+    # The voxel-wise kernels read one relaxation an iteration and one float of x0 and
+    # norm a voxel (a norm that does not broadcast to x0, or of another type or
+    # device, is the tensor expressions' to take or to refuse).
+    if (omega.dim() == 1 and x0.numel() == ctx.n_cols and norm.dtype == torch.float32
+            and (norm.dim() == 0 or norm.device == x0.device) and norm.dim() <= x0.dim()
+            and all(a in (1, b) for a, b in zip(reversed(norm.shape), reversed(x0.shape)))):
+        return _UnrolledMLEM.apply(x0, omega.contiguous(), norm.to(x0.device).expand(x0.shape).contiguous(),
+                                   ctx, sino_i, keep)
+    return _UnrolledTensors.apply(x0, omega, norm, ctx, sino_i, keep)

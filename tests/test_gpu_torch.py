@@ -241,3 +241,48 @@ def test_relax_steps_match_tensor_expressions(n):
                 slack = 2.0 ** -20 + 2.0 ** -23 * torch.log(rs).abs()
                 assert torch.all((d(du) - wdu).abs() <= slack * wdu.abs() + 1e-45)
                 assert abs(float(part.sum() - terms.sum())) <= 2.0 ** -19 * float(terms.abs().sum()) + 1e-45
+
+
+@pytest.mark.parametrize("keep_bytes", [2 << 30, 0])
+@pytest.mark.parametrize("shape", ["K", "K1", "KC", "K1C", "norm-scalar", "norm-1C", "norm-double"])
+def test_unrolled_mlem_broadcasts_omega_and_norm(shape, keep_bytes):
+    """A relaxation per iteration or per voxel, and norms of other shapes and
+    types: image and gradients against float64 autograd over the dense matrix.
+    An iteration adds at most (40 + 60 + 10) 2^-23 relative to a positive image, and
+    an image error enters the next one about threefold: 1e-4 after three; the
+    gradients' terms have both signs, 1e-3 as for the finite differences above."""
+    from mlem_b200 import formats
+    rng = np.random.default_rng(23)
+    R, C, K = 301, 157, 1 if shape in ("K1C", "norm-1C", "norm-double") else 3
+    lens = rng.integers(0, 40, R)
+    el = np.zeros(int(lens.sum()), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, C, el.size)
+    el["value"] = rng.uniform(0.1, 1.7, el.size)
+    m = formats.Csr4(R, C, np.cumsum(lens).astype(np.uint64), el)
+    A = torch.zeros((R, C), dtype=torch.float64, device="cuda")
+    A.index_put_((torch.from_numpy(np.repeat(np.arange(R), lens)).cuda(),
+                  torch.from_numpy(el["index"].astype(np.int64)).cuda()),
+                 torch.from_numpy(el["value"].astype(np.float64)).cuda(), accumulate=True)
+    s = torch.from_numpy(rng.poisson(20, R).astype(np.int32)).cuda()
+    om = {"KC": (K, C), "K1": (K, 1), "K1C": (K, 1, C)}.get(shape, (K,))
+    omega = torch.from_numpy(rng.uniform(0.6, 1.2, om).astype(np.float32)).cuda().requires_grad_()
+    x0 = torch.from_numpy(rng.uniform(0.5, 2.0, C).astype(np.float32)).cuda().requires_grad_()
+    norm = {"norm-scalar": torch.tensor(17.0), "norm-1C": A.sum(0).float()[None],
+            "norm-double": A.sum(0)}.get(shape, A.sum(0).float())
+    with api.Context.from_matrix(m) as ctx:
+        out = torch_ext.unrolled_mlem(x0, omega, s, ctx, norm=norm, keep_bytes=keep_bytes)
+        v = torch.from_numpy(rng.uniform(-1.0, 2.0, tuple(out.shape)).astype(np.float32)).cuda()
+        gx, gw = torch.autograd.grad((out * v.to(out.dtype)).sum(), (x0, omega))
+    x64, w64, n64 = (t.detach().double().cuda() for t in (x0, omega, norm))
+    x64.requires_grad_()
+    w64.requires_grad_()
+    x = x64
+    for k in range(K):
+        f = (A @ x.reshape(-1))
+        c = torch.where(f != 0, s.double() / torch.where(f != 0, f, 1.0), 0.0)
+        r = (A.t() @ c) / torch.where(n64 != 0, n64, 1.0)
+        x = x * torch.where(r > 0, torch.where(r > 0, r, 1.0) ** w64[k], 0.0)
+    hx, hw = torch.autograd.grad((x * v.double()).sum(), (x64, w64))
+    assert out.shape == x.shape and gx.shape == x0.shape and gw.shape == omega.shape
+    for got, want, tol in ((out, x, 1e-4), (gx, hx, 1e-3), (gw, hw, 1e-3)):
+        assert float((got.detach().double() - want.detach()).norm()) <= tol * float(want.detach().norm())
