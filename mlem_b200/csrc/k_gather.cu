@@ -176,9 +176,18 @@ struct FwOp {
             } else {  // eight counts held over the row cost more than this wait
                 g_counts<VW>(sino + (size_t)p.r * B + off, s);
             }
+            // A row without counts in the tile's frames has calcCorrel 0 whatever its
+            // projection, NaN included, walked or not.
+            int any = 0;
+#pragma unroll
+            for (int i = 0; i < VW; ++i) any |= s[i];
+            if constexpr (BT > VW) {  // two writers hold the tile's counts
+                static_assert(BT == 2 * VW, "one exchange between the writing lanes");
+                any |= __shfl_xor_sync((gmask & (0u - gmask)) * 3u, any, 1);
+            }
             float t[VW];
 #pragma unroll
-            for (int i = 0; i < VW; ++i) t[i] = correl_of(s[i], acc[i]);
+            for (int i = 0; i < VW; ++i) t[i] = any ? correl_of(s[i], acc[i]) : 0.0f;
             g_store<VW>(c + o, t);
         }
     }

@@ -71,6 +71,53 @@ def test_gather_passes_against_float64(kind):
                         assert np.all(np.abs(got - ref) <= 2.0 ** -23 * (cnt + 1) * mag), (way, B, group, shift)
 
 
+def empty_tiles(s, tile):
+    """Where all counts of the row's frame tile are 0, [R, B]."""
+    R, B = s.shape
+    return np.repeat(~s.reshape(R, B // tile, tile).any(axis=2), tile, axis=1)
+
+
+def test_rows_without_counts_drop_what_is_not_finite():
+    """calcCorrel of a row without counts in its frame tile is 0 also where its
+    projection is NaN, for every tile and visit, with and without the list of rows with
+    counts: such rows carry no NaN into the image."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(8)
+    R, C = 3000, 2000
+    lens = rng.integers(1, 5, R)
+    el = np.zeros(int(lens.sum()), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, C, el.size)
+    el["value"] = rng.uniform(0.1, 1.7, el.size)
+    m = formats.Csr4(R, C, np.cumsum(lens).astype(np.uint64), el)
+    A = np.zeros((R, C), bool)
+    A[np.repeat(np.arange(R), lens), el["index"]] = True
+    bad = rng.random(C) < 0.05
+    hit = A[:, bad].any(axis=1)
+    st = torch.cuda.current_stream().cuda_stream
+    for flags in (0, api.FLAG_NO_ROW_ORDER):
+        with api.Context.from_matrix(m, flags=flags) as ctx:
+            for B in (1, 2, 4, 8, 16, 32):
+                s = rng.poisson(2, (R, B)).astype(np.int32)
+                s[rng.random(R) < 0.5] = 0
+                s[::3, : B // 2] = 0
+                x = np.where(bad[:, None], np.nan, rng.uniform(0.5, 2.0, (C, B))).astype(np.float32)
+                xd, sd = torch.from_numpy(x).cuda(), torch.from_numpy(s).cuda()
+                c = torch.empty((R, B), device="cuda")
+                ctx.fwproj_correl_d(xd.data_ptr(), sd.data_ptr(), c.data_ptr(), B, st)
+                want = hit[:, None] & ~empty_tiles(s, min(B, 16))
+                assert np.array_equal(np.isnan(c.cpu().numpy()), want), B
+                assert not c.cpu().numpy()[empty_tiles(s, min(B, 16))].any()
+                for tile in (t for t in (1, 2, 4, 8, 16) if t <= B):
+                    for visit in (api.VISIT_FILE,) + (() if flags else (api.VISIT_SORTED,)):
+                        ctx.set_sinograms(np.ascontiguousarray(s.T))
+                        ctx.set_tuning(api.BK_CSC, 32, tile, 8, visit)
+                        ctx.set_images(np.ascontiguousarray(x.T))
+                        ctx.iterate(1)
+                        nan_rows = hit[:, None] & ~empty_tiles(s, tile)
+                        ref = bad[:, None] | (A.T.astype(np.float32) @ nan_rows.astype(np.float32) > 0)
+                        assert np.array_equal(np.isnan(ctx.get_images().T), ref), (B, tile, visit, flags)
+
+
 def test_default_frame_tile_follows_the_frames():
     """Without a chosen tuning the frame tile is the widest one of the frame
     count; a chosen one stays."""
