@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kRelaxThreads) k_relax_grad(const float* g, co
         const bool pos = ri > 0.0f;
         const float rs = pos ? ri : 1.0f;
         const float p = pos ? powf(rs, w) : 0.0f;
-        if (pos) s += (double)(gi * (xi * p) * logf(rs));
+        s += (double)(gi * (xi * p) * (pos ? logf(rs) : 0.0f));  // not finite where g or x is not
         gx[i] = gi * p;
         du[i] = over_norm(pos ? gi * xi * w * powf(rs, w - 1.0f) : 0.0f, norm[i]);
     }

@@ -243,6 +243,25 @@ def test_relax_steps_match_tensor_expressions(n):
                 assert abs(float(part.sum() - terms.sum())) <= 2.0 ** -19 * float(terms.abs().sum()) + 1e-45
 
 
+@pytest.mark.parametrize("where", ["g", "x"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_relax_grad_keeps_what_is_not_finite(where, value):
+    """An infinite or NaN gradient or image at a voxel whose ratio is 0 shows in
+    omega's gradient, as 0 times it does in the tensor expressions."""
+    n = 300
+    t = {k: torch.full((n,), 1.5, device="cuda") for k in ("g", "x", "r", "norm", "gx", "du")}
+    om = torch.tensor([0.7], device="cuda")
+    part = torch.empty(api.RELAX_PARTIALS, dtype=torch.float64, device="cuda")
+    t["r"][137] = 0.0
+    t[where][137] = value
+    with api.Context(np.array([1], np.uint64), np.zeros(1, api.ELEM_DTYPE), 1, n) as ctx:
+        ctx.relax_grad_d(t["g"].data_ptr(), None, t["x"].data_ptr(), t["r"].data_ptr(), t["norm"].data_ptr(),
+                         om.data_ptr(), t["gx"].data_ptr(), t["du"].data_ptr(), part.data_ptr(),
+                         torch.cuda.current_stream().cuda_stream)
+        assert part.sum().isnan()
+        assert t["gx"].isnan().sum() == (where == "g") and t["du"][137] == 0.0
+
+
 @pytest.mark.parametrize("keep_bytes", [2 << 30, 0])
 @pytest.mark.parametrize("shape", ["K", "K1", "KC", "K1C", "norm-scalar", "norm-1C", "norm-double"])
 def test_unrolled_mlem_broadcasts_omega_and_norm(shape, keep_bytes):
