@@ -178,7 +178,8 @@ class _UnrolledMLEM(torch.autograd.Function):
     @staticmethod
     def backward(fctx, g):
         ctx = fctx.mctx
-        saved = fctx.saved_tensors
+        # what saved-tensor hooks hand back, as the kernels read it
+        saved = [t.to(device=g.device, dtype=torch.float32).contiguous() for t in fctx.saved_tensors]
         xs, omega, norm = saved[:3]
         K = omega.shape[0]
         g = g.contiguous()
@@ -236,7 +237,7 @@ class _UnrolledTensors(torch.autograd.Function):
     @staticmethod
     def backward(fctx, g):
         ctx = fctx.mctx
-        xs, omega, norm, *kept = fctx.saved_tensors
+        xs, omega, norm, *kept = (t.to(g.device).contiguous() for t in fctx.saved_tensors)
         g = g.contiguous()
         d_omega = torch.zeros_like(omega)
         for k in range(omega.shape[0] - 1, -1, -1):
@@ -251,7 +252,7 @@ class _UnrolledTensors(torch.autograd.Function):
             du = torch.where(norm != 0, dr / torch.where(norm != 0, norm, torch.ones_like(norm)), dr)
             du = du.to(torch.float32).contiguous()
             out = torch.empty_like(du)
-            _adjoint(ctx, du, fctx.sino_i, f, out)
+            _adjoint(ctx, du, fctx.sino_i, f.to(torch.float32), out)
             g = g * p + out
         return g, d_omega, None, None, None, None
 

@@ -305,3 +305,25 @@ def test_unrolled_mlem_broadcasts_omega_and_norm(shape, keep_bytes):
     assert out.shape == x.shape and gx.shape == x0.shape and gw.shape == omega.shape
     for got, want, tol in ((out, x, 1e-4), (gx, hx, 1e-3), (gw, hw, 1e-3)):
         assert float((got.detach().double() - want.detach()).norm()) <= tol * float(want.detach().norm())
+
+
+@pytest.mark.parametrize("per_voxel", [False, True])
+@pytest.mark.parametrize("keep_bytes", [2 << 30, 0])
+def test_unrolled_mlem_under_saved_tensor_hooks(small, keep_bytes, per_voxel):
+    """Hooks that hand the saved tensors back on the host, in double or strided give
+    the gradients of the plain call, up to the order of float atomics."""
+    m, sino, ctx = small
+    s = torch.tensor(sino, device="cuda")
+    hooks = [(lambda t: t, lambda t: t), (lambda t: t.cpu(), lambda t: t),
+             (lambda t: t.double(), lambda t: t), (lambda t: t, lambda t: torch.stack([t, t], -1)[..., 0])]
+    grads = []
+    for pack, unpack in hooks:
+        x0 = torch.full((m.n_cols,), 0.5, device="cuda", requires_grad=True)
+        om = torch.tensor([1.0, 0.8], device="cuda")
+        om = (om[:, None].repeat(1, m.n_cols) if per_voxel else om).requires_grad_()
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            x = torch_ext.unrolled_mlem(x0, om, s, ctx, keep_bytes=keep_bytes)
+        grads.append(torch.autograd.grad((x * x).sum(), (x0, om)))
+    for got in grads[1:]:
+        for a, b in zip(got, grads[0]):
+            assert float((a - b).norm()) <= 1e-5 * float(b.norm())
