@@ -322,7 +322,11 @@ int mlem_get_subsets(const mlem_ctx* ctx, uint32_t* n_subsets);
 /* Column sums of subset s (natural voxel order, C floats); n_subsets >= 2. */
 int mlem_subset_column_sums(mlem_ctx* ctx, uint32_t s, float* out);
 
-/* ---- device-pointer entry points (torch extension, custom drivers) ------ */
+/* ---- device-pointer entry points (torch extension, custom drivers) ------
+ * They enqueue on `stream` and return.  Calls of one context on several streams
+ * take turns with its scratch; a call on a stream that is being captured takes
+ * its scratch as memory nodes of the graph instead, so that replays share
+ * nothing with other calls or graphs. */
 /* y[R][B] = A x[C][B]. */
 int mlem_fwproj_d(mlem_ctx* ctx, const float* x, float* y, uint32_t n_frames, void* stream);
 /* x[C][B] = A^T y[R][B]. */
@@ -338,8 +342,8 @@ int mlem_fwproj_correl_d(mlem_ctx* ctx, const float* x, const int32_t* sino, flo
  * frames, a power of two up to 16 so that none is padded); the sorted visits
  * then leave out the rows whose counts are zero in every frame, as an
  * iteration does.  Summation order varies from run to run (float atomics).
- * Not in the bit-exact mode; must not run concurrently with the context's
- * own iterations. */
+ * Not in the bit-exact mode; with sino NULL it must not run concurrently with
+ * the calls that set the context's sinograms or iterate on them. */
 int mlem_fused_update_d(mlem_ctx* ctx, const float* x, const int32_t* sino, float* update,
                         uint32_t n_frames, void* stream);
 /* x[C][B] *= calcUpdate factor(A^T correl[R][B], norm)  (fused, CSC). */
@@ -369,8 +373,7 @@ int mlem_bkproj_frames_d(mlem_ctx* ctx, const float* y, float* x, uint32_t n_fra
  *                         adjoint of calcCorrel and both projections.
  * Each is one pass over the matrix; rows without counts are skipped before
  * their elements are read.  Summation order varies from run to run.  Not in
- * the bit-exact mode nor with MLEM_FLAG_MIRROR_KERNELS; must not run
- * concurrently with the context's own iterations or mlem_fused_update_d. */
+ * the bit-exact mode nor with MLEM_FLAG_MIRROR_KERNELS. */
 int mlem_ratio_rows_d(mlem_ctx* ctx, const float* x, const int32_t* sino, float* rows,
                       float* update, void* stream);
 int mlem_adjoint_update_d(mlem_ctx* ctx, const float* du, const int32_t* sino, const float* rows,

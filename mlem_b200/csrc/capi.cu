@@ -186,48 +186,81 @@ void brick_order(uint32_t nx, uint32_t ny, uint32_t nz, std::vector<uint32_t>& p
     for (uint64_t k = 0; k < C; ++k) perm[order[k]] = (uint32_t)k;
 }
 
-// Scratch for converting caller vectors between natural and device order.
-int perm_scratch(mlem_ctx* c, size_t floats) {
-    if (c->pscratch_floats >= floats) return MLEM_OK;
-    for (auto& p : c->pscratch) {
-        if (p) { cudaFree(p); c->device_bytes -= c->pscratch_floats * 4; }
-        p = nullptr;
+// Scratch of one device-pointer call: two voxel vectors in device order (contexts
+// that keep one of their own), a row vector and a work counter, as far as asked for.
+// A call on a stream that is being captured gets memory nodes of its graph, so that
+// a replay shares it with no other call, replay or later growth; the others share
+// the context's blocks in turns, each waiting for the last one's scratch_end.
+struct CallScratch {
+    float* voxels[2] = {nullptr, nullptr};
+    float* rows = nullptr;
+    unsigned int* counter = nullptr;  // 0 before the call; the call leaves it 0
+    void* nodes = nullptr;
+};
+
+int grow(mlem_ctx* c, float** p, size_t* have, size_t want) {
+    if (*have >= want) return MLEM_OK;
+    if (*p) {
+        cudaFree(*p);  // waits for the calls that use it
+        c->device_bytes -= *have * 4;
     }
-    c->pscratch_floats = 0;
-    for (auto& p : c->pscratch) TRY(dev_alloc(c, &p, floats));
-    c->pscratch_floats = floats;
+    *p = nullptr;
+    *have = 0;
+    TRY(dev_alloc(c, p, want));
+    *have = want;
     return MLEM_OK;
 }
 
-// Voxel and row vectors of Bd frames for one projection of B caller frames on `st`
+int scratch_begin(mlem_ctx* c, cudaStream_t st, size_t voxels, size_t rows, bool counter,
+                  CallScratch* s) {
+    if (!voxels && !rows && !counter) return MLEM_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(c, cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        auto whole = [](size_t n) { return (n + 63) & ~size_t(63); };
+        const size_t v = whole(voxels), r = whole(rows);
+        float* p = nullptr;
+        CK(c, cudaMallocAsync(reinterpret_cast<void**>(&p), (2 * v + r + 64) * 4, st));
+        s->nodes = p;
+        s->voxels[0] = p;
+        s->voxels[1] = p + v;
+        s->rows = p + 2 * v;
+        s->counter = reinterpret_cast<unsigned int*>(p + 2 * v + r);
+        if (counter) CK(c, cudaMemsetAsync(s->counter, 0, 256, st));
+        return MLEM_OK;
+    }
+    for (int i = 0; i < 2; ++i) TRY(grow(c, &c->pscratch[i], &c->pscratch_floats[i], voxels));
+    TRY(grow(c, &c->rscratch, &c->rscratch_floats, rows));
+    if (!c->ev_scratch) CK(c, cudaEventCreateWithFlags(&c->ev_scratch, cudaEventDisableTiming));
+    CK(c, cudaStreamWaitEvent(st, c->ev_scratch, 0));
+    for (int i = 0; i < 2; ++i) s->voxels[i] = c->pscratch[i];
+    s->rows = c->rscratch;
+    s->counter = c->counter + 8;  // a cache sector from the iteration's own
+    return MLEM_OK;
+}
+
+int scratch_end(mlem_ctx* c, cudaStream_t st, const CallScratch& s) {
+    if (s.nodes) CK(c, cudaFreeAsync(s.nodes, st));
+    else if (s.voxels[0] || s.rows || s.counter) CK(c, cudaEventRecord(c->ev_scratch, st));
+    return MLEM_OK;
+}
+size_t voxel_scratch(const mlem_ctx* c, uint32_t B) { return c->bricked ? (size_t)c->C * B : 0; }
+
+// Voxel and row vectors of Bd interleaved frames for one projection on `st`
 // (frame_voxels, frame_rows); false where they do not fit beside the matrix or where the
 // stream is being captured (a graph may be replayed beside, or after, a call that
 // uses or replaces them), and the caller's frame count is walked as it is.  Calls
 // on several streams take turns: each waits for the last one's frame_room_done.
-bool frame_room(mlem_ctx* c, uint32_t B, uint32_t Bd, cudaStream_t st) {
+bool frame_room(mlem_ctx* c, uint32_t Bd, cudaStream_t st) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return false;
     }
-    // what a later capture of the same call needs
-    if (c->bricked && perm_scratch(c, (size_t)c->C * B) != MLEM_OK) {
+    const size_t voxels = (((size_t)c->C * Bd + 63) & ~(size_t)63), floats = voxels + (size_t)c->R * Bd;
+    if (grow(c, &c->fscratch, &c->fscratch_floats, floats) != MLEM_OK) {
         c->err.clear();
         return false;
-    }
-    const size_t voxels = (((size_t)c->C * Bd + 63) & ~(size_t)63), floats = voxels + (size_t)c->R * Bd;
-    if (c->fscratch_floats < floats) {
-        if (c->fscratch) {
-            cudaFree(c->fscratch);
-            c->device_bytes -= c->fscratch_floats * 4;
-        }
-        c->fscratch = nullptr;
-        c->fscratch_floats = 0;
-        if (dev_alloc(c, &c->fscratch, floats) != MLEM_OK) {
-            c->err.clear();
-            return false;
-        }
-        c->fscratch_floats = floats;
     }
     if ((!c->ev_frames && cudaEventCreateWithFlags(&c->ev_frames, cudaEventDisableTiming) != cudaSuccess) ||
         cudaStreamWaitEvent(st, c->ev_frames, 0) != cudaSuccess) {
@@ -1752,12 +1785,12 @@ void mlem_destroy(mlem_ctx* c) {
                     (void*)c->hist_zeros, (void*)c->hist_subn, (void*)c->tmp_r[0],
                     (void*)c->tmp_r[1], (void*)c->tmp_c[0], (void*)c->tmp_c[1], (void*)c->tmp_c[2],
                     (void*)c->tmp_sino, (void*)c->tmp_d, (void*)c->norm_nat, (void*)c->perm,
-                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->fscratch, (void*)c->row_order,
-                    (void*)c->row_ranges, (void*)c->counter, (void*)c->long_segs, (void*)c->f_long_d,
+                    (void*)c->pscratch[0], (void*)c->pscratch[1], (void*)c->rscratch, (void*)c->fscratch, (void*)c->row_order,
+                    (void*)c->row_ranges, (void*)c->counter, (void*)c->long_segs,
                     (void*)c->sub_norm,
                     (void*)c->sub_file, (void*)c->sub_file_ranges, (void*)c->sub_sorted,
                     (void*)c->sub_sorted_ranges, (void*)c->mirror_lut, (void*)c->mirror_vox,
-                    (void*)c->f_mirror_d, (void*)c->act_order, (void*)c->act_ranges,
+                    (void*)c->act_order, (void*)c->act_ranges,
                     (void*)c->act_tmp, (void*)c->act_n, (void*)c->act_z,
                     (void*)c->celems_vis, (void*)c->row_pos, (void*)c->csc_act,
                     (void*)c->csc_act_len, (void*)c->pos_keep, (void*)c->act_order_alt,
@@ -1771,7 +1804,7 @@ void mlem_destroy(mlem_ctx* c) {
     if (c->slots) cudaFreeHost(c->slots);
     for (cudaStream_t q : {c->up_stream, c->down_stream, c->side})
         if (q) { cudaStreamSynchronize(q); cudaStreamDestroy(q); }
-    for (cudaEvent_t e : {c->ev_image, c->ev_census, c->ev_frames})
+    for (cudaEvent_t e : {c->ev_image, c->ev_census, c->ev_frames, c->ev_scratch})
         if (e) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) {
         dev_free(c->sstage[i]);
@@ -2719,19 +2752,17 @@ int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* strea
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = fw_stride(c, B);
-    if (Bd != B && frame_room(c, B, Bd, st)) {
+    if (Bd != B && frame_room(c, Bd, st)) {
         CK(c, permute_to_device(x, frame_voxels(c), c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
         TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
         CK(c, permute_to_natural(frame_rows(c, Bd), y, nullptr, c->R, B, Bd, st));
         return frame_room_done(c, st);
     }
-    const float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
-        xd = c->pscratch[0];
-    }
-    return project_rows(c, xd, y, B, st);
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), 0, false, &s));
+    if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, B, B, st));
+    TRY(project_rows(c, c->bricked ? s.voxels[0] : x, y, B, st));
+    return scratch_end(c, st, s);
 }
 
 int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
@@ -2739,20 +2770,18 @@ int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* strea
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = bk_stride(c, B);
-    if (Bd != B && frame_room(c, B, Bd, st)) {
+    if (Bd != B && frame_room(c, Bd, st)) {
         CK(c, permute_to_device(y, frame_rows(c, Bd), nullptr, c->R, B, Bd, st));
         TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
         CK(c, permute_to_natural(frame_voxels(c), x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
         return frame_room_done(c, st);
     }
-    float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        xd = c->pscratch[0];
-    }
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), 0, false, &s));
+    float* xd = c->bricked ? s.voxels[0] : x;
     TRY(project_columns(c, y, xd, B, st));
     if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, B, st));
-    return MLEM_OK;
+    return scratch_end(c, st, s);
 }
 
 int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* stream) {
@@ -2760,7 +2789,7 @@ int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = fw_stride(c, B);
-    if (!frame_room(c, B, Bd, st))
+    if (!frame_room(c, Bd, st))
         return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
     CK(c, interleave_f32(x, frame_voxels(c), c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
     TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
@@ -2773,7 +2802,7 @@ int mlem_bkproj_frames_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = bk_stride(c, B);
-    if (!frame_room(c, B, Bd, st))
+    if (!frame_room(c, Bd, st))
         return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
     CK(c, interleave_f32(y, frame_rows(c, Bd), c->R, B, Bd, nullptr, st));
     TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
@@ -2786,12 +2815,10 @@ int mlem_fwproj_correl_d(mlem_ctx* c, const float* x, const int32_t* sino, float
     if (!c || !x || !sino || !correl || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    const float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
-        xd = c->pscratch[0];
-    }
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), 0, false, &s));
+    if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, B, B, st));
+    const float* xd = c->bricked ? s.voxels[0] : x;
     const LaunchCfg cfg = cfg_for_frames(c, B);
     if (c->mirrored) {  // the full rows' sums, then calcCorrel in place
         CK(c, cudaMemsetAsync(correl, 0, (size_t)c->R * B * 4, st));
@@ -2799,11 +2826,11 @@ int mlem_fwproj_correl_d(mlem_ctx* c, const float* x, const int32_t* sino, float
             CK(c, mirror_fwproj(csr_visit(c, c->tuning), c->mirror, xd, B, f0, cfg.frame_tile,
                                 correl, c->n_sm, c->tuning.blocks_per_sm, st));
         CK(c, correl_inplace(correl, sino, (uint64_t)c->R * B, st));
-        return MLEM_OK;
+        return scratch_end(c, st, s);
     }
     for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
         CK(c, fwproj(csr_view(c), xd, B, f0, sino, correl, nullptr, cfg, st));
-    return MLEM_OK;
+    return scratch_end(c, st, s);
 }
 
 int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float* u, uint32_t B,
@@ -2823,34 +2850,26 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
     }
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    if (c->mirrored) {  // the full rows' sums in a buffer of the context, then the scatter
+    // row sums: the mirrored method's full rows', or the long rows'
+    const size_t row_sums = (c->mirrored ? (size_t)c->R : (size_t)c->n_long) * B;
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), row_sums, !c->mirrored, &s));
+    if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, B, B, st));
+    const float* xd = c->bricked ? s.voxels[0] : x;
+    float* ud = c->bricked ? s.voxels[1] : u;
+    if (c->mirrored) {  // the full rows' sums, then the scatter
         const LaunchCfg cfg = cfg_for_frames(c, B);
-        const float* xd = x;
-        float* ud = u;
-        if (c->bricked) {
-            TRY(perm_scratch(c, (size_t)c->C * B));
-            CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
-            xd = c->pscratch[0];
-            ud = c->pscratch[1];
-        }
-        if (c->f_mirror_d_floats < (size_t)c->R * B) {
-            dev_free(c->f_mirror_d);
-            c->f_mirror_d = nullptr;
-            c->f_mirror_d_floats = 0;
-            TRY(dev_alloc(c, &c->f_mirror_d, (size_t)c->R * B));
-            c->f_mirror_d_floats = (size_t)c->R * B;
-        }
         const SparseView v = csr_visit(c, c->tuning);
-        CK(c, cudaMemsetAsync(c->f_mirror_d, 0, (size_t)c->R * B * 4, st));
+        CK(c, cudaMemsetAsync(s.rows, 0, (size_t)c->R * B * 4, st));
         CK(c, cudaMemsetAsync(ud, 0, (size_t)c->C * B * 4, st));
         for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
-            CK(c, mirror_fwproj(v, c->mirror, xd, B, f0, cfg.frame_tile, c->f_mirror_d, c->n_sm,
+            CK(c, mirror_fwproj(v, c->mirror, xd, B, f0, cfg.frame_tile, s.rows, c->n_sm,
                                 c->tuning.blocks_per_sm, st));
         for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
-            CK(c, mirror_bkproj(v, c->mirror, c->f_mirror_d, sino, B, f0, cfg.frame_tile, ud,
+            CK(c, mirror_bkproj(v, c->mirror, s.rows, sino, B, f0, cfg.frame_tile, ud,
                                 c->n_sm, c->tuning.blocks_per_sm, st));
         if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, B, st));
-        return MLEM_OK;
+        return scratch_end(c, st, s);
     }
     // the context's one-pass tuning when it has one, else sorted rows in chunks
     mlem_tuning t = c->has_one_pass ? c->one_pass : c->tuning;
@@ -2862,21 +2881,6 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
     t.bk_mode = MLEM_BK_FUSED;
     t.frame_tile = cfg_for_frames(c, B).frame_tile;
     if (chunk_visit(t.visit)) t.group = 32;
-    const float* xd = x;
-    float* ud = u;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
-        xd = c->pscratch[0];
-        ud = c->pscratch[1];
-    }
-    if (c->n_long && c->f_long_d_floats < (size_t)c->n_long * B) {
-        dev_free(c->f_long_d);
-        c->f_long_d = nullptr;
-        c->f_long_d_floats = 0;
-        TRY(dev_alloc(c, &c->f_long_d, (size_t)c->n_long * B));
-        c->f_long_d_floats = (size_t)c->n_long * B;
-    }
     CK(c, cudaMemsetAsync(ud, 0, (size_t)c->C * B * 4, st));
     SparseView v = csr_visit(c, t);
     if (c->n_long) v.long_len = kLongRowElems;
@@ -2885,14 +2889,12 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
         v.vrange = c->act_ranges;
         v.n_dev = c->act_n;
     }
-    // a counter of its own (a cache sector from the iteration's), so that this
-    // call and the context's graph never share one
-    TRY(fused_pass(c, t, v, xd, sino, ud, B, c->counter + 8, st));
+    TRY(fused_pass(c, t, v, xd, sino, ud, B, s.counter, st));
     if (c->n_long)
         CK(c, long_rows_pass(csr_view(c), c->long_segs, c->n_long_segs, c->n_long, xd, B,
-                             t.frame_tile, sino, c->f_long_d, ud, c->n_sm, st));
+                             t.frame_tile, sino, s.rows, ud, c->n_sm, st));
     if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, B, st));
-    return MLEM_OK;
+    return scratch_end(c, st, s);
 }
 
 // The two one-pass kernels of the unrolled MLEM's backward pass (k_adjoint.cu):
@@ -2907,20 +2909,15 @@ static int backward_pass(mlem_ctx* c, int op, const float* x, const int32_t* sin
                     "the backward-pass kernels walk full rows (not MLEM_FLAG_MIRROR_KERNELS)");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    const float* xd = x;
-    float* ud = u;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, 1, 1, st));
-        xd = c->pscratch[0];
-        ud = c->pscratch[1];
-    }
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, 1), 0, true, &s));
+    if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, 1, 1, st));
+    const float* xd = c->bricked ? s.voxels[0] : x;
+    float* ud = c->bricked ? s.voxels[1] : u;
     CK(c, cudaMemsetAsync(ud, 0, (size_t)c->C * 4, st));
-    // the counter slot of mlem_fused_update_d: these calls, like it, must not
-    // run concurrently with the context's own iterations
-    CK(c, adjoint_pass(op, csr_view(c), xd, sino, rows, ud, c->counter + 8, c->n_sm, st));
+    CK(c, adjoint_pass(op, csr_view(c), xd, sino, rows, ud, s.counter, c->n_sm, st));
     if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, 1, 1, st));
-    return MLEM_OK;
+    return scratch_end(c, st, s);
 }
 
 int mlem_ratio_rows_d(mlem_ctx* c, const float* x, const int32_t* sino, float* rows, float* update,
@@ -2960,17 +2957,15 @@ int mlem_bkproj_update_d(mlem_ctx* c, const float* correl, float* x, uint32_t B,
         return fail(c, MLEM_ERR_STATE, "fused back projection needs the CSC copy of the full matrix");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    float* xd = x;
-    if (c->bricked) {
-        TRY(perm_scratch(c, (size_t)c->C * B));
-        CK(c, permute_to_device(x, c->pscratch[0], c->perm, c->C, B, B, st));
-        xd = c->pscratch[0];
-    }
+    CallScratch s;
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), 0, false, &s));
+    if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, B, B, st));
+    float* xd = c->bricked ? s.voxels[0] : x;
     const LaunchCfg cfg = cfg_for_frames(c, B);
     for (uint32_t f0 = 0; f0 < B; f0 += (uint32_t)cfg.frame_tile)
         CK(c, bkproj_csc(csc_view(c), correl, B, f0, c->norm, xd, nullptr, cfg, st));
     if (c->bricked) CK(c, permute_to_natural(xd, x, c->perm, c->C, B, B, st));
-    return MLEM_OK;
+    return scratch_end(c, st, s);
 }
 
 int mlem_apply_update_d(mlem_ctx* c, const float* update, float* x, uint32_t B, void* stream) {

@@ -56,8 +56,13 @@ struct mlem_ctx {
     uint32_t grid[3] = {0, 0, 0};
     uint32_t* perm = nullptr;
     std::vector<uint32_t> perm_host, iperm_host;
+    // Scratch of the device-pointer calls (scratch_begin): voxel vectors in device
+    // order, row sums; ev_scratch: the last call that used them or counter + 8.
     float* pscratch[2] = {nullptr, nullptr};
-    size_t pscratch_floats = 0;
+    size_t pscratch_floats[2] = {0, 0};
+    float* rscratch = nullptr;
+    size_t rscratch_floats = 0;
+    cudaEvent_t ev_scratch = nullptr;
     // Voxel and row vectors of the projections' interleaved, padded frames
     // (frame_room); ev_frames: the last call that used them.
     float* fscratch = nullptr;
@@ -92,8 +97,6 @@ struct mlem_ctx {
     mlem::LongSeg* long_segs = nullptr;
     uint32_t n_long_segs = 0, n_long = 0;
     float* f_long = nullptr;
-    float* f_long_d = nullptr;  // the same for mlem_fused_update_d (any frame count)
-    size_t f_long_d_floats = 0;
 
     // Ordered subsets (mlem_set_subsets): row r in subset r % n_subsets.
     // sub_norm[s * C ...]: subset column sums (device voxel order); the visiting
@@ -177,13 +180,11 @@ struct mlem_ctx {
 
     // Mirrors applied in the kernels (MLEM_FLAG_MIRROR_KERNELS): the matrix
     // arrays hold the stored elements only; norm holds the full matrix's
-    // column sums; f_mirror_d is the per-row sum buffer of mlem_fused_update_d.
+    // column sums.
     bool mirrored = false;
     mlem::MirrorView mirror;
     uint32_t* mirror_lut = nullptr;
     uint32_t* mirror_vox = nullptr;
-    float* f_mirror_d = nullptr;
-    size_t f_mirror_d_floats = 0;
 
     // region-blocked copy of the matrix (MLEM_BK_REGION), for one frame tile
     mlem::RegionBlocks rb;

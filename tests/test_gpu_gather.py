@@ -265,3 +265,89 @@ def test_frame_scratch_on_two_streams_and_under_capture():
         torch.cuda.synchronize()
         # rows of at most 4 products below 1.7: n 2^-23 sum |v x|
         assert torch.allclose(out, ref[0], rtol=0, atol=4 * 6.8 * 2.0 ** -23)
+
+
+@pytest.mark.parametrize("kind", ["many-rows", "long-rows", "mirrored"])
+def test_device_calls_on_two_streams_and_under_capture(kind):
+    """The device-pointer calls of a context with a grid (voxel scratch), with long rows
+    and with mirrored kernels (row scratch) on two streams, and two captured ones replayed
+    on two streams beside eager calls that make the scratch grow: each gives what it gives
+    alone, and none spoils the calls after it.  Float atomics: 1e-5 relative."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(13)
+    if kind == "mirrored":
+        from test_symmetry_oracle import sym_matrix
+        m = sym_matrix(7, seed=3, grid=(8, 8, 4))
+    else:
+        m = matrix("many-rows", rng)
+        if kind == "long-rows":
+            lens = np.diff(np.concatenate([[0], m.row_end.astype(np.int64)]))
+            lens[[5, 70]] = 40000
+            el = np.zeros(int(lens.sum()), formats.ELEM_DTYPE)
+            el["index"] = rng.integers(0, m.n_cols, el.size)
+            el["value"] = rng.uniform(0.1, 1.7, el.size)
+            m = formats.Csr4(m.n_rows, m.n_cols, np.cumsum(lens).astype(np.uint64), el, grid=(30, 40, 25))
+    with (api.Context.symmetric(m, flags=api.FLAG_MIRROR_KERNELS) if kind == "mirrored" else
+          api.Context.from_matrix(m)) as ctx:
+        R, C = ctx.n_rows, ctx.n_cols
+        gen = torch.Generator(device="cuda").manual_seed(1)
+
+        def rand(*shape):
+            return torch.rand(shape, generator=gen, device="cuda") + 0.1
+
+        def calls(B):
+            x, y, s = rand(C, B), rand(R, B), torch.randint(0, 4, (R, B), generator=gen, device="cuda", dtype=torch.int32)
+            f = [(R, lambda o, st: ctx.fwproj_d(x.data_ptr(), o.data_ptr(), B, st)),
+                 (C, lambda o, st: ctx.bkproj_d(y.data_ptr(), o.data_ptr(), B, st)),
+                 (R, lambda o, st: ctx.fwproj_correl_d(x.data_ptr(), s.data_ptr(), o.data_ptr(), B, st)),
+                 (C, lambda o, st: ctx.fused_update_d(x.data_ptr(), s.data_ptr(), o.data_ptr(), B, st))]
+            if B == 1 and kind != "mirrored":
+                f += [(C, lambda o, st: ctx.adjoint_update_d(x.data_ptr(), s.data_ptr(), y.data_ptr(), o.data_ptr(), st))]
+            return [(torch.empty((n, B), device="cuda"), g) for n, g in f]
+
+        def close(a, b):
+            return float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+        here = torch.cuda.current_stream().cuda_stream
+        sets = [calls(1), calls(1)]
+        refs = []
+        for one in sets:
+            refs.append([])
+            for o, g in one:
+                g(o, here)
+                refs[-1].append(o.clone())
+        side = [torch.cuda.Stream() for _ in sets]
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for (k, (a, ga)), (b, gb) in zip(enumerate(sets[0]), reversed(sets[1])):
+                for o, g, q in ((a, ga, side[0]), (b, gb, side[1])):
+                    with torch.cuda.stream(q):
+                        o.zero_()
+                        g(o, q.cuda_stream)
+        torch.cuda.synchronize()
+        assert all(close(o, r) for one, ref in zip(sets, refs) for (o, _), r in zip(one, ref))
+        graphs = []
+        for one, q in zip(sets, side):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1], stream=q):
+                for o, g in one:
+                    g(o, q.cuda_stream)
+        for o, g in calls(5) + calls(16):  # the eager calls' scratch grows
+            g(o, here)
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for one, graph, q in zip(sets, graphs, side):
+                with torch.cuda.stream(q):
+                    for o, _ in one:
+                        o.zero_()
+                    graph.replay()
+            for o, g in calls(2):
+                g(o, here)
+        torch.cuda.synchronize()
+        assert all(close(o, r) for one, ref in zip(sets, refs) for (o, _), r in zip(one, ref))
+        for one, ref in zip(sets, refs):
+            for (o, g), r in zip(one, ref):
+                o.zero_()
+                g(o, here)
+                assert close(o, r)
+        del graphs
