@@ -949,13 +949,15 @@ int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, cudaStr
 }
 
 // The tuning a run takes: the context's, or the autotuner's one-pass tuning
-// (mlem_ctx::one_pass) where it chose the CSC method in visiting order: for ordered
-// subsets, and while there is no cut copy of the current sinograms -- in steps of
-// one iteration per sinogram (plain-full: 2.24 ms a streamed step against 2.57 for
-// the CSC method over every entry) and in what follows them.
+// (mlem_ctx::one_pass): for ordered subsets, which no other method runs, and, where it
+// chose the CSC method in visiting order, while there is no cut copy of the current
+// sinograms -- in steps of one iteration per sinogram (plain-full: 2.24 ms a streamed
+// step against 2.57 for the CSC method over every entry) and in what follows them.
 const mlem_tuning& tuning_for(const mlem_ctx* c, bool steps) {
-    const bool instead = c->has_one_pass && csc_by_visit(c, c->tuning) &&
-                         (steps || c->n_subsets > 1 || (c->tuned_cut && !c->csc_act_ready));
+    const bool instead = c->has_one_pass && c->tuning.bk_mode != MLEM_BK_FUSED &&
+                         (c->n_subsets > 1 ||
+                          (csc_by_visit(c, c->tuning) &&
+                           (steps || (c->tuned_cut && !c->csc_act_ready))));
     return instead ? c->one_pass : c->tuning;
 }
 

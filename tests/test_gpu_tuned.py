@@ -68,3 +68,27 @@ def test_autotuned_context_streams_steps_and_subsets():
         ctx.set_subsets(3)
         with pytest.raises(api.MlemError):  # the caller's own choice is refused, as before
             ctx.iterate(1)
+
+
+@pytest.mark.parametrize("frames", [1, 16])
+@pytest.mark.parametrize("flags", [0, api.FLAG_NO_ROW_ORDER])
+def test_subsets_after_autotune_whatever_it_chose(flags, frames):
+    """Ordered subsets run on the one-pass tuning of an autotuned context also where the
+    CSC method in file order, the atomic or the region method won the comparison."""
+    g = synth.Geometry(64, 64, 32, 60000, 40, 200, seed=9)
+    m = synth.host_matrix(g)
+    rng = np.random.default_rng(4)
+    s = rng.poisson(4, (frames, g.n_rows)).astype(np.int32)
+    with api.Context.from_matrix(m, flags=flags) as ctx:
+        ctx.set_sinograms(s)
+        ctx.init_images()
+        chosen = ctx.autotune()
+        ctx.set_subsets(3)
+        ctx.init_images()
+        assert ctx.kernels_per_iteration() >= 6  # a pass and an update for every subset
+        ctx.iterate(2)
+        got = ctx.get_images()
+        for b in {0, frames - 1}:
+            assert ob.rel_l2(got[b], ob.osem(m, s[b], 2, 3)[0]) <= TOL
+        ctx.set_subsets(1)
+        assert ctx.tuning() == chosen
