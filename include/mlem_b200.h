@@ -119,10 +119,11 @@ typedef struct {
  * the copy, as does selecting the method; mlem_step_host and
  * mlem_stream_host, one iteration per sinogram, walk the whole CSC in
  * visiting order instead (the copy takes about as long as the back
- * projection saves in six iterations), or run the one-pass method where
- * mlem_autotune chose the CSC method over it.  The CSC method's sums
- * are a fixed function of the matrix, the sinograms and the entry point, the
- * same from run to run. */
+ * projection saves in six iterations), and so does mlem_iterate after them;
+ * but where mlem_autotune chose the CSC method over the one-pass method, the
+ * steps run the latter, whose sums (float atomics) vary from run to run.  The
+ * CSC method's sums are a fixed function of the matrix, the sinograms and the
+ * entry point, the same from run to run. */
 typedef struct {
     int bk_mode;        /* MLEM_BK_CSC, MLEM_BK_ATOMIC, MLEM_BK_FUSED or MLEM_BK_REGION */
     int group;          /* lanes per row/column: 4, 8, 16 or 32 */
@@ -296,11 +297,13 @@ int mlem_measure_l2_rates(int device, double* rates);
 int mlem_get_tuning(const mlem_ctx* ctx, mlem_tuning* out);
 int mlem_set_tuning(mlem_ctx* ctx, const mlem_tuning* t);
 /* Time every valid configuration for the current B on the device and keep
- * the fastest (deterministic_only != 0 restricts to MLEM_BK_CSC).  Where
- * that is MLEM_BK_CSC with MLEM_VISIT_SORTED among all methods, the fastest
- * one-pass configuration is kept beside it for mlem_step_host,
- * mlem_stream_host and ordered subsets.  The image state is restored
- * afterwards. */
+ * the fastest (deterministic_only != 0 restricts to MLEM_BK_CSC).  Among all
+ * methods, the fastest one-pass configuration is kept beside it: for ordered
+ * subsets, mlem_fused_update_d and, where the fastest is MLEM_BK_CSC with
+ * MLEM_VISIT_SORTED, mlem_step_host and mlem_stream_host, which then run it
+ * although mlem_get_tuning names the CSC method (mlem_set_tuning with that
+ * result, or deterministic_only, makes them run the CSC method).  The image
+ * state is restored afterwards. */
 int mlem_autotune(mlem_ctx* ctx, int deterministic_only, mlem_tuning* best);
 
 /* ---- ordered subsets (OSEM) ---------------------------------------------
@@ -336,7 +339,7 @@ int mlem_fwproj_correl_d(mlem_ctx* ctx, const float* x, const int32_t* sino, flo
                          uint32_t n_frames, void* stream);
 /* update[C][B] = A^T calcCorrel(sino[R][B], A x[C][B]) in one pass over the
  * matrix (the one-pass kernels, with the context's row visit when it is tuned
- * to MLEM_BK_FUSED, else sorted rows in chunks): the partial update of a row
+ * to MLEM_BK_FUSED, the one mlem_autotune kept, else sorted rows in chunks): the partial update of a row
  * shard (mlem_mpi/fusedmpimlem.cpp:205-225) or the numerator of calcUpdate.
  * sino NULL: the context's own sinograms (mlem_set_sinograms with n_frames
  * frames, a power of two up to 16 so that none is padded); the sorted visits

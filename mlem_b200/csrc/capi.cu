@@ -950,14 +950,13 @@ int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, cudaStr
 
 // The tuning a run takes: the context's, or the autotuner's one-pass tuning
 // (mlem_ctx::one_pass): for ordered subsets, which no other method runs, and, where it
-// chose the CSC method in visiting order, while there is no cut copy of the current
-// sinograms -- in steps of one iteration per sinogram (plain-full: 2.24 ms a streamed
-// step against 2.57 for the CSC method over every entry) and in what follows them.
+// chose the CSC method in visiting order, in steps of one iteration per sinogram, which
+// have no cut copy of the sinograms (plain-full: 2.24 ms a streamed step against 2.57 for
+// the CSC method over every entry).  mlem_iterate without subsets always runs the
+// method that mlem_get_tuning names.
 const mlem_tuning& tuning_for(const mlem_ctx* c, bool steps) {
     const bool instead = c->has_one_pass && c->tuning.bk_mode != MLEM_BK_FUSED &&
-                         (c->n_subsets > 1 ||
-                          (csc_by_visit(c, c->tuning) &&
-                           (steps || (c->tuned_cut && !c->csc_act_ready))));
+                         (c->n_subsets > 1 || (steps && csc_by_visit(c, c->tuning)));
     return instead ? c->one_pass : c->tuning;
 }
 
@@ -2580,7 +2579,6 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
         free_csc_vis(c);
     c->tuning = best;
     c->one_pass = one_pass;
-    c->tuned_cut = c->csc_act_ready;
     c->has_one_pass = one_pass.bk_mode == MLEM_BK_FUSED && one_pass.ms_per_iter < 1e30;
     c->tile_follows = false;
     c->graph_dirty = true;

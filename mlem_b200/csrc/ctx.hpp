@@ -191,12 +191,11 @@ struct mlem_ctx {
     size_t rb_bytes = 0;
 
     mlem_tuning tuning{};
-    // The best one-pass tuning the autotuner saw, where it chose the CSC method in
-    // visiting order: what runs where that method cannot (ordered subsets) or pays
-    // for a cut copy it cannot use (one iteration per sinogram).
+    // The best one-pass tuning the autotuner saw among all methods: what runs where the
+    // chosen one cannot (ordered subsets) or, as the CSC method in visiting order, would
+    // want a cut copy it does not have (one iteration per sinogram).  See tuning_for.
     mlem_tuning one_pass{};
     bool has_one_pass = false;
-    bool tuned_cut = false;  // the chosen method was timed over the cut copy
     bool tile_follows = true;  // no tuning chosen yet: the frame tile follows the frame count
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;

@@ -1,7 +1,7 @@
 """An autotuned context that chose the CSC method in visiting order: what that
 method cannot run, or has no cut copy for, runs on the best one-pass tuning the
-autotuner saw -- streamed and single host steps, the iterations after them, and
-ordered subsets -- and a tuning chosen by the caller is left alone."""
+autotuner saw -- streamed and single host steps, and ordered subsets -- and a tuning
+chosen by the caller is left alone."""
 import numpy as np
 import pytest
 
@@ -92,3 +92,25 @@ def test_subsets_after_autotune_whatever_it_chose(flags, frames):
             assert ob.rel_l2(got[b], ob.osem(m, s[b], 2, 3)[0]) <= TOL
         ctx.set_subsets(1)
         assert ctx.tuning() == chosen
+
+
+def test_iterations_after_streamed_steps_run_the_chosen_method():
+    """mlem_iterate after streamed steps runs the method that tuning() names: the CSC
+    method's sums are the same from run to run, the steps' float atomics are not."""
+    g = synth.Geometry(64, 64, 32, 60000, 40, 200, seed=9)
+    m = synth.host_matrix(g)
+    rng = np.random.default_rng(2)
+    sinos = [rng.poisson(4, (16, g.n_rows)).astype(np.int32) for _ in range(2)]
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_sinograms(sinos[0])
+        ctx.init_images()
+        start = ctx.get_images()
+        if ctx.autotune()["bk_mode"] != api.BK_CSC:
+            pytest.skip("the CSC method did not win the comparison here")
+        got = []
+        for _ in range(4):
+            ctx.stream_host(sinos)
+            ctx.set_images(start)
+            ctx.iterate(3)
+            got.append(ctx.get_images())
+        assert all(np.array_equal(a, got[0]) for a in got[1:])
