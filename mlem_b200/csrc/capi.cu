@@ -1287,14 +1287,17 @@ int ensure_history(mlem_ctx* c, int n) {
 
 namespace {
 
-// Drops the iteration graph and the streaming steps' second one (any new
-// capture of the first invalidates the second).
-void drop_graph(mlem_ctx* c) {
-    if (c->graph) cudaGraphExecDestroy(c->graph);
-    if (c->graph_alt) cudaGraphExecDestroy(c->graph_alt);
-    c->graph = nullptr;
-    c->graph_alt = nullptr;
-    c->graph_iters = 0;
+void drop_graph(cudaGraphExec_t* g) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+}
+
+// Drops the iteration graphs (but `keep`) and the streaming steps' second one.
+void drop_graphs(mlem_ctx* c, const cudaGraphExec_t* keep = nullptr) {
+    for (auto& kind : c->graphs)
+        for (auto& g : kind)
+            if (&g.exec != keep) drop_graph(&g.exec);
+    if (!keep) drop_graph(&c->graph_alt);
 }
 
 // Capture `n` iterations (slot reset + n x (iteration + statistics), or the
@@ -1322,20 +1325,19 @@ int capture_into(mlem_ctx* c, const mlem_tuning& t, int n, bool stats, cudaGraph
     return MLEM_OK;
 }
 
-int capture(mlem_ctx* c, const mlem_tuning& t, int n, bool stats) {
-    drop_graph(c);
-    TRY(capture_into(c, t, n, stats, &c->graph));
-    c->graph_iters = n;
-    c->graph_stats = stats;
-    c->graph_one_pass = &t == &c->one_pass;
+// The graph of n iterations of tuning t (mlem_ctx::tuning or one_pass), with the
+// census or not, captured when the last one of that kind is no longer it.
+int graph_for(mlem_ctx* c, const mlem_tuning& t, int n, bool stats, cudaGraphExec_t** out) {
+    if (c->graph_dirty) drop_graphs(c);
     c->graph_dirty = false;
+    auto& g = c->graphs[stats][&t == &c->one_pass];
+    if (!g.exec || g.iters != n) {
+        drop_graph(&g.exec);
+        TRY(capture_into(c, t, n, stats, &g.exec));
+        g.iters = n;
+    }
+    *out = &g.exec;
     return MLEM_OK;
-}
-
-// Whether the captured graph is n iterations of tuning t (with the census or not).
-bool graph_is(const mlem_ctx* c, const mlem_tuning& t, int n, bool stats) {
-    return !c->graph_dirty && c->graph && c->graph_iters == n && c->graph_stats == stats &&
-           c->graph_one_pass == (&t == &c->one_pass);
 }
 
 int ensure_tmp(mlem_ctx* c) {
@@ -1778,7 +1780,7 @@ void mlem_destroy(mlem_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    drop_graph(c);
+    drop_graphs(c);
     free_frames(c);
     region_free(&c->rb);
     for (void* p : {(void*)c->row_ptr, (void*)c->elems, (void*)c->col_ptr, (void*)c->celems,
@@ -2068,12 +2070,13 @@ int mlem_iterate(mlem_ctx* c, int n, double* sums, uint64_t* zeros, uint64_t* su
     const int chunk = std::min(n, 64);
     const bool stats = sums || zeros || subn;  // the census only when the caller takes it
     TRY(ensure_history(c, chunk));
-    if (!graph_is(c, t, chunk, stats)) TRY(capture(c, t, chunk, stats));
+    cudaGraphExec_t* graph = nullptr;
+    TRY(graph_for(c, t, chunk, stats, &graph));
     int done = 0;
     while (done < n) {
         const int k = std::min(chunk, n - done);
         if (k == chunk) {
-            CK(c, cudaGraphLaunch(c->graph, c->stream));
+            CK(c, cudaGraphLaunch(*graph, c->stream));
         } else {
             if (stats) CK(c, cudaMemsetAsync(c->stats_slot, 0, 4, c->stream));
             for (int i = 0; i < k; ++i) TRY(enqueue_iteration(c, t, stats));
@@ -2131,11 +2134,9 @@ int mlem_step_host(mlem_ctx* c, const int32_t* sino, float* images, uint32_t B) 
     const mlem_tuning& t = tuning_for(c, true);
     if (t.bk_mode == MLEM_BK_REGION && !(c->flags & MLEM_FLAG_EXACT))
         TRY(ensure_region(c, t.frame_tile));
-    if (!graph_is(c, t, 1, false)) {
-        TRY(ensure_history(c, 1));
-        TRY(capture(c, t, 1, false));
-    }
-    CK(c, cudaGraphLaunch(c->graph, c->stream));
+    cudaGraphExec_t* graph = nullptr;
+    TRY(graph_for(c, t, 1, false, &graph));
+    CK(c, cudaGraphLaunch(*graph, c->stream));
     TRY(download_images(c, images));
     CK(c, cudaStreamSynchronize(c->stream));
     if (counts) {
@@ -2195,11 +2196,9 @@ static int stream_steps(mlem_ctx* c, const int32_t* const* sinos, float* const* 
         TRY(build_active(c, false, false));
         ++c->sino_gen;
         const mlem_tuning& t = tuning_for(c, true);
-        if (!graph_is(c, t, 1, false)) {
-            TRY(ensure_history(c, 1));
-            TRY(capture(c, t, 1, false));
-        }
-        CK(c, cudaGraphLaunch(c->graph, c->stream));
+        cudaGraphExec_t* graph = nullptr;
+        TRY(graph_for(c, t, 1, false, &graph));
+        CK(c, cudaGraphLaunch(*graph, c->stream));
         if (images && images[k]) {  // this iteration's images, once the buffer's last download is done
             CK(c, cudaStreamWaitEvent(c->stream, c->ev_dfree[cur], 0));
             if (Bp == 1 && !c->bricked)
@@ -2272,10 +2271,8 @@ static int stream_steps_overlap(mlem_ctx* c, const int32_t* const* sinos, float*
         c->graph_dirty = true;
     }
     const mlem_tuning& t = tuning_for(c, true);
-    if (!graph_is(c, t, 1, false)) {
-        TRY(ensure_history(c, 1));
-        TRY(capture(c, t, 1, false));
-    }
+    cudaGraphExec_t* first = nullptr;
+    TRY(graph_for(c, t, 1, false, &first));
     if (!c->graph_alt) {
         swap_sets(c);
         const int s = capture_into(c, t, 1, false, &c->graph_alt);
@@ -2285,7 +2282,7 @@ static int stream_steps_overlap(mlem_ctx* c, const int32_t* const* sinos, float*
     const SinoSet set[2] = {{c->sino, c->act_order, c->act_ranges, c->act_n, c->act_z},
                             {c->sino_alt, c->act_order_alt, c->act_ranges_alt, c->act_n_alt,
                              c->act_z_alt}};
-    const cudaGraphExec_t graph[2] = {c->graph, c->graph_alt};
+    const cudaGraphExec_t graph[2] = {*first, c->graph_alt};
     // set q takes step j's sinograms once the step two before has iterated on it
     auto upload = [&](uint32_t j, int q) -> int {
         CK(c, cudaStreamWaitEvent(c->up_stream, c->ev_sfree[q], 0));
@@ -2328,7 +2325,8 @@ static int stream_steps_overlap(mlem_ctx* c, const int32_t* const* sinos, float*
     }
     if ((n - 1) & 1) {  // the last sinograms are in the second set: it becomes the first
         swap_sets(c);
-        std::swap(c->graph, c->graph_alt);
+        std::swap(*first, c->graph_alt);
+        drop_graphs(c, first);  // the other kinds' graphs hold the set that is now the second
     }
     return MLEM_OK;
 }

@@ -65,9 +65,10 @@ struct mlem_batch {
     unsigned int* counter = nullptr;  // one counter per group, kCounterStride apart
     bool scheduled = false;
 
-    cudaGraphExec_t graph = nullptr;
-    int graph_iters = 0;
-    bool graph_stats = false;  // the graph holds the census
+    struct {  // captured iterations, without and with the census
+        cudaGraphExec_t exec = nullptr;
+        int iters = 0;
+    } graphs[2];
     bool graph_dirty = true;
     std::vector<const void*> graph_sig;  // context pointers the graph holds
 
@@ -401,27 +402,38 @@ int batch_reset_slots(mlem_batch* b) {
     return MLEM_OK;
 }
 
-void batch_drop_graph(mlem_batch* b) {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-    b->graph_iters = 0;
+void batch_drop_graphs(mlem_batch* b) {
+    for (auto& g : b->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
 }
 
-int batch_capture(mlem_batch* b, int n, bool stats) {
-    batch_drop_graph(b);
-    BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    int s = stats ? batch_reset_slots(b) : MLEM_OK;
-    for (int i = 0; i < n && s == MLEM_OK; ++i) s = batch_enqueue(b, stats);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-    if (s != MLEM_OK) { if (g) cudaGraphDestroy(g); return s; }
-    if (e != cudaSuccess) return bfail(b, MLEM_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&b->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return bfail(b, MLEM_ERR_CUDA, "instantiate: %s", cudaGetErrorString(e));
-    b->graph_iters = n;
-    b->graph_stats = stats;
+// The graph of n iterations, with the census or not, captured when the last one is
+// no longer it.
+int batch_graph(mlem_batch* b, int n, bool stats, cudaGraphExec_t* out) {
+    if (b->graph_dirty) batch_drop_graphs(b);
     b->graph_dirty = false;
+    auto& mine = b->graphs[stats];
+    if (!mine.exec || mine.iters != n) {
+        if (mine.exec) cudaGraphExecDestroy(mine.exec);
+        mine.exec = nullptr;
+        BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+        int s = stats ? batch_reset_slots(b) : MLEM_OK;
+        for (int i = 0; i < n && s == MLEM_OK; ++i) s = batch_enqueue(b, stats);
+        cudaGraph_t g = nullptr;
+        cudaError_t e = cudaStreamEndCapture(b->stream, &g);
+        if (s != MLEM_OK) { if (g) cudaGraphDestroy(g); return s; }
+        if (e != cudaSuccess) return bfail(b, MLEM_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
+        e = cudaGraphInstantiate(&mine.exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            mine.exec = nullptr;
+            return bfail(b, MLEM_ERR_CUDA, "instantiate: %s", cudaGetErrorString(e));
+        }
+        mine.iters = n;
+    }
+    *out = mine.exec;
     return MLEM_OK;
 }
 
@@ -439,7 +451,7 @@ int batch_time(mlem_batch* b, int reps, cudaEvent_t e0, cudaEvent_t e1, double* 
 }
 
 void batch_free(mlem_batch* b) {
-    batch_drop_graph(b);
+    batch_drop_graphs(b);
     dev_free(b->items_d);
     dev_free(b->counter);
 }
@@ -785,13 +797,13 @@ int mlem_batch_iterate(mlem_batch* b, int n, double* const* sums) {
     TRY(batch_refresh(b, chunk));
     bool stats = false;  // the census only when the caller takes it
     for (size_t i = 0; sums && i < b->ctx.size(); ++i) stats = stats || sums[i];
-    if (b->graph_dirty || !b->graph || b->graph_iters != chunk || b->graph_stats != stats)
-        TRY(batch_capture(b, chunk, stats));
+    cudaGraphExec_t graph = nullptr;
+    TRY(batch_graph(b, chunk, stats, &graph));
     int done = 0;
     while (done < n) {
         const int k = std::min(chunk, n - done);
         if (k == chunk) {
-            BCK(b, cudaGraphLaunch(b->graph, b->stream));
+            BCK(b, cudaGraphLaunch(graph, b->stream));
         } else {
             if (stats) TRY(batch_reset_slots(b));
             for (int i = 0; i < k; ++i) TRY(batch_enqueue(b, stats));

@@ -197,10 +197,13 @@ struct mlem_ctx {
     mlem_tuning one_pass{};
     bool has_one_pass = false;
     bool tile_follows = true;  // no tuning chosen yet: the frame tile follows the frame count
-    cudaGraphExec_t graph = nullptr;
-    int graph_iters = 0;
-    bool graph_stats = false;  // the graph holds the census
-    bool graph_one_pass = false;  // the graph was captured with one_pass, not tuning
+    // Captured iterations, one graph for every kind of run (graph_for): without or
+    // with the census, of tuning or of one_pass, so that calls of different kinds in
+    // turn do not capture each time.
+    struct {
+        cudaGraphExec_t exec = nullptr;
+        int iters = 0;
+    } graphs[2][2];
     bool graph_dirty = true;
 
     std::string err;

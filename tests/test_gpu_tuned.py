@@ -114,3 +114,49 @@ def test_iterations_after_streamed_steps_run_the_chosen_method():
             ctx.iterate(3)
             got.append(ctx.get_images())
         assert all(np.array_equal(a, got[0]) for a in got[1:])
+
+
+def captures(call):
+    """Graphs instantiated by call()."""
+    torch = pytest.importorskip("torch")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU,
+                                            torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+    return sum(e.count for e in prof.key_averages() if e.key.startswith("cudaGraphInstantiate"))
+
+
+def test_kinds_of_iterations_in_turn_keep_their_graphs():
+    """Single iterations with and without statistics and host steps in turn are captured
+    once each, not on every call; the streamed steps' two buffer sets, swapped after an
+    odd number of them, do not leave another kind with a graph of the wrong one."""
+    g = synth.Geometry(16, 16, 8, 900, 20, 60, seed=1)
+    m = synth.host_matrix(g)
+    rng = np.random.default_rng(6)
+    s, s2 = (rng.poisson(4, (2, g.n_rows)).astype(np.int32) for _ in range(2))
+    with api.Context.from_matrix(m) as ctx, api.Context.from_matrix(m) as other:
+        for c in (ctx, other):
+            c.set_tuning(api.BK_FUSED, 32, 1, 8, api.VISIT_SORTED)
+            c.set_sinograms(s)
+            c.init_images()
+        x = ctx.get_images()
+        batch = api.Batch([other])
+
+        def turn():
+            ctx.iterate(1, stats=True)
+            ctx.iterate(1, stats=False)
+            ctx.step_host(s, x)
+            batch.iterate(2, stats=True)
+            batch.iterate(2, stats=False)
+
+        assert captures(lambda: (turn(), turn())) > 0
+        assert captures(lambda: (turn(), turn(), turn())) == 0
+        batch.close()
+        for n in (1, 2, 3):  # the last sinograms in either set
+            ctx.iterate(2, stats=False)
+            ctx.stream_host([s2] * (n - 1) + [s])
+            for stats in (True, False):
+                ctx.init_images()
+                ctx.iterate(2, stats=stats)
+                got = ctx.get_images()
+                for b in range(2):
+                    assert ob.rel_l2(got[b], ob.mlem(m, s[b], 2)[0]) <= TOL
