@@ -352,7 +352,8 @@ __device__ __forceinline__ void fused_row_range(const SparseView& csr, const flo
 // registers for the scatter.  For matrices of short rows (SparseView::short_rows):
 // beyond 256 elements a row's rest is read one load at a time, which on rows of
 // 1,500 elements cost a third (6.2e9 elements: 44 ms against 33 for
-// fused_row_range), and row lengths have 32 bits.  Against
+// fused_row_range) and behind 1 % of rows of 2,000 a fifth, and row lengths have
+// 32 bits.  Against
 // fused_row_range (B200): plain-full 2.11 -> 2.08 ms, 1,048,576 rows 543 -> 532
 // us, eight subsets of 500,003 rows 282 -> 248 us in chunks, 253 -> 247 in grid
 // stride, 65,536 rows 22.6 -> 19.4 and 21.0 -> 18.3 us.  The adjoint kernels'

@@ -160,3 +160,44 @@ def test_kinds_of_iterations_in_turn_keep_their_graphs():
                 got = ctx.get_images()
                 for b in range(2):
                     assert ob.rel_l2(got[b], ob.mlem(m, s[b], 2)[0]) <= TOL
+
+
+def kernels(call):
+    """Names of the kernels launched by call()."""
+    torch = pytest.importorskip("torch")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+    return " ".join(e.key for e in prof.key_averages())
+
+
+def rows_of(lens, seed, n_cols=5000):
+    from mlem_b200 import formats
+    rng = np.random.default_rng(seed)
+    el = np.zeros(int(lens.sum()), formats.ELEM_DTYPE)
+    el["index"] = rng.integers(0, n_cols, el.size)
+    el["value"] = rng.uniform(0.05, 1.7, el.size)
+    return formats.Csr4(lens.size, n_cols, np.cumsum(lens).astype(np.uint64), el)
+
+
+@pytest.mark.parametrize("visit", [api.VISIT_SORTED, api.VISIT_SORTED_CHUNKED])
+@pytest.mark.parametrize("longest,mean,pipelined", [(256, 200, True), (400, 100, True), (401, 100, False),
+                                                    (400, 200, False), (2000, 100, False)])
+def test_pipelined_one_pass_walk_by_row_lengths(longest, mean, pipelined, visit):
+    """The pipelined one-frame walk takes matrices whose rows fit its batch, or mostly
+    do and end within five loads of it; longer rows go to the general walk.  Either
+    agrees with the oracle, rows that end at and beyond the batch among them."""
+    rng = np.random.default_rng(longest)
+    lens = rng.integers(2 * mean - 256, 257, 6000) if mean > 128 else rng.integers(0, 2 * mean - 20, 6000)
+    lens[:: 6000 // 20] = longest
+    if longest > 256:
+        lens[1:400:40] = 257, 287, 288, 289, 320, 352, 353, 383, 384, 399
+    assert lens.max() == longest and (lens.mean() > 128) == (mean > 128)
+    m = rows_of(lens, longest)
+    s = rng.poisson(5, m.n_rows).astype(np.int32)
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_tuning(api.BK_FUSED, 32, 1, 4, visit)
+        ctx.set_sinograms(s)
+        ctx.init_images()
+        ran = kernels(lambda: ctx.iterate(3))
+        assert ("k_fused_row_one" in ran or "k_fused_chunked_one" in ran) == pipelined, ran
+        assert ob.rel_l2(ctx.get_images()[0], ob.mlem(m, s, 3)[0]) <= TOL
