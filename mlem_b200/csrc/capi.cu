@@ -78,6 +78,8 @@ SparseView csr_view(const mlem_ctx* c) {
     SparseView v{c->row_ptr, reinterpret_cast<const uint4*>(c->elems), c->R, c->Z,
                  c->row_order, c->row_order ? c->row_ranges : nullptr};
     v.max_len = c->max_row_len;
+    // of the whole matrix, also where a view is cut to some of its rows
+    v.eight_a_lane = c->max_row_len <= 256 && c->Z > 128ull * c->R;
     // Every row in one batch of 256, or most rows and never more than five loads beyond
     // it (one_pass_rows' rest of a row).  200,000 rows, us per iteration sorted and in
     // chunks, the general walk against one_pass_rows: a fifth of the rows of 400 elements

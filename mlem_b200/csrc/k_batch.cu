@@ -208,7 +208,7 @@ cudaError_t fused_chunked(const SparseView& csr, const float* x, uint32_t B, int
     // that the row stays in registers for its scatter (1,048,576 rows of 200 elements
     // 1,038 -> 1,005 to 1,018 us per iteration).  Other rows lose with eight (120,007 of
     // odd lengths 84.7 -> 88.3 us, 400,000 of up to 470 1,068 -> 1,137).
-    if (frame_tile == 4 && csr.max_len <= 256 && csr.nnz > 128ull * csr.n)
+    if (frame_tile == 4 && csr.eight_a_lane)
         return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<4, 8>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);
     switch (frame_tile) {
         case 1: return launch_dependent(csr.n <= kDependentMost, k_fused_chunked<1>, grid, threads, 0, st, csr, x, B, sino, u, chunk_rows, counter);

@@ -53,6 +53,8 @@ struct SparseView {
     // The rows fit the pipelined one-frame one-pass walk (one_pass_rows), which
     // handles 256 elements of a row at once and the rest one load at a time.
     bool short_rows = false;
+    // Rows that eight elements a lane hold and four mostly do not (fused_chunked).
+    bool eight_a_lane = false;
     // The gather passes walk a row from the memory line it starts in, so that the
     // grouping of its sum depends on where it is stored.  Not with the CSC in file
     // order, whose sums do not depend on the voxel layout.

@@ -201,3 +201,24 @@ def test_pipelined_one_pass_walk_by_row_lengths(longest, mean, pipelined, visit)
         ran = kernels(lambda: ctx.iterate(3))
         assert ("k_fused_row_one" in ran or "k_fused_chunked_one" in ran) == pipelined, ran
         assert ob.rel_l2(ctx.get_images()[0], ob.mlem(m, s, 3)[0]) <= TOL
+
+
+@pytest.mark.parametrize("subsets", [1, 8])
+@pytest.mark.parametrize("mean", [40, 200])
+def test_depth_of_the_four_frame_walk_by_row_lengths(mean, subsets):
+    """Eight elements a lane at four frames for rows longer than four hold, of the whole
+    matrix or of its subsets alike."""
+    rng = np.random.default_rng(mean)
+    m = rows_of(rng.integers(mean - 20, mean + 21, 4000), mean)
+    s = rng.poisson(5, (4, m.n_rows)).astype(np.int32)
+    with api.Context.from_matrix(m) as ctx:
+        ctx.set_sinograms(s)
+        ctx.set_tuning(api.BK_FUSED, 32, 4, 4, api.VISIT_SORTED_CHUNKED)
+        ctx.set_subsets(subsets)
+        ctx.init_images()
+        ran = kernels(lambda: ctx.iterate(2))
+        assert ("k_fused_chunked<4, 8>" in ran) == (mean > 128), ran
+        got = ctx.get_images()
+    for b in (0, 3):
+        ref = ob.mlem(m, s[b], 2)[0] if subsets == 1 else ob.osem(m, s[b], 2, subsets)[0]
+        assert ob.rel_l2(got[b], ref) <= TOL
