@@ -425,18 +425,20 @@ struct BkRun {
     }
 };
 
-// Lanes per row.  A configuration's smaller groups are taken as given; 32 (the
-// default) means up to a warp, and as few as 8 lanes where rows are many: the
+// Lanes per row.  A configuration's groups of 4 and 8 are taken as given; 16 and 32 (the
+// default) mean at most that many, and as few as 8 lanes where rows are many: the
 // rows (or columns) next to one another in a warp are neighbouring rays
 // (voxels), which share lines of the gathered vector, and no lane idles
 // behind the end of a row.  Plain-full forward + back projection at one frame
 // 2.38 ms with 32 lanes, 1.98 with 16, 1.93 with 8; 1,048,576 rows at 16
-// frames 2.42, 2.13, 2.08 ms.  More lanes where 8 would leave half of the
+// frames 2.42, 2.13, 2.08 ms; 200,003 rows at one frame forward 70.7 us with 16 and 54.6
+// with 8, back projection 84.1 and 62.6.  More lanes where 8 would leave half of the
 // resident warps without a row, or where the longest row would outlast four
 // times a group's share of the elements.
 int gather_lanes(const SparseView& s, const LaunchCfg& cfg) {
-    if (cfg.group != 32) return cfg.group;
+    if (cfg.group < 16) return cfg.group;
     for (int g : {8, 16}) {
+        if (g == cfg.group) return g;
         const uint64_t groups = (uint64_t)cfg.sm_count * kGatherCtas * kGatherThreads / g;
         const uint64_t used = std::min<uint64_t>(s.n, groups);
         if (used * 2 >= groups && s.max_len <= 4 * (s.nnz / used)) return g;

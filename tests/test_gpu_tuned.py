@@ -222,3 +222,20 @@ def test_depth_of_the_four_frame_walk_by_row_lengths(mean, subsets):
     for b in (0, 3):
         ref = ob.mlem(m, s[b], 2)[0] if subsets == 1 else ob.osem(m, s[b], 2, subsets)[0]
         assert ob.rel_l2(got[b], ref) <= TOL
+
+
+@pytest.mark.parametrize("rows,lanes", [(300, {4: 4, 8: 8, 16: 16, 32: 32}), (150000, {4: 4, 8: 8, 16: 8, 32: 8})])
+def test_lanes_of_the_gather_passes(rows, lanes):
+    """Groups of 16 and 32 lanes are the most a row gets: eight where rows are many."""
+    rng = np.random.default_rng(rows)
+    m = rows_of(rng.integers(1, 9, rows), rows, n_cols=rows)
+    s = rng.poisson(5, rows).astype(np.int32)
+    ref = ob.mlem(m, s, 2)[0]
+    with api.Context.from_matrix(m) as ctx:
+        for group, used in lanes.items():
+            ctx.set_tuning(api.BK_CSC, group, 1, 8)
+            ctx.set_sinograms(s)
+            ctx.init_images()
+            ran = kernels(lambda: ctx.iterate(2))
+            assert f"k_fwproj<{used}, 1" in ran, (group, ran)
+            assert ob.rel_l2(ctx.get_images()[0], ref) <= TOL
