@@ -634,9 +634,10 @@ cudaError_t copy_pageable(mlem_ctx* c, void* host, void* dev, size_t bytes, bool
         return to_host ? cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream)
                        : cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream);
     };
+    if (bytes < kStagedCopy) return plain();  // first: asking for the cores is a system call
     const int T = (int)std::min<size_t>({(size_t)kSlotThreads, (size_t)std::thread::hardware_concurrency(),
                                          bytes / (2 * kSlotBytes)});
-    if (bytes < kStagedCopy || T < 2) return plain();
+    if (T < 2) return plain();
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
     else if (at.type != cudaMemoryTypeUnregistered) return plain();
