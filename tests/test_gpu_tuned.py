@@ -239,3 +239,18 @@ def test_lanes_of_the_gather_passes(rows, lanes):
             ran = kernels(lambda: ctx.iterate(2))
             assert f"k_fwproj<{used}, 1" in ran, (group, ran)
             assert ob.rel_l2(ctx.get_images()[0], ref) <= TOL
+
+
+@pytest.mark.parametrize("rows,frames,on_device", [(601, 3, False), (25000, 1, False), (5000, 5, False),
+                                                   (25001, 1, True), (5001, 5, True)])
+def test_count_sums_where_they_are_cheap(rows, frames, on_device):
+    """Few counts are added on the host, many on the device, to the same start value."""
+    rng = np.random.default_rng(rows)
+    m = rows_of(np.ones(rows, np.int64), rows, n_cols=50)
+    s = rng.integers(-5, 1 << 30, (frames, rows)).astype(np.int32)
+    with api.Context.from_matrix(m) as ctx:
+        ran = kernels(lambda: ctx.set_sinograms(s))
+        assert ("k_count_sums" in ran) == on_device, ran
+        total = ctx.column_sums().astype(np.float64).cumsum()[-1]
+        want = [np.float32(float(s[b].sum(dtype=np.int64)) / total) for b in range(frames)]
+        assert np.array_equal(ctx.init_images(), want)
