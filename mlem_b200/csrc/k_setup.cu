@@ -402,7 +402,9 @@ __global__ void k_count_sums(const int32_t* __restrict__ s, uint64_t total, uint
 
 // Frame-major [B][n] <-> interleaved [n][Bp], V frames per access on the
 // interleaved side; a thread keeps to one item, so the frame-major side is
-// coalesced and no thread divides an index.  Pad frames are written as 0.
+// coalesced and no thread divides an index.  Pad frames are written as 0.  Where
+// the items do not fill the SMs, blockIdx.y takes a share of the frames (1,001
+// voxels of 32 frames: a thread's 32 loads in turn cost 4 us).
 template <typename T, int V>
 struct alignas(V * sizeof(T)) FrameVec {
     T v[V];
@@ -414,7 +416,7 @@ __global__ void k_interleave(const T* __restrict__ in, T* __restrict__ out, uint
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         T* to = out + (perm ? (uint64_t)perm[i] : i) * Bp;
-        for (uint32_t b0 = 0; b0 < Bp; b0 += V) {
+        for (uint32_t b0 = blockIdx.y * V; b0 < Bp; b0 += gridDim.y * V) {
             FrameVec<T, V> f;
 #pragma unroll
             for (int k = 0; k < V; ++k) f.v[k] = b0 + k < B ? in[(uint64_t)(b0 + k) * n + i] : T(0);
@@ -429,7 +431,7 @@ __global__ void k_deinterleave(const T* __restrict__ in, T* __restrict__ out, ui
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const T* from = in + (perm ? (uint64_t)perm[i] : i) * Bp;
-        for (uint32_t b0 = 0; b0 < B; b0 += V) {
+        for (uint32_t b0 = blockIdx.y * V; b0 < B; b0 += gridDim.y * V) {
             const FrameVec<T, V> f = *reinterpret_cast<const FrameVec<T, V>*>(from + b0);
 #pragma unroll
             for (int k = 0; k < V; ++k)
@@ -698,9 +700,10 @@ template <typename T, bool TO_FRAMES>
 cudaError_t run_interleave(const T* in, T* out, uint64_t n, uint32_t B, uint32_t Bp,
                            const uint32_t* perm, cudaStream_t st) {
     if (n * B == 0) return cudaSuccess;
-    const unsigned grid = elementwise_grid(n);
     auto go = [&](auto v) {
         constexpr int V = decltype(v)::value;
+        const unsigned gx = elementwise_grid(n);
+        const dim3 grid(gx, std::min<unsigned>((unsigned)ceil_div(Bp, V), std::max(1u, kB200SMs * 4u / gx)));
         if (TO_FRAMES) k_deinterleave<T, V><<<grid, 256, 0, st>>>(in, out, n, B, Bp, perm);
         else k_interleave<T, V><<<grid, 256, 0, st>>>(in, out, n, B, Bp, perm);
         return cudaGetLastError();
