@@ -366,6 +366,14 @@ int mlem_apply_update_d(mlem_ctx* ctx, const float* update, float* x, uint32_t n
  * (mlem_fwproj_d and mlem_bkproj_d can be captured). */
 int mlem_fwproj_frames_d(mlem_ctx* ctx, const float* x, float* y, uint32_t n_frames, void* stream);
 int mlem_bkproj_frames_d(mlem_ctx* ctx, const float* y, float* x, uint32_t n_frames, void* stream);
+/* The same in the caller's scratch, mlem_frames_scratch's number of floats on a
+ * 256-byte boundary, free again once the call's work on `stream` is done.  Such calls
+ * share nothing with others and can be captured. */
+int mlem_frames_scratch(const mlem_ctx* ctx, uint32_t n_frames, uint64_t* floats);
+int mlem_fwproj_frames_in_d(mlem_ctx* ctx, const float* x, float* y, uint32_t n_frames,
+                            float* scratch, void* stream);
+int mlem_bkproj_frames_in_d(mlem_ctx* ctx, const float* y, float* x, uint32_t n_frames,
+                            float* scratch, void* stream);
 /* The two one-pass kernels of the unrolled MLEM's backward pass (one frame,
  * device pointers, natural voxel order; no counterpart in the reference):
  *   mlem_ratio_rows_d:    update = A^T calcCorrel(sino, A x) as

@@ -397,13 +397,28 @@ class Context:
     def bkproj_d(self, y_ptr: int, x_ptr: int, n_frames: int = 1, stream: int = 0) -> None:
         self._chk(core_lib().mlem_bkproj_d(self._h, y_ptr, x_ptr, n_frames, stream))
 
-    def fwproj_frames_d(self, x_ptr: int, y_ptr: int, n_frames: int, stream: int = 0) -> None:
-        """fwproj_d on frame-major vectors, x[B][C] and y[B][R]."""
-        self._chk(core_lib().mlem_fwproj_frames_d(self._h, x_ptr, y_ptr, n_frames, stream))
+    def frames_scratch(self, n_frames: int) -> int:
+        """Floats of scratch that fwproj_frames_d and bkproj_frames_d need."""
+        n = ctypes.c_uint64()
+        self._chk(core_lib().mlem_frames_scratch(self._h, n_frames, ctypes.byref(n)))
+        return n.value
 
-    def bkproj_frames_d(self, y_ptr: int, x_ptr: int, n_frames: int, stream: int = 0) -> None:
-        """bkproj_d on frame-major vectors, y[B][R] and x[B][C]."""
-        self._chk(core_lib().mlem_bkproj_frames_d(self._h, y_ptr, x_ptr, n_frames, stream))
+    def fwproj_frames_d(self, x_ptr: int, y_ptr: int, n_frames: int, stream: int = 0,
+                        scratch_ptr: int = 0) -> None:
+        """fwproj_d on frame-major vectors, x[B][C] and y[B][R]; scratch: the caller's
+        (frames_scratch floats) or, 0, the context's."""
+        if scratch_ptr:
+            self._chk(core_lib().mlem_fwproj_frames_in_d(self._h, x_ptr, y_ptr, n_frames, scratch_ptr, stream))
+        else:
+            self._chk(core_lib().mlem_fwproj_frames_d(self._h, x_ptr, y_ptr, n_frames, stream))
+
+    def bkproj_frames_d(self, y_ptr: int, x_ptr: int, n_frames: int, stream: int = 0,
+                        scratch_ptr: int = 0) -> None:
+        """bkproj_d on frame-major vectors, y[B][R] and x[B][C]; scratch as above."""
+        if scratch_ptr:
+            self._chk(core_lib().mlem_bkproj_frames_in_d(self._h, y_ptr, x_ptr, n_frames, scratch_ptr, stream))
+        else:
+            self._chk(core_lib().mlem_bkproj_frames_d(self._h, y_ptr, x_ptr, n_frames, stream))
 
     def fwproj_correl_d(self, x_ptr, sino_ptr, correl_ptr, n_frames=1, stream=0) -> None:
         self._chk(core_lib().mlem_fwproj_correl_d(self._h, x_ptr, sino_ptr, correl_ptr, n_frames,

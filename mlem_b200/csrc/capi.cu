@@ -252,8 +252,13 @@ int scratch_end(mlem_ctx* c, cudaStream_t st, const CallScratch& s) {
 }
 size_t voxel_scratch(const mlem_ctx* c, uint32_t B) { return c->bricked ? (size_t)c->C * B : 0; }
 
+// Voxel and row vectors of Bd interleaved frames, back to back in one block.
+size_t frame_voxels(const mlem_ctx* c, uint32_t Bd) { return ((size_t)c->C * Bd + 63) & ~(size_t)63; }
+size_t frame_floats(const mlem_ctx* c, uint32_t Bd) { return frame_voxels(c, Bd) + (size_t)c->R * Bd; }
+float* frame_rows(const mlem_ctx* c, float* block, uint32_t Bd) { return block + frame_voxels(c, Bd); }
+
 // Voxel and row vectors of Bd interleaved frames for one projection on `st`
-// (frame_voxels, frame_rows); false where they do not fit beside the matrix or where the
+// in the context's block; false where they do not fit beside the matrix or where the
 // stream is being captured (a graph may be replayed beside, or after, a call that
 // uses or replaces them), and the caller's frame count is walked as it is.  Calls
 // on several streams take turns: each waits for the last one's frame_room_done.
@@ -263,8 +268,7 @@ bool frame_room(mlem_ctx* c, uint32_t Bd, cudaStream_t st) {
         cudaGetLastError();
         return false;
     }
-    const size_t voxels = (((size_t)c->C * Bd + 63) & ~(size_t)63), floats = voxels + (size_t)c->R * Bd;
-    if (grow(c, &c->fscratch, &c->fscratch_floats, floats) != MLEM_OK) {
+    if (grow(c, &c->fscratch, &c->fscratch_floats, frame_floats(c, Bd)) != MLEM_OK) {
         c->err.clear();
         return false;
     }
@@ -275,8 +279,6 @@ bool frame_room(mlem_ctx* c, uint32_t Bd, cudaStream_t st) {
     }
     return true;
 }
-float* frame_voxels(mlem_ctx* c) { return c->fscratch; }
-float* frame_rows(mlem_ctx* c, uint32_t Bd) { return c->fscratch + (((size_t)c->C * Bd + 63) & ~(size_t)63); }
 int frame_room_done(mlem_ctx* c, cudaStream_t st) {
     CK(c, cudaEventRecord(c->ev_frames, st));
     return MLEM_OK;
@@ -2767,9 +2769,10 @@ int mlem_fwproj_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* strea
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = fw_stride(c, B);
     if (Bd != B && frame_room(c, Bd, st)) {
-        CK(c, permute_to_device(x, frame_voxels(c), c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
-        TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
-        CK(c, permute_to_natural(frame_rows(c, Bd), y, nullptr, c->R, B, Bd, st));
+        float* rows = frame_rows(c, c->fscratch, Bd);
+        CK(c, permute_to_device(x, c->fscratch, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+        TRY(project_rows(c, c->fscratch, rows, Bd, st));
+        CK(c, permute_to_natural(rows, y, nullptr, c->R, B, Bd, st));
         return frame_room_done(c, st);
     }
     CallScratch s;
@@ -2785,9 +2788,10 @@ int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* strea
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = bk_stride(c, B);
     if (Bd != B && frame_room(c, Bd, st)) {
-        CK(c, permute_to_device(y, frame_rows(c, Bd), nullptr, c->R, B, Bd, st));
-        TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
-        CK(c, permute_to_natural(frame_voxels(c), x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
+        float* rows = frame_rows(c, c->fscratch, Bd);
+        CK(c, permute_to_device(y, rows, nullptr, c->R, B, Bd, st));
+        TRY(project_columns(c, rows, c->fscratch, Bd, st));
+        CK(c, permute_to_natural(c->fscratch, x, c->bricked ? c->perm : nullptr, c->C, B, Bd, st));
         return frame_room_done(c, st);
     }
     CallScratch s;
@@ -2798,30 +2802,54 @@ int mlem_bkproj_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* strea
     return scratch_end(c, st, s);
 }
 
-int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* stream) {
-    if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
+int mlem_frames_scratch(const mlem_ctx* c, uint32_t B, uint64_t* floats) {
+    if (!c || !floats || B == 0) return fail(const_cast<mlem_ctx*>(c), MLEM_ERR_INVALID, "bad argument");
+    *floats = frame_floats(c, std::max(fw_stride(c, B), bk_stride(c, B)));
+    return MLEM_OK;
+}
+
+int mlem_fwproj_frames_in_d(mlem_ctx* c, const float* x, float* y, uint32_t B, float* scratch,
+                            void* stream) {
+    if (!c || !x || !y || !scratch || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t Bd = fw_stride(c, B);
-    if (!frame_room(c, Bd, st))
-        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
-    CK(c, interleave_f32(x, frame_voxels(c), c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
-    TRY(project_rows(c, frame_voxels(c), frame_rows(c, Bd), Bd, st));
-    CK(c, deinterleave_f32(frame_rows(c, Bd), y, c->R, B, Bd, nullptr, st));
-    return frame_room_done(c, st);
+    float* rows = frame_rows(c, scratch, Bd);
+    CK(c, interleave_f32(x, scratch, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
+    TRY(project_rows(c, scratch, rows, Bd, st));
+    CK(c, deinterleave_f32(rows, y, c->R, B, Bd, nullptr, st));
+    return MLEM_OK;
+}
+
+int mlem_bkproj_frames_in_d(mlem_ctx* c, const float* y, float* x, uint32_t B, float* scratch,
+                            void* stream) {
+    if (!c || !x || !y || !scratch || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
+    TRY(set_device(c));
+    cudaStream_t st = (cudaStream_t)stream;
+    const uint32_t Bd = bk_stride(c, B);
+    float* rows = frame_rows(c, scratch, Bd);
+    CK(c, interleave_f32(y, rows, c->R, B, Bd, nullptr, st));
+    TRY(project_columns(c, rows, scratch, Bd, st));
+    CK(c, deinterleave_f32(scratch, x, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
+    return MLEM_OK;
+}
+
+int mlem_fwproj_frames_d(mlem_ctx* c, const float* x, float* y, uint32_t B, void* stream) {
+    if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
+    TRY(set_device(c));
+    if (!frame_room(c, fw_stride(c, B), (cudaStream_t)stream))
+        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", fw_stride(c, B));
+    TRY(mlem_fwproj_frames_in_d(c, x, y, B, c->fscratch, stream));
+    return frame_room_done(c, (cudaStream_t)stream);
 }
 
 int mlem_bkproj_frames_d(mlem_ctx* c, const float* y, float* x, uint32_t B, void* stream) {
     if (!c || !x || !y || B == 0) return fail(c, MLEM_ERR_INVALID, "bad argument");
     TRY(set_device(c));
-    cudaStream_t st = (cudaStream_t)stream;
-    const uint32_t Bd = bk_stride(c, B);
-    if (!frame_room(c, Bd, st))
-        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", Bd);
-    CK(c, interleave_f32(y, frame_rows(c, Bd), c->R, B, Bd, nullptr, st));
-    TRY(project_columns(c, frame_rows(c, Bd), frame_voxels(c), Bd, st));
-    CK(c, deinterleave_f32(frame_voxels(c), x, c->C, B, Bd, c->bricked ? c->perm : nullptr, st));
-    return frame_room_done(c, st);
+    if (!frame_room(c, bk_stride(c, B), (cudaStream_t)stream))
+        return fail(c, MLEM_ERR_NOMEM, "no room for %u interleaved frames", bk_stride(c, B));
+    TRY(mlem_bkproj_frames_in_d(c, y, x, B, c->fscratch, stream));
+    return frame_room_done(c, (cudaStream_t)stream);
 }
 
 int mlem_fwproj_correl_d(mlem_ctx* c, const float* x, const int32_t* sino, float* correl,

@@ -327,3 +327,31 @@ def test_unrolled_mlem_under_saved_tensor_hooks(small, keep_bytes, per_voxel):
     for got in grads[1:]:
         for a, b in zip(got, grads[0]):
             assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("frames", [2, 3, 6, 17])
+def test_projections_of_several_frames_leave_no_memory_on_the_context(small, frames):
+    """Their scratch is torch's: the context's device memory stays what it is, also when
+    they are captured before any call has run, and the results are those of the
+    interleaved entry points."""
+    m = small[0]
+    st = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(frames)
+    with api.Context.from_matrix(m) as ctx:
+        held = ctx.info.device_bytes
+        for project, call, n, n_out in ((torch_ext.forward_project, ctx.fwproj_d, m.n_cols, m.n_rows),
+                                        (torch_ext.back_project, ctx.bkproj_d, m.n_rows, m.n_cols)):
+            v = torch.rand((frames, n), generator=gen, device="cuda")
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                captured = project(v, ctx)
+            got = project(v, ctx)
+            assert ctx.info.device_bytes == held
+            keep = [torch.rand_like(got) for _ in range(4)]  # over the scratch that is free again
+            captured.zero_()
+            graph.replay()
+            del graph
+            vi, out = v.t().contiguous(), torch.empty((n_out, frames), device="cuda")
+            call(vi.data_ptr(), out.data_ptr(), frames, st)
+            assert torch.equal(got, out.t()) and torch.equal(captured, got) and len(keep) == 4
+            held = ctx.info.device_bytes  # the interleaved call's own scratch stays
