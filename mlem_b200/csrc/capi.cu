@@ -2054,7 +2054,8 @@ int mlem_set_sinograms(mlem_ctx* c, const int32_t* sino, uint32_t B) {
 
 int mlem_init_images(mlem_ctx* c, float* initial) {
     if (!c) return fail(nullptr, MLEM_ERR_INVALID, "null context");
-    if (!c->B) return fail(c, MLEM_ERR_STATE, "mlem_set_sinograms must come first");
+    // (mlem_step_host changes the frame count without summing its sinograms)
+    if (!c->B || c->sumin.size() < c->B) return fail(c, MLEM_ERR_STATE, "mlem_set_sinograms must come first");
     TRY(set_device(c));
     FrameValues init{};
     for (uint32_t b = 0; b < c->B; ++b) init.v[b] = (float)(c->sumin[b] / c->sumnorm);

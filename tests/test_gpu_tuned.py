@@ -254,3 +254,20 @@ def test_count_sums_where_they_are_cheap(rows, frames, on_device):
         total = ctx.column_sums().astype(np.float64).cumsum()[-1]
         want = [np.float32(float(s[b].sum(dtype=np.int64)) / total) for b in range(frames)]
         assert np.array_equal(ctx.init_images(), want)
+
+
+def test_start_images_need_the_sums_of_the_frames():
+    """mlem_init_images after a host step with more frames than mlem_set_sinograms
+    has summed is refused, not read past the sums."""
+    m = rows_of(np.full(50, 3), 1, n_cols=40)
+    s = np.ones((6, 50), np.int32)
+    with api.Context.from_matrix(m) as ctx:
+        for before in (None, s[:2]):
+            if before is not None:
+                ctx.set_sinograms(before)
+            ctx.step_host(s, np.ones((6, 40), np.float32))
+            with pytest.raises(api.MlemError) as e:
+                ctx.init_images()
+            assert e.value.status == api.MLEM_ERR_STATE
+        ctx.set_sinograms(s)
+        assert ctx.init_images().size == 6
