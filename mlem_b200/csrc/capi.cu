@@ -110,6 +110,7 @@ LaunchCfg cfg_of(const mlem_ctx* c, const mlem_tuning& t) {
     cfg.frame_tile = t.frame_tile;
     cfg.blocks_per_sm = t.blocks_per_sm;
     cfg.sm_count = c->n_sm;
+    cfg.each_frame = c->tile_follows;  // nobody chose the tile: the results do not show it
     return cfg;
 }
 
@@ -1368,6 +1369,7 @@ LaunchCfg cfg_for_frames(const mlem_ctx* c, uint32_t B) {
     for (int v : {16, 8, 4, 2})
         if (B % v == 0) { t = v; break; }
     cfg.frame_tile = t;
+    cfg.each_frame = false;
     return cfg;
 }
 

@@ -104,7 +104,7 @@ struct FwOp {
     float* y;
     uint32_t B, off;
     uint32_t gmask;
-    bool writer;
+    bool writer, each;
     struct Row {
         const uint2* b;
         uint64_t n;                // elements
@@ -176,8 +176,8 @@ struct FwOp {
             } else {  // eight counts held over the row cost more than this wait
                 g_counts<VW>(sino + (size_t)p.r * B + off, s);
             }
-            // A row without counts in the tile's frames has calcCorrel 0 whatever its
-            // projection, NaN included, walked or not.
+            // A count of 0 has calcCorrel 0 whatever the projection, NaN included, where the
+            // row has none in the tile or (each) in its frame.
             int any = 0;
 #pragma unroll
             for (int i = 0; i < VW; ++i) any |= s[i];
@@ -187,7 +187,7 @@ struct FwOp {
             }
             float t[VW];
 #pragma unroll
-            for (int i = 0; i < VW; ++i) t[i] = any ? correl_of(s[i], acc[i]) : 0.0f;
+            for (int i = 0; i < VW; ++i) t[i] = (each ? s[i] : any) ? correl_of(s[i], acc[i]) : 0.0f;
             g_store<VW>(c + o, t);
         }
     }
@@ -374,9 +374,9 @@ __device__ __forceinline__ void gather_walk(const Op& op, const float* __restric
 template <int G, int BT, bool SKIP>
 __global__ void __launch_bounds__(kGatherThreads, kGatherCtas)
     k_fwproj(SparseView csr, const float* __restrict__ x, uint32_t B, uint32_t f0,
-             const int32_t* __restrict__ sino, float* __restrict__ c, float* __restrict__ y) {
+             const int32_t* __restrict__ sino, float* __restrict__ c, float* __restrict__ y, bool each) {
     MLEM_GATHER_SETUP
-    const FwOp<G, BT, SKIP> op{csr, sino, c, y, B, off, gmask, lane < FL};
+    const FwOp<G, BT, SKIP> op{csr, sino, c, y, B, off, gmask, lane < FL, each};
     gather_walk<G, BT>(op, x, B, off, v, stride, gmask);
 }
 
@@ -409,9 +409,9 @@ struct FwRun {
         if constexpr (BT <= 4)
             if (c && !y && !csr.n_dev)
                 return launch_dependent(cfg.dependent && csr.n <= kDependentMost, k_fwproj<G, BT, true>, grid, kGatherThreads, 0, st, csr, x, B,
-                                        f0, sino, c, y);
+                                        f0, sino, c, y, cfg.each_frame);
         return launch_dependent(cfg.dependent && csr.n <= kDependentMost, k_fwproj<G, BT, false>, grid, kGatherThreads, 0, st, csr, x, B, f0,
-                                sino, c, y);
+                                sino, c, y, cfg.each_frame);
     }
 };
 

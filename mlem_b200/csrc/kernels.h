@@ -79,6 +79,10 @@ struct LaunchCfg {
     int blocks_per_sm = 8;
     int sm_count = 148;
     bool dependent = true;  // small launches may be programmatic dependents
+    // calcCorrel of a count of 0 is 0 whatever the projection (NaN included): for every
+    // frame on its own, as passes of one frame have it, or for rows without a count in
+    // the whole tile.
+    bool each_frame = false;
 };
 
 // Valid launch configuration (group 4..32, frame tile 1..16, 1..8 blocks/SM).

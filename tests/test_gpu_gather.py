@@ -107,6 +107,14 @@ def test_rows_without_counts_drop_what_is_not_finite():
                 want = hit[:, None] & ~empty_tiles(s, min(B, 16))
                 assert np.array_equal(np.isnan(c.cpu().numpy()), want), B
                 assert not c.cpu().numpy()[empty_tiles(s, min(B, 16))].any()
+                # no tuning chosen: the widest tile, each frame on its own
+                with api.Context.from_matrix(m, flags=flags) as own:
+                    own.set_sinograms(np.ascontiguousarray(s.T))
+                    assert own.tuning()["frame_tile"] == min(B, 16)
+                    own.set_images(np.ascontiguousarray(x.T))
+                    own.iterate(1)
+                    ref = bad[:, None] | (A.T.astype(np.float32) @ (hit[:, None] & (s != 0)).astype(np.float32) > 0)
+                    assert np.array_equal(np.isnan(own.get_images().T), ref), (B, flags)
                 for tile in (t for t in (1, 2, 4, 8, 16) if t <= B):
                     for visit in (api.VISIT_FILE,) + (() if flags else (api.VISIT_SORTED,)):
                         ctx.set_sinograms(np.ascontiguousarray(s.T))
