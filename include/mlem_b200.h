@@ -120,8 +120,9 @@ typedef struct {
  * mlem_stream_host, one iteration per sinogram, walk the whole CSC in
  * visiting order instead (the copy takes about as long as the back
  * projection saves in six iterations), and so does mlem_iterate after them;
- * but where mlem_autotune chose the CSC method over the one-pass method, the
- * steps run the latter, whose sums (float atomics) vary from run to run.  The
+ * but where mlem_autotune chose the CSC method and found the one-pass method
+ * faster than the walk over the whole CSC, the steps run the latter, whose
+ * sums (float atomics) vary from run to run.  The
  * CSC method's sums are a fixed function of the matrix, the sinograms and the
  * entry point, the same from run to run. */
 typedef struct {
@@ -301,8 +302,9 @@ int mlem_set_tuning(mlem_ctx* ctx, const mlem_tuning* t);
  * the fastest (deterministic_only != 0 restricts to MLEM_BK_CSC).  Among all
  * methods, the fastest one-pass configuration is kept beside it: for ordered
  * subsets, mlem_fused_update_d and, where the fastest is MLEM_BK_CSC with
- * MLEM_VISIT_SORTED, mlem_step_host and mlem_stream_host, which then run it
- * although mlem_get_tuning names the CSC method (mlem_set_tuning with that
+ * MLEM_VISIT_SORTED but slower than it without the cut copy, mlem_step_host
+ * and mlem_stream_host, which then run it although mlem_get_tuning names the
+ * CSC method (mlem_set_tuning with that
  * result, or deterministic_only, makes them run the CSC method).  The image
  * state is restored afterwards. */
 int mlem_autotune(mlem_ctx* ctx, int deterministic_only, mlem_tuning* best);

@@ -966,12 +966,13 @@ int fused_pass(mlem_ctx* c, const mlem_tuning& t, const SparseView& csr, cudaStr
 // The tuning a run takes: the context's, or the autotuner's one-pass tuning
 // (mlem_ctx::one_pass): for ordered subsets, which no other method runs, and, where it
 // chose the CSC method in visiting order, in steps of one iteration per sinogram, which
-// have no cut copy of the sinograms (plain-full: 2.24 ms a streamed step against 2.57 for
-// the CSC method over every entry).  mlem_iterate without subsets always runs the
-// method that mlem_get_tuning names.
+// have no cut copy of the sinograms, if it was the faster one then (plain-full: 2.24 ms a
+// streamed step against 2.57 for the CSC method over every entry; 400,000 rows at 16
+// frames 2.7 ms against 1.7).  mlem_iterate without subsets always runs the method that
+// mlem_get_tuning names.
 const mlem_tuning& tuning_for(const mlem_ctx* c, bool steps) {
     const bool instead = c->has_one_pass && c->tuning.bk_mode != MLEM_BK_FUSED &&
-                         (c->n_subsets > 1 || (steps && csc_by_visit(c, c->tuning)));
+                         (c->n_subsets > 1 || (steps && c->steps_one_pass && csc_by_visit(c, c->tuning)));
     return instead ? c->one_pass : c->tuning;
 }
 
@@ -2586,6 +2587,21 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
                     CK(c, cudaMemcpyAsync(c->x, saved, xb, cudaMemcpyDeviceToDevice, c->stream));
                 }
             }
+    // the chosen method as steps of one iteration per sinogram run it, without the cut copy
+    double whole_ms = best.ms_per_iter;
+    if (csc_by_visit(c, best) && c->csc_act_ready) {
+        c->csc_act_ready = false;
+        int s = enqueue_iteration(c, best, false);
+        if (s == MLEM_OK && cudaEventRecord(e0, c->stream) == cudaSuccess)
+            for (int i = 0; i < 2 && s == MLEM_OK; ++i) s = enqueue_iteration(c, best, false);
+        c->csc_act_ready = true;
+        if (s != MLEM_OK) return s;
+        CK(c, cudaEventRecord(e1, c->stream));
+        CK(c, cudaEventSynchronize(e1));
+        float ms = 0.0f;
+        CK(c, cudaEventElapsedTime(&ms, e0, e1));
+        whole_ms = ms / 2.0;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     CK(c, cudaMemcpyAsync(c->x, saved, xb, cudaMemcpyDeviceToDevice, c->stream));
@@ -2599,6 +2615,7 @@ int mlem_autotune(mlem_ctx* c, int deterministic_only, mlem_tuning* best_out) {
     c->tuning = best;
     c->one_pass = one_pass;
     c->has_one_pass = one_pass.bk_mode == MLEM_BK_FUSED && one_pass.ms_per_iter < 1e30;
+    c->steps_one_pass = one_pass.ms_per_iter < whole_ms;
     c->tile_follows = false;
     c->graph_dirty = true;
     if (best_out) *best_out = best;

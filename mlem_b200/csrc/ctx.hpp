@@ -196,6 +196,7 @@ struct mlem_ctx {
     // want a cut copy it does not have (one iteration per sinogram).  See tuning_for.
     mlem_tuning one_pass{};
     bool has_one_pass = false;
+    bool steps_one_pass = false;  // it was faster than the chosen method without a cut copy
     bool tile_follows = true;  // no tuning chosen yet: the frame tile follows the frame count
     // Captured iterations, one graph for every kind of run (graph_for): without or
     // with the census, of tuning or of one_pass, so that calls of different kinds in

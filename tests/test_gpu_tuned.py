@@ -271,3 +271,34 @@ def test_start_images_need_the_sums_of_the_frames():
             assert e.value.status == api.MLEM_ERR_STATE
         ctx.set_sinograms(s)
         assert ctx.init_images().size == 6
+
+
+def test_steps_of_an_autotuned_context_run_the_faster_method():
+    """Host steps and streamed steps after mlem_autotune do not run the one-pass method
+    where the chosen CSC method over every entry is clearly faster."""
+    torch = pytest.importorskip("torch")
+    g = synth.Geometry(128, 128, 64, 300000, 150, 250, seed=1)
+    s = np.random.default_rng(1).poisson(4, (16, g.n_rows)).astype(np.int32)
+
+    def ms(ctx):
+        x = np.full((16, ctx.n_cols), 0.5, np.float32)
+        ctx.step_host(s, x)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            ctx.step_host(s, x)
+        at = {e.key: e.device_time_total for e in prof.key_averages()}
+        return (sum(t for k, t in at.items() if "k_fused" in k),
+                sum(t for k, t in at.items() if "k_fwproj" in k or "k_bkproj_csc" in k))
+
+    with api.Context.siddon(g) as ctx:
+        ctx.set_sinograms(s)
+        ctx.init_images()
+        ctx.set_tuning(api.BK_FUSED, 32, 16, 4, api.VISIT_SORTED_CHUNKED)
+        one_pass = ms(ctx)[0]
+        ctx.set_tuning(api.BK_CSC, 32, 16, 8, api.VISIT_SORTED)
+        two_pass = ms(ctx)[1]
+        ctx.set_sinograms(s)
+        ctx.init_images()
+        chosen = ctx.autotune()
+        if chosen["bk_mode"] != api.BK_CSC or one_pass < 1.1 * two_pass:
+            pytest.skip("the two methods are too close here")
+        assert ms(ctx)[0] == 0
