@@ -128,7 +128,7 @@ typedef struct {
 typedef struct {
     int bk_mode;        /* MLEM_BK_CSC, MLEM_BK_ATOMIC, MLEM_BK_FUSED or MLEM_BK_REGION */
     int group;          /* lanes per row/column: 4, 8, 16 or 32 (the projections over rows
-                           and CSC columns take 16 and 32 as the most, 8 where rows are many) */
+                           and CSC columns take it as the most: fewer where rows are many) */
     int frame_tile;     /* frames per pass over the matrix: 1, 2, 4, 8 or 16 */
     int blocks_per_sm;  /* 1..8 blocks of 256 threads per SM (chunked visit: 1, 2 or 4 CTAs
                            of 1024, 512 or 256 threads; staged visit: 1..4 CTAs of 256) */

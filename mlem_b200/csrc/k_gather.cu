@@ -425,20 +425,23 @@ struct BkRun {
     }
 };
 
-// Lanes per row.  A configuration's groups of 4 and 8 are taken as given; 16 and 32 (the
-// default) mean at most that many, and as few as 8 lanes where rows are many: the
+// Lanes per row.  A configuration's group (32 is the default) means at most that many,
+// and as few as 8 lanes where rows are many, 4 where they also have few elements: the
 // rows (or columns) next to one another in a warp are neighbouring rays
 // (voxels), which share lines of the gathered vector, and no lane idles
 // behind the end of a row.  Plain-full forward + back projection at one frame
 // 2.38 ms with 32 lanes, 1.98 with 16, 1.93 with 8; 1,048,576 rows at 16
 // frames 2.42, 2.13, 2.08 ms; 200,003 rows at one frame forward 70.7 us with 16 and 54.6
-// with 8, back projection 84.1 and 62.6.  More lanes where 8 would leave half of the
+// with 8, back projection 84.1 and 62.6.  500,000 rows of 0 to 3 elements, forward at one
+// frame 50 us with 8 and 26 with 4, of 4 to 12 elements 54 and 30 (98 and 72 at 16
+// frames); 300,000 rows of 10 to 30 elements 36 and 33, 69 and 51 at 8 frames, the back
+// projections alike, of 30 to 60 elements 60 and 64.  More lanes where 8 would leave half of the
 // resident warps without a row, or where the longest row would outlast four
 // times a group's share of the elements.
 int gather_lanes(const SparseView& s, const LaunchCfg& cfg) {
-    if (cfg.group < 16) return cfg.group;
-    for (int g : {8, 16}) {
-        if (g == cfg.group) return g;
+    for (int g : {4, 8, 16}) {
+        if (g >= cfg.group) return cfg.group;
+        if (g == 4 && s.nnz > 12ull * s.n) continue;
         const uint64_t groups = (uint64_t)cfg.sm_count * kGatherCtas * kGatherThreads / g;
         const uint64_t used = std::min<uint64_t>(s.n, groups);
         if (used * 2 >= groups && s.max_len <= 4 * (s.nnz / used)) return g;

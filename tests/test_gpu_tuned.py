@@ -224,11 +224,15 @@ def test_depth_of_the_four_frame_walk_by_row_lengths(mean, subsets):
         assert ob.rel_l2(got[b], ref) <= TOL
 
 
-@pytest.mark.parametrize("rows,lanes", [(300, {4: 4, 8: 8, 16: 16, 32: 32}), (150000, {4: 4, 8: 8, 16: 8, 32: 8})])
-def test_lanes_of_the_gather_passes(rows, lanes):
-    """Groups of 16 and 32 lanes are the most a row gets: eight where rows are many."""
+@pytest.mark.parametrize("rows,mean,lanes", [(300, 5, {4: 4, 8: 8, 16: 16, 32: 32}),
+                                             (150000, 5, {4: 4, 8: 4, 16: 4, 32: 4}),
+                                             (12000, 5, {4: 4, 8: 8, 16: 8, 32: 8}),
+                                             (150000, 16, {4: 4, 8: 8, 16: 8, 32: 8})])
+def test_lanes_of_the_gather_passes(rows, mean, lanes):
+    """A group is the most lanes a row gets: eight where rows are many, four where they
+    are also short."""
     rng = np.random.default_rng(rows)
-    m = rows_of(rng.integers(1, 9, rows), rows, n_cols=rows)
+    m = rows_of(rng.integers(1, 2 * mean, rows), rows, n_cols=rows)
     s = rng.poisson(5, rows).astype(np.int32)
     ref = ob.mlem(m, s, 2)[0]
     with api.Context.from_matrix(m) as ctx:
