@@ -432,16 +432,22 @@ struct BkRun {
 // behind the end of a row.  Plain-full forward + back projection at one frame
 // 2.38 ms with 32 lanes, 1.98 with 16, 1.93 with 8; 1,048,576 rows at 16
 // frames 2.42, 2.13, 2.08 ms; 200,003 rows at one frame forward 70.7 us with 16 and 54.6
-// with 8, back projection 84.1 and 62.6.  500,000 rows of 0 to 3 elements, forward at one
-// frame 50 us with 8 and 26 with 4, of 4 to 12 elements 54 and 30 (98 and 72 at 16
-// frames); 300,000 rows of 10 to 30 elements 36 and 33, 69 and 51 at 8 frames, the back
-// projections alike, of 30 to 60 elements 60 and 64.  More lanes where 8 would leave half of the
-// resident warps without a row, or where the longest row would outlast four
-// times a group's share of the elements.
-int gather_lanes(const SparseView& s, const LaunchCfg& cfg) {
+// with 8, back projection 84.1 and 62.6.  Four lanes: 500,000 rows of 0 to 3 elements,
+// forward at one frame 50 us with 8 and 26 with 4, of 4 to 12 elements 54 and 30 (98 and 72
+// at 16 frames), the back projections alike; forward passes of up to eight frames also on
+// rows of up to kFourLaneRow elements: 400,000 rows of 15, 31, 44 and 60 on average 50 ->
+// 29, 50 -> 37, 52 -> 42 and 63 -> 48 us at one frame, 58 -> 42, 70 -> 49, 76 -> 58 and 86
+// -> 72 at four, 20,000 to 60,000 rows alike with either; at 16 frames 120,000 rows of 17
+// and of 59 lose (34 -> 38, 48 -> 52).  Back projections of columns of 54 elements lose at
+// one frame (95 -> 121 us), of 38 at 16 (130 -> 142).  More lanes where 8 would leave half
+// of the resident warps without a row, or where the longest row would outlast four times a
+// group's share of the elements.
+constexpr uint64_t kFourLaneRow = 64, kFourLane = 12;
+// (`four`: elements a row up to which four lanes take it.)
+int gather_lanes(const SparseView& s, const LaunchCfg& cfg, uint64_t four) {
     for (int g : {4, 8, 16}) {
         if (g >= cfg.group) return cfg.group;
-        if (g == 4 && s.nnz > 12ull * s.n) continue;
+        if (g == 4 && s.nnz > four * s.n) continue;
         const uint64_t groups = (uint64_t)cfg.sm_count * kGatherCtas * kGatherThreads / g;
         const uint64_t used = std::min<uint64_t>(s.n, groups);
         if (used * 2 >= groups && s.max_len <= 4 * (s.nnz / used)) return g;
@@ -472,8 +478,9 @@ cudaError_t dispatch_tile(const LaunchCfg& cfg, cudaStream_t st, Args... args) {
 }
 
 template <template <int, int> class K, typename... Args>
-cudaError_t dispatch_lanes(const SparseView& s, const LaunchCfg& cfg, cudaStream_t st, Args... args) {
-    switch (gather_lanes(s, cfg)) {
+cudaError_t dispatch_lanes(uint64_t four, const SparseView& s, const LaunchCfg& cfg, cudaStream_t st,
+                           Args... args) {
+    switch (gather_lanes(s, cfg, four)) {
         case 4: return dispatch_tile<K, 4>(cfg, st, s, args...);
         case 8: return dispatch_tile<K, 8>(cfg, st, s, args...);
         case 16: return dispatch_tile<K, 16>(cfg, st, s, args...);
@@ -493,7 +500,7 @@ cudaError_t fwproj(const SparseView& csr, const float* x, uint32_t B, uint32_t f
     t.frame_tile = aligned_tile(cfg.frame_tile, x, sino, c, y);
     cudaError_t e = cudaSuccess;
     for (uint32_t f = f0; f < f0 + (uint32_t)cfg.frame_tile && e == cudaSuccess; f += (uint32_t)t.frame_tile)
-        e = dispatch_lanes<FwRun>(csr, t, st, x, B, f, sino, c, y);
+        e = dispatch_lanes<FwRun>(t.frame_tile < 16 ? kFourLaneRow : kFourLane, csr, t, st, x, B, f, sino, c, y);
     return e;
 }
 
@@ -506,7 +513,7 @@ cudaError_t bkproj_csc(const SparseView& csc, const float* c, uint32_t B, uint32
     t.frame_tile = aligned_tile(cfg.frame_tile, c, norm ? x : u, nullptr, nullptr);
     cudaError_t e = cudaSuccess;
     for (uint32_t f = f0; f < f0 + (uint32_t)cfg.frame_tile && e == cudaSuccess; f += (uint32_t)t.frame_tile)
-        e = dispatch_lanes<BkRun>(csc, t, st, c, B, f, norm, x, u);
+        e = dispatch_lanes<BkRun>(kFourLane, csc, t, st, c, B, f, norm, x, u);
     return e;
 }
 

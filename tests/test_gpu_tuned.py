@@ -227,7 +227,8 @@ def test_depth_of_the_four_frame_walk_by_row_lengths(mean, subsets):
 @pytest.mark.parametrize("rows,mean,lanes", [(300, 5, {4: 4, 8: 8, 16: 16, 32: 32}),
                                              (150000, 5, {4: 4, 8: 4, 16: 4, 32: 4}),
                                              (12000, 5, {4: 4, 8: 8, 16: 8, 32: 8}),
-                                             (150000, 16, {4: 4, 8: 8, 16: 8, 32: 8})])
+                                             (150000, 16, {4: 4, 8: 4, 16: 4, 32: 4}),
+                                             (150000, 70, {4: 4, 8: 8, 16: 8, 32: 8})])
 def test_lanes_of_the_gather_passes(rows, mean, lanes):
     """A group is the most lanes a row gets: eight where rows are many, four where they
     are also short."""
@@ -306,3 +307,21 @@ def test_steps_of_an_autotuned_context_run_the_faster_method():
         if chosen["bk_mode"] != api.BK_CSC or one_pass < 1.1 * two_pass:
             pytest.skip("the two methods are too close here")
         assert ms(ctx)[0] == 0
+
+
+def test_four_lanes_a_row_by_frames():
+    """Rows of 12 to 64 elements: four lanes in forward passes of up to eight frames, eight
+    at 16 and in the back projection of columns as long."""
+    rng = np.random.default_rng(5)
+    m = rows_of(rng.integers(1, 80, 60000), 60000, n_cols=60000)
+    for frames, lanes in ((1, 4), (4, 4), (8, 4), (16, 8)):
+        s = rng.poisson(5, (frames, m.n_rows)).astype(np.int32)
+        with api.Context.from_matrix(m) as ctx:
+            ctx.set_sinograms(s)
+            ctx.set_tuning(api.BK_CSC, 32, frames, 8)
+            ctx.init_images()
+            ran = kernels(lambda: ctx.iterate(2))
+            assert f"k_fwproj<{lanes}, {frames}" in ran and f"k_bkproj_csc<8, {frames}>" in ran, ran
+            got = ctx.get_images()
+        for b in {0, frames - 1}:
+            assert ob.rel_l2(got[b], ob.mlem(m, s[b], 2)[0]) <= TOL
