@@ -171,9 +171,12 @@ __device__ __forceinline__ void ld_vec_if(const float* p, bool in, float (&v)[VW
 // loads, which the compiler spaces out (1,048,576 rows: 16 frames 4,499 us eager,
 // 3,864 conditional; 4 frames 1,322 and 1,127).  At one frame, and at two with a
 // warp per row, eager is at least as fast in either order (two frames, 16 lanes: 992
-// and 963).
+// and 963).  Four lanes a row want conditional loads at two frames in the sorted visit
+// too (1,048,576 rows 1,951 us eager, 1,858 conditional; 200,003 rows 95.2 and 93.0).
 template <int G, int BT, bool SORTED>
-constexpr bool eager_loads() { return SORTED || BT == 1 || (BT == 2 && G == 32); }
+constexpr bool eager_loads() {
+    return BT == 1 || (BT == 2 && G == 32) || (SORTED && !(BT == 2 && G == 4));
+}
 
 // Elements a lane loads before it gathers (memory-level parallelism).  A
 // full-warp group takes 8 (a 150-250-element row is one batch) at one and two
