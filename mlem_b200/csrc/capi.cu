@@ -1378,7 +1378,7 @@ LaunchCfg cfg_for_frames(const mlem_ctx* c, uint32_t B) {
 // B, or the padded count whose passes cost least -- a frame count that is no
 // multiple of a wide tile otherwise walks the matrix once per one, two or four
 // frames.  Cost of a pass by its tile, forward + back projection of 1,048,576
-// rows: 490, 656, 890, 1340, 2100 us for 1, 2, 4, 8, 16 frames.
+// rows: 490, 656, 890, 1340, 2100 us for 1, 2, 4, 8, 16 frames.  Only the ratios enter.
 uint32_t projection_stride(uint32_t B) {
     auto cost = [](uint32_t n) {
         for (auto t : {std::pair<uint32_t, double>{16, 2100.0}, {8, 1340.0}, {4, 890.0}, {2, 656.0}})
