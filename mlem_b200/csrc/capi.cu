@@ -2912,10 +2912,21 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
     }
     TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    // row sums: the mirrored method's full rows', or the long rows'
+    // the context's one-pass tuning when it has one, else sorted rows in chunks
+    mlem_tuning t = c->has_one_pass ? c->one_pass : c->tuning;
+    if (t.bk_mode != MLEM_BK_FUSED) {
+        t.visit = c->row_order ? MLEM_VISIT_SORTED_CHUNKED : MLEM_VISIT_FILE;
+        t.blocks_per_sm = c->row_order ? 4 : 8;
+        t.group = 32;
+    }
+    t.bk_mode = MLEM_BK_FUSED;
+    t.frame_tile = cfg_for_frames(c, B).frame_tile;
+    if (chunk_visit(t.visit)) t.group = 32;
+    // row sums: the mirrored method's full rows', or the long rows'; a counter for
+    // the walks that take their rows in chunks
     const size_t row_sums = (c->mirrored ? (size_t)c->R : (size_t)c->n_long) * B;
     CallScratch s;
-    TRY(scratch_begin(c, st, voxel_scratch(c, B), row_sums, !c->mirrored, &s));
+    TRY(scratch_begin(c, st, voxel_scratch(c, B), row_sums, !c->mirrored && chunk_visit(t.visit), &s));
     if (c->bricked) CK(c, permute_to_device(x, s.voxels[0], c->perm, c->C, B, B, st));
     const float* xd = c->bricked ? s.voxels[0] : x;
     float* ud = c->bricked ? s.voxels[1] : u;
@@ -2933,16 +2944,6 @@ int mlem_fused_update_d(mlem_ctx* c, const float* x, const int32_t* sino, float*
         if (c->bricked) CK(c, permute_to_natural(ud, u, c->perm, c->C, B, B, st));
         return scratch_end(c, st, s);
     }
-    // the context's one-pass tuning when it has one, else sorted rows in chunks
-    mlem_tuning t = c->has_one_pass ? c->one_pass : c->tuning;
-    if (t.bk_mode != MLEM_BK_FUSED) {
-        t.visit = c->row_order ? MLEM_VISIT_SORTED_CHUNKED : MLEM_VISIT_FILE;
-        t.blocks_per_sm = c->row_order ? 4 : 8;
-        t.group = 32;
-    }
-    t.bk_mode = MLEM_BK_FUSED;
-    t.frame_tile = cfg_for_frames(c, B).frame_tile;
-    if (chunk_visit(t.visit)) t.group = 32;
     CK(c, cudaMemsetAsync(ud, 0, (size_t)c->C * B * 4, st));
     SparseView v = csr_visit(c, t);
     if (c->n_long) v.long_len = kLongRowElems;
